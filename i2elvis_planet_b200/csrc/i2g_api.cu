@@ -768,10 +768,61 @@ int i2g_set_nodes(i2g_ctx *c, const double *ro, const double *nu, const double *
     return set_nodes_impl(c, f, cudaMemcpyHostToDevice);
 }
 
+// Whether kernels may write `count` doubles through every non-NULL out[k]: memory
+// of the context's device, whole inside its allocation, aligned, and no two of
+// the arrays overlapping.  Anything else (host memory, another device, a short
+// buffer) is left to cudaMemcpy, which copies or refuses it as it always did.
+static bool device_outputs(const i2g_ctx *c, double *const *out, int k, int64_t count)
+{
+    typedef int (*range_fn)(unsigned long long *, size_t *, unsigned long long);
+    static const range_fn range = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return (range_fn)f;
+    }();
+    if (!range) return false;
+    const uintptr_t bytes = (uintptr_t)count * sizeof(double);
+    for (int a = 0; a < k; a++) {
+        if (!out[a]) continue;
+        const uintptr_t p = (uintptr_t)out[a];
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, out[a]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeDevice || at.device != c->dev || p % sizeof(double)) return false;
+        unsigned long long base = 0;
+        size_t size = 0;
+        if (range(&base, &size, (unsigned long long)p) != 0 || p + bytes > base + size) return false;
+        for (int b = 0; b < a; b++) {
+            const uintptr_t q = (uintptr_t)out[b];
+            if (q && p < q + bytes && q < p + bytes) return false;
+        }
+    }
+    return true;
+}
+
 static int get_nodes_impl(i2g_ctx *c, double *const *f, cudaMemcpyKind kind)
 {
     if (!c) return I2G_EINVAL;
     CK(cudaSetDevice(c->dev));
+    if (kind == cudaMemcpyDeviceToDevice && device_outputs(c, f, N_N, c->nn)) {
+        CopyFields F{};
+        static_assert(N_N == kCopyFields, "node fields");
+        for (int k = 0; k < N_N; k++) {
+            F.in[k] = c->node[k];
+            F.out[k] = f[k];
+        }
+        c->launches += launch_copy_fields(c->stream, F, c->nn);
+        CKL();
+        CK(cudaStreamSynchronize(c->stream));
+        return I2G_OK;
+    }
     for (int k = 0; k < N_N; k++)
         if (f[k]) CK(cudaMemcpyAsync(f[k], c->node[k], sizeof(double) * (size_t)c->nn, kind, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -1006,6 +1057,19 @@ static int get_markers_impl(i2g_ctx *c, int64_t n, double *x, double *y, double 
     double *outs[6] = {x, y, T, eta, p, tmax};
     double *ins[6] = {b.x, b.y, b.T, b.eta, b.p, b.tmax};
     double *stage[6] = {s.x, s.y, s.T, s.eta, s.p, s.tmax};
+    if (!host && n > 0 && !tmax && !type && device_outputs(c, outs, kUnsortFields, n)) {
+        // straight into the caller's arrays; the averaging payload is free
+        // between calls (48 bytes per marker or more)
+        UnsortFields F{};
+        for (int k = 0; k < kUnsortFields; k++) {
+            F.in[k] = ins[k];
+            F.out[k] = outs[k];
+        }
+        c->launches += launch_unsort_fields(c->stream, F, n, b.id, c->payload, c->sb.perm1, c->ndeferred);
+        CKL();
+        CK(cudaStreamSynchronize(c->stream));
+        return I2G_OK;
+    }
     for (int k = 0; k < 6; k++) {
         if (!outs[k] || n <= 0) continue;
         c->launches += launch_unsort_f64(c->stream, n, b.id, ins[k], stage[k]);

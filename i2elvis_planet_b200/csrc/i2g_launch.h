@@ -55,6 +55,24 @@ int launch_iota(cudaStream_t s, int32_t *a, int64_t n);
 int launch_unsort_f64(cudaStream_t s, int64_t n, const int32_t *id, const double *in, double *out);
 int launch_unsort_i8(cudaStream_t s, int64_t n, const int32_t *id, const int8_t *in, int8_t *out);
 int launch_unsort_f64_f32(cudaStream_t s, int64_t n, const int32_t *id, const double *in, float *out);
+// several FP64 marker fields at once: out[k][id[j]] = in[k][j] (out[k] NULL: not
+// asked for); records: scratch of 48 n bytes,
+// bands: n device ints, verdict: one
+constexpr int kUnsortFields = 5;
+constexpr int64_t kUnsortDirectBytes = 96 << 20;
+struct UnsortFields {
+    const double *in[kUnsortFields];
+    double *out[kUnsortFields];
+};
+int launch_unsort_fields(cudaStream_t s, const UnsortFields &F, int64_t n, const int32_t *id, void *records,
+                         int32_t *bands, int32_t *verdict);
+// out[k][i] = in[k][i] of n doubles (out[k] NULL: skipped)
+constexpr int kCopyFields = 9;
+struct CopyFields {
+    const double *in[kCopyFields];
+    double *out[kCopyFields];
+};
+int launch_copy_fields(cudaStream_t s, const CopyFields &F, int64_t n);
 // markers in the caller's order (FP64, or FP32 when f32) -> cell keys; -> sorted device order
 int launch_keys_in(cudaStream_t s, const GridView &G, const void *x, const void *y, int64_t n, bool f32,
                    int32_t *key);

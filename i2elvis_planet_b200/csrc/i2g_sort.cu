@@ -337,6 +337,145 @@ __global__ void k_unsort_f64(int64_t n, const int32_t *__restrict__ id, const do
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) out[id[j]] = in[j];
 }
 
+// ------------------------------------------------------------- state read-out
+// Device arrays in the caller's order from the marker storage (i2g_get_markers_dev),
+// every asked field in one pass.  Bound by memory: 8 B read and 8 B written per
+// marker and field, plus the index once.
+//   direct  out[id[j]] = in[j] for every field.  Right while neighbours in storage
+//           are neighbours in the caller's order (their stores fill whole sectors
+//           in L2) or the outputs fit L2.
+//   staged  first into bands of 2048 caller indices, each marker as one 48-byte
+//           record (its fields and its index) at the next place of its band, then
+//           each band through shared memory into the fields.  A caller order
+//           unrelated to the cells makes every 8-byte store of the direct form a
+//           request and a partial sector of its own; a record is written by three
+//           neighbouring lanes, and a band's open sectors fill in L2.
+// k_unsort_sample decides between the two on the device, from the index distances
+// of 4096 neighbours in storage.
+__global__ void __launch_bounds__(1024) k_unsort_sample(int64_t n, const int32_t *__restrict__ id,
+                                                        int32_t *__restrict__ scattered)
+{
+    __shared__ int far;
+    if (threadIdx.x == 0) far = 0;
+    __syncthreads();
+    const int64_t step = (n - 1) / 4096, near = n / 64;
+    int c = 0;
+    for (int k = 0; k < 4; k++) {
+        const int64_t j = (threadIdx.x * 4 + k) * step;
+        const int64_t d = (int64_t)id[j + 1] - id[j];
+        c += (d < 0 ? -d : d) > near;
+    }
+    atomicAdd(&far, c);
+    __syncthreads();
+    if (threadIdx.x == 0) *scattered = far > 2048;
+}
+
+// skip: NULL, or the sample's verdict that makes this kernel leave the work to the staged pair
+__global__ void __launch_bounds__(256) k_unsort_fields(const __grid_constant__ UnsortFields F, int64_t n,
+                                                       const int32_t *__restrict__ id,
+                                                       const int32_t *__restrict__ skip)
+{
+    if (skip && *skip) return;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
+        const int32_t i = id[j];
+        double v[kUnsortFields];
+#pragma unroll
+        for (int k = 0; k < kUnsortFields; k++)
+            if (F.out[k]) v[k] = F.in[k][j];
+#pragma unroll
+        for (int k = 0; k < kUnsortFields; k++)
+            if (F.out[k]) F.out[k][i] = v[k];
+    }
+}
+
+// A band holds exactly its 2048 indices' records, so its room needs no count.
+constexpr int kBand = 2048;
+constexpr int kBandStride = 8;  // ints between two bands' counters (a sector each)
+__global__ void __launch_bounds__(256) k_unsort_bands(const __grid_constant__ UnsortFields F, int64_t n,
+                                                      const int32_t *__restrict__ id, double2 *__restrict__ rec,
+                                                      int32_t *__restrict__ used, const int32_t *__restrict__ go)
+{
+    __shared__ double2 buf[8][96];
+    if (!*go) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t j0 = (int64_t)blockIdx.x * blockDim.x + w * 32; j0 < n; j0 += stride) {
+        const int64_t j = j0 + lane;
+        int64_t at = -1;
+        if (j < n) {
+            const int32_t i = id[j];
+            const int b = i / kBand;
+            at = (int64_t)b * kBand + atomicAdd(used + (int64_t)b * kBandStride, 1);
+            double v[6];
+#pragma unroll
+            for (int k = 0; k < kUnsortFields; k++) v[k] = F.out[k] ? F.in[k][j] : 0.0;
+            v[5] = __hiloint2double(0, i);
+#pragma unroll
+            for (int k = 0; k < 3; k++) buf[w][3 * lane + k] = make_double2(v[2 * k], v[2 * k + 1]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const int q = 32 * k + lane, r = q / 3;
+            const int64_t d = __shfl_sync(0xffffffffu, at, r);
+            if (d >= 0) rec[3 * d + (q - 3 * r)] = buf[w][q];
+        }
+        __syncwarp();
+    }
+}
+
+struct BandSmem {
+    double v[kUnsortFields][kBand];
+};
+__global__ void __launch_bounds__(512) k_unsort_place(const __grid_constant__ UnsortFields F, int64_t n,
+                                                      const double2 *__restrict__ rec,
+                                                      const int32_t *__restrict__ go)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    BandSmem &S = *reinterpret_cast<BandSmem *>(smraw);
+    if (!*go) return;
+    const int nb = (int)((n + kBand - 1) / kBand);
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+        const int64_t i0 = (int64_t)b * kBand;
+        const int m = (int)(n - i0 < kBand ? n - i0 : kBand);
+        for (int q = threadIdx.x; q < m; q += blockDim.x) {
+            double v[6];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const double2 u = __ldcs(rec + 3 * (i0 + q) + k);
+                v[2 * k] = u.x;
+                v[2 * k + 1] = u.y;
+            }
+            const int i = __double2loint(v[5]) - (int)i0;
+#pragma unroll
+            for (int k = 0; k < kUnsortFields; k++) S.v[k][i] = v[k];
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < m; q += blockDim.x)
+#pragma unroll
+            for (int k = 0; k < kUnsortFields; k++)
+                if (F.out[k]) F.out[k][i0 + q] = S.v[k][q];
+        __syncthreads();
+    }
+}
+
+// node fields into the caller's device arrays, all of them in one launch; W
+// doubles per access
+template <class W>
+__global__ void __launch_bounds__(256) k_copy_fields(const __grid_constant__ CopyFields F, int64_t n)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    W v[kCopyFields];
+#pragma unroll
+    for (int k = 0; k < kCopyFields; k++)
+        if (F.out[k]) v[k] = reinterpret_cast<const W *>(F.in[k])[i];
+#pragma unroll
+    for (int k = 0; k < kCopyFields; k++)
+        if (F.out[k]) reinterpret_cast<W *>(F.out[k])[i] = v[k];
+}
+
 // cell keys of markers in the caller's order, from FP64 or FP32 (reference storage)
 // coordinates; an FP32 coordinate enters as the double it widens to
 template <class R>
@@ -558,6 +697,46 @@ int launch_unsort_f64(cudaStream_t s, int64_t n, const int32_t *id, const double
 {
     if (n <= 0) return 0;
     k_unsort_f64<<<blocks_for(n, 256, 148 * 16), 256, 0, s>>>(n, id, in, out);
+    return 1;
+}
+
+// The staged form moves 96 B per marker besides the fields, so it needs three
+// fields or more, and outputs beyond what L2 holds (kUnsortDirectBytes): five
+// fields in a random order take 52 us direct, 114 staged at 1.44M markers (58 MB)
+// and 235 against 153 at 2.56M (102 MB), 3.9 against 1.6 ms at 36M, where a pass
+// and a copy per field took 7.3 ms.  In cell order direct takes 0.51 ms there
+// (5.9 TB/s).
+int launch_unsort_fields(cudaStream_t s, const UnsortFields &F, int64_t n, const int32_t *id, void *records,
+                         int32_t *bands, int32_t *verdict)
+{
+    if (n <= 0) return 0;
+    int nf = 0;
+    for (int k = 0; k < kUnsortFields; k++) nf += F.out[k] != nullptr;
+    if (nf < 3 || n * nf * (int64_t)sizeof(double) <= kUnsortDirectBytes) {
+        k_unsort_fields<<<blocks_for(n, 256, INT32_MAX), 256, 0, s>>>(F, n, id, nullptr);
+        return 1;
+    }
+    static unsigned long long attr = 0;
+    allow_dynamic_smem((const void *)k_unsort_place, (int)sizeof(BandSmem), &attr);
+    const int64_t nbands = (n + kBand - 1) / kBand;
+    cudaMemsetAsync(bands, 0, sizeof(int32_t) * kBandStride * nbands, s);
+    k_unsort_sample<<<1, 1024, 0, s>>>(n, id, verdict);
+    k_unsort_fields<<<blocks_for(n, 256, 148 * 32), 256, 0, s>>>(F, n, id, verdict);
+    k_unsort_bands<<<blocks_for(n, 256, 148 * 32), 256, 0, s>>>(F, n, id, static_cast<double2 *>(records), bands,
+                                                               verdict);
+    k_unsort_place<<<blocks_for(n, kBand, 148 * 2), 512, sizeof(BandSmem), s>>>(
+        F, n, static_cast<const double2 *>(records), verdict);
+    return 4;
+}
+
+int launch_copy_fields(cudaStream_t s, const CopyFields &F, int64_t n)
+{
+    uintptr_t a = 0;
+    for (int k = 0; k < kCopyFields; k++) a |= (uintptr_t)F.out[k] | (F.out[k] ? (uintptr_t)F.in[k] : 0);
+    if ((a & 15) == 0 && n % 2 == 0)
+        k_copy_fields<double2><<<blocks_for(n / 2, 256, INT32_MAX), 256, 0, s>>>(F, n / 2);
+    else
+        k_copy_fields<double><<<blocks_for(n, 256, INT32_MAX), 256, 0, s>>>(F, n);
     return 1;
 }
 
