@@ -1986,16 +1986,17 @@ int i2g_adjoint_setup(i2g_ctx *c, int32_t nmodes, const double *mode_vx, const d
         TRY(dalloc(c, &A.dT, c->cap));
         TRY(dalloc(c, &A.type_by_id, c->cap));
         TRY(dalloc(c, &A.lam, c->cap));
-        A.nblk = (int32_t)std::min<int64_t>((c->cap + 127) / 128, 148 * 8);
+        A.nblk = (int32_t)std::min<int64_t>((c->cap + 127) / 128, 148 * 64);
         if (A.nblk < 1) A.nblk = 1;
         TRY(dalloc(c, &A.dapart, (int64_t)A.nblk * kMaxModes));
     }
     // interleave to [node][mode] so one stencil corner reads every mode at once
-    std::vector<double> hx((size_t)(nn * nmodes)), hy((size_t)(nn * nmodes));
+    const int ld = mode_capacity(nmodes);
+    std::vector<double> hx((size_t)(nn * ld), 0.0), hy((size_t)(nn * ld), 0.0);
     for (int32_t m = 0; m < nmodes; m++)
         for (int64_t i = 0; i < nn; i++) {
-            hx[(size_t)(i * nmodes + m)] = mode_vx[(size_t)(m * nn + i)];
-            hy[(size_t)(i * nmodes + m)] = mode_vy[(size_t)(m * nn + i)];
+            hx[(size_t)(i * ld + m)] = mode_vx[(size_t)(m * nn + i)];
+            hy[(size_t)(i * ld + m)] = mode_vy[(size_t)(m * nn + i)];
         }
     CK(cudaMemcpyAsync(A.mvx, hx.data(), sizeof(double) * hx.size(), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(A.mvy, hy.data(), sizeof(double) * hy.size(), cudaMemcpyHostToDevice, c->stream));
@@ -2022,7 +2023,7 @@ int i2g_adjoint_forward(i2g_ctx *c, const double *amps, int32_t nsteps, double t
         A.ck_segs = nseg;
     }
     CK(cudaMemcpyAsync(A.amps, amps, sizeof(double) * A.nm, cudaMemcpyHostToDevice, c->stream));
-    c->launches += launch_combine_modes(c->stream, c->nn, A.nm, A.mvx, A.mvy, A.amps, c->g[G_VX], c->g[G_VY],
+    c->launches += launch_combine_modes(c->stream, c->nn, A.nm, mode_capacity(A.nm), A.mvx, A.mvy, A.amps, c->g[G_VX], c->g[G_VY],
                                         c->vxf, c->vyf);
     if (c->vxf) {
         c->launches += launch_quads(c->stream, c->nx, c->ny, c->vxf, c->vxq);

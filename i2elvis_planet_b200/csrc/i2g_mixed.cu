@@ -114,9 +114,9 @@ int launch_adjoint_mixed(const StepLaunch &L, const MoveArgs &A, const AdjLaunch
     if (n <= 0) return 0;
     k_adj_avg<true><<<grid_for(n, 256, 148 * 16), 256, 0, L.stream>>>(L.G, L.M, L.types, J.gridmod, J.tmp_ambient, J.tk,
                                                                   J.w1, J.g, J.T0, J.lam, J.dT);
-    AdjView Md{J.mvx, J.mvy, J.nmodes};
-    k_adj_rk4<true><<<J.nblk, 128, 0, L.stream>>>(L.G, Md, A, L.types, J.type_by_id, J.ck, n, J.nsteps, J.every,
-                                               J.lam, J.dapart);
+    AdjView Md{J.mvx, J.mvy};
+    launch_adj_rk4<true>(L.stream, L.G, Md, A, L.types, n, J.nmodes, J.type_by_id, J.ck, J.nsteps, J.every, J.lam,
+                       J.dapart, J.nblk);
     return 2;
 }
 

@@ -563,7 +563,7 @@ __global__ void k_t0(GridView G, MarkerView M, const int64_t *__restrict__ slot0
 }
 
 // ------------------------------------------------------------- adjoint helpers
-__global__ void k_combine_modes(int64_t nn, int32_t nm, const double *__restrict__ mvx,
+__global__ void k_combine_modes(int64_t nn, int32_t nm, int32_t ld, const double *__restrict__ mvx,
                                 const double *__restrict__ mvy, const double *__restrict__ amps,
                                 double *__restrict__ vx, double *__restrict__ vy, float *__restrict__ vxf,
                                 float *__restrict__ vyf)
@@ -572,8 +572,8 @@ __global__ void k_combine_modes(int64_t nn, int32_t nm, const double *__restrict
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += stride) {
         double a = 0.0, b = 0.0;
         for (int m = 0; m < nm; m++) {
-            a += amps[m] * mvx[i * nm + m];
-            b += amps[m] * mvy[i * nm + m];
+            a += amps[m] * mvx[i * ld + m];
+            b += amps[m] * mvy[i * ld + m];
         }
         vx[i] = a;
         vy[i] = b;
@@ -589,14 +589,16 @@ __global__ void k_ckpt(MarkerView M, double2 *__restrict__ ck)
         ck[M.id[j]] = make_double2(M.x[j], M.y[j]);
 }
 
-// out[m] = sum over blocks b in order of part[b][m]
+// out[m] = sum over blocks b of part[b][m]: a warp per mode, lane l the blocks l,
+// l + 32, ... in order, then the lanes in a fixed tree
 __global__ void k_sum_partials(const double *__restrict__ part, int32_t nblk, int32_t nm, double *__restrict__ out)
 {
-    const int m = threadIdx.x;
+    const int m = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (m >= nm) return;
     double s = 0.0;
-    for (int32_t b = 0; b < nblk; b++) s += part[(int64_t)b * nm + m];
-    out[m] = s;
+    for (int32_t b = lane; b < nblk; b += 32) s += part[(int64_t)b * nm + m];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) out[m] = s;
 }
 
 // ------------------------------------------------------------- host launchers
@@ -877,10 +879,10 @@ int launch_quarters(cudaStream_t s, int64_t nx, int64_t ny, const float *vxf, co
     return 1;
 }
 
-int launch_combine_modes(cudaStream_t s, int64_t nn, int32_t nm, const double *mvx, const double *mvy,
+int launch_combine_modes(cudaStream_t s, int64_t nn, int32_t nm, int32_t ld, const double *mvx, const double *mvy,
                          const double *amps, double *vx, double *vy, float *vxf, float *vyf)
 {
-    k_combine_modes<<<blocks_for(nn, 256, 148 * 16), 256, 0, s>>>(nn, nm, mvx, mvy, amps, vx, vy, vxf, vyf);
+    k_combine_modes<<<blocks_for(nn, 256, 148 * 16), 256, 0, s>>>(nn, nm, ld, mvx, mvy, amps, vx, vy, vxf, vyf);
     return 1;
 }
 
@@ -893,7 +895,7 @@ int launch_ckpt(cudaStream_t s, const MarkerView &M, double2 *ck)
 
 int launch_sum_partials(cudaStream_t s, const double *part, int32_t nblk, int32_t nm, double *out)
 {
-    k_sum_partials<<<1, 32, 0, s>>>(part, nblk, nm, out);
+    k_sum_partials<<<1, 32 * nm, 0, s>>>(part, nblk, nm, out);
     return 1;
 }
 
