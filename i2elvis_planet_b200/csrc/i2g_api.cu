@@ -109,7 +109,7 @@ struct i2g_ctx {
     struct Fused {
         bool enabled = true;         // i2g_set_fused
         int32_t cap = 0;             // places per cell bucket; 0 = buckets not allocated
-        float4 *ra = nullptr;        // [ncells * cap] 16-byte records
+        float4 *ra = nullptr;        // 16-byte records (rec_place)
         OvfRec *ovf = nullptr;       // [max_markers]
         FusedCounters *ctr = nullptr;
         int32_t *treset = nullptr;   // [max_markers]
@@ -382,9 +382,10 @@ int fused_buckets(i2g_ctx *c, int32_t count_max)
     c->fz.cap = 0;
     // too large for the fused path: the places must fit an int32, and the cell
     // sums are exact only for fewer than 2^19 records in a cell (k_cellnodes)
-    if (c->ncells * cap >= (int64_t)INT32_MAX || count_max >= (1 << 18)) return I2G_OK;
+    const int64_t places = (c->ncells + 31) / 32 * 32 * cap;  // strips of 32 cells (rec_place)
+    if (places >= (int64_t)INT32_MAX || count_max >= (1 << 18)) return I2G_OK;
     if (alloc_injected(c)) return fail(c, I2G_ENOMEM, "fused buckets: injected failure (I2G_FAIL_ALLOC_AT)");
-    cudaError_t e = cudaMalloc((void **)&c->fz.ra, sizeof(float4) * (size_t)(c->ncells * cap) + 64);
+    cudaError_t e = cudaMalloc((void **)&c->fz.ra, sizeof(float4) * (size_t)places);
     if (e != cudaSuccess) {
         cudaGetLastError();
         c->fz.ra = nullptr;

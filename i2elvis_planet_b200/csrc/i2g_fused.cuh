@@ -14,10 +14,9 @@
 //                  (ncells x cap places; a full bucket spills to an overflow
 //                  list).  No sort: the markers stay where they are.
 //   k_cellnodes    a CTA per tile of 31 x (8G - 1) nodes: a warp per cell column,
-//                  a lane per cell, each lane adds its cell's records into
-//                  per-slot sums and forms its corner sums, the warps exchange
-//                  the halves of every node's sum in shared memory, and the nodes
-//                  are finished in place.
+//                  a lane per cell (two on small grids), each lane adds its cell's
+//                  records into per-slot sums; the cells' sums meet in shared
+//                  memory, where a thread per node finishes it.
 //
 // Order independence.  The records arrive in their buckets in whatever order the
 // atomics grant, so every sum is made exact, and exact sums do not depend on the
@@ -60,9 +59,9 @@ struct OvfRec {
 
 struct FusedMove {
     AvgArgsK avg;                // the averaging's constants
-    uint8_t tinfo[kAvgTypes];    // per rock type: bits 0-1 type slot, bit 2 immobile
+    uint8_t type[kAvgTypes];     // per rock type: rec_type_byte
     int32_t cap;                 // places per bucket
-    float4 *ra;                  // [ncells * cap] the records (rec_pack)
+    float4 *ra;                  // [cells, whole strips of 32, * cap] the records (rec_pack, rec_place)
     OvfRec *ovf;                 // [markers]
     int32_t *count;              // [ncells] records per cell (zeroed before the launch)
     FusedCounters *ctr;          // part/novf/ntreset zeroed before the launch
@@ -227,15 +226,24 @@ __device__ __forceinline__ unsigned lane_lt()
     return m;
 }
 
-// The 16-byte averaging record {x word, y word, T, type word}:
-//   x word: w1 of x in [0, 1] as fixed point w1 2^24 (bits 0-24), log-viscosity bits 21-27 (25-31)
-//   y word: w1 of y likewise (bits 0-24), log-viscosity bits 28-34 (25-31)
+// The 16-byte averaging record {x word, y word, T, log-viscosity word}:
+//   x word: w1 of x in [0, 1] as fixed point w1 2^24 (bits 0-24), log-viscosity bits 25-31 (25-31)
+//   y word: w1 of y likewise (bits 0-24), log-viscosity bits 21-24 (25-28), immobile
+//           (bit 29), type slot (bits 30-31)
 //   T: the marker temperature, FP32
-//   type word: type slot (bits 0-1), immobile (bit 2), log-viscosity bits 35-63 (3-31)
+//   the last word: log-viscosity bits 32-63
 // The log-viscosity is rounded to its 43 leading bits (sign, exponent, 31
 // fraction bits: 2.3e-10 of itself); the cell sums turn w1 back into an FP64
-// number with one FMA, and w0 = 1 - w1 exactly there.
+// number with one FMA, exactly, and take every field apart with at most three
+// bit operations.
 constexpr uint32_t kWeightMask = 0x1FFFFFFu;
+constexpr uint32_t kRecImmobile = 1u << 29;
+constexpr int kRecSlotShift = 30;
+// tinfo[] of a rock type (slot | immobile << 2) as the y word's top byte has it
+__host__ __device__ constexpr uint8_t rec_type_byte(uint8_t tinfo)
+{
+    return (uint8_t)((tinfo & 3u) << 6 | (tinfo & 4u) << 3);
+}
 __device__ __forceinline__ uint32_t weight_fix(double w)
 {
     w = w < 0.0 ? 0.0 : (w > 1.0 ? 1.0 : w);
@@ -251,21 +259,32 @@ __device__ __forceinline__ float4 rec_with_lnu(float4 r, double lnu)
 {
     const unsigned long long b = (unsigned long long)__double_as_longlong(lnu) + (1ull << 20);
     const uint32_t lo = (uint32_t)b, hi = (uint32_t)(b >> 32);
-    const uint32_t x = (__float_as_uint(r.x) & kWeightMask) | ((lo >> 21) << 25);
-    const uint32_t y = (__float_as_uint(r.y) & kWeightMask) | (((lo >> 28) | (hi << 4)) << 25);
-    const uint32_t w = (__float_as_uint(r.w) & 7u) | (hi & ~7u);
-    return make_float4(__uint_as_float(x), __uint_as_float(y), r.z, __uint_as_float(w));
+    const uint32_t x = (__float_as_uint(r.x) & kWeightMask) | (lo & ~kWeightMask);
+    const uint32_t y = (__float_as_uint(r.y) & ~0x1E000000u) | ((lo << 4) & 0x1E000000u);
+    return make_float4(__uint_as_float(x), __uint_as_float(y), r.z, __uint_as_float(hi));
 }
-__device__ __forceinline__ float4 rec_pack(uint32_t wx, uint32_t wy, float tk, uint32_t tinfo, double lnu)
+// type: the rock type's rec_type_byte
+__device__ __forceinline__ float4 rec_pack(uint32_t wx, uint32_t wy, float tk, uint32_t type, double lnu)
 {
-    return rec_with_lnu(make_float4(__uint_as_float(wx), __uint_as_float(wy), tk, __uint_as_float(tinfo)), lnu);
+    return rec_with_lnu(make_float4(__uint_as_float(wx), __uint_as_float(wy | type << 24), tk, 0.f), lnu);
+}
+__device__ __forceinline__ double rec_lnu(uint32_t x, uint32_t y, uint32_t w)
+{
+    return __hiloint2double((int)w, (int)((x & ~kWeightMask) | ((y >> 4) & 0x01E00000u)));
 }
 __device__ __forceinline__ double rec_lnu(float4 r)
 {
-    const uint32_t x = __float_as_uint(r.x), y = __float_as_uint(r.y), w = __float_as_uint(r.w);
-    const uint32_t lo = ((x >> 25) << 21) | (((y >> 25) & 0xFu) << 28);
-    const uint32_t hi = (w & ~7u) | (y >> 29);
-    return __hiloint2double((int)hi, (int)lo);
+    return rec_lnu(__float_as_uint(r.x), __float_as_uint(r.y), __float_as_uint(r.w));
+}
+__device__ __forceinline__ int rec_slot(float4 r) { return (int)(__float_as_uint(r.y) >> kRecSlotShift); }
+__device__ __forceinline__ bool rec_immobile(float4 r) { return (__float_as_uint(r.y) & kRecImmobile) != 0; }
+
+// The place of record `slot` of a cell's bucket: buckets of 32 consecutive cells are
+// interleaved by pairs of records (a 32-byte sector), so that a warp that reads the
+// same pair of 32 neighbouring cells reads 1 KB in a row.  cap is even.
+__host__ __device__ __forceinline__ int32_t rec_place(int32_t cell, int32_t slot, int32_t cap)
+{
+    return (cell >> 5) * (cap << 5) + ((slot >> 1) << 6) + ((cell & 31) << 1) + (slot & 1);
 }
 
 // the log-viscosity of a record from the marker's viscosity (the radmax override
@@ -376,7 +395,7 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
         // viscalc in k_fused_deferred (a place is kept for it here)
         lnu = eta > 0 ? record_lnu(G, V, x, y, eta) : 0.0;
         defer = !(eta > 0);
-        rec = rec_pack(weight_fix(wx1), weight_fix(wy1), (float)mtk, (uint32_t)F.tinfo[mt], lnu);
+        rec = rec_pack(weight_fix(wx1), weight_fix(wy1), (float)mtk, (uint32_t)F.type[mt], lnu);
     }
     uint32_t cnt = 0;
     if (ok) {
@@ -385,9 +404,8 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
         cnt = (uint32_t)slot + 1u;
         int32_t place;  // bucket place, or -(overflow index + 1)
         if (slot < F.cap) {
-            const int64_t at = (int64_t)key * F.cap + slot;
-            F.ra[at] = rec;
-            place = (int32_t)at;
+            place = rec_place(key, slot, F.cap);
+            F.ra[place] = rec;
         } else {
             const int32_t o = atomicAdd(&F.ctr->novf, 1);
             OvfRec r;
@@ -531,12 +549,18 @@ __global__ void __launch_bounds__(128) k_fused_deferred(const __grid_constant__ 
 }
 
 // ----------------------------------------------------------------- sums and nodes
-// The rounding of one averaging call, derived from the counters.  A term t of a
-// sum is replaced by fma(a, b, c) - c = t rounded to the nearest multiple of the
-// sum's quantum q = 2^(e - 52), c = 1.5 * 2^e, where 2^e exceeds the largest
-// magnitude any node's sum can reach (4 x the largest cell count x the largest
-// |term|): every partial sum is then an integer multiple of q below 2^52 q, an
-// exact FP64 number, whatever the order of the additions.
+// The rounding of one averaging call, derived from the counters: two ways to add
+// terms in FP64 so that the sum does not depend on their order.
+//   quant   a term t becomes fma(a, b, c) - c, t rounded to the nearest multiple of
+//           the quantum q = 2^(e - 52), c = 1.5 * 2^e, where 2^e exceeds the largest
+//           magnitude any node's sum can reach (4 x the largest cell count x the
+//           largest |term|): every partial sum is an integer multiple of q below
+//           2^52 q, an exact FP64 number.  Opposite terms stay opposite.
+//   floors  the sum starts at c / 2 and takes each term as fma(a, b, sum) rounded
+//           down: it stays in its binade (a cell's sum is at most a quarter of a
+//           node's), so every term adds its floor to a multiple of q / 2, whatever
+//           came before it (to the nearest, ties would depend on that).  One FP64
+//           operation per term.
 struct QConst {
     double cw, ctk, cnu;  // weights, temperature x weight, log-viscosity x weight
     // a node goes to k_node_guard where a weight sum is below thr_w (thr_nuw for
@@ -548,8 +572,9 @@ struct QConst {
 __device__ __forceinline__ QConst qconst_of(uint32_t cmax, uint32_t tkb, uint32_t lnb, int viscmod)
 {
     QConst Q;
-    // weights are FP32 in [0, 1] up to a rounding: bound them by 1 + 2^-20
-    const double Nn = 4.0 * (double)(cmax > 0 ? cmax : 1u), Sw = Nn * (1.0 + 0x1p-20);
+    // weights are in [-1, 1]; up to Nn terms reach a node (at least 4 a cell: the
+    // cell sums run whole batches)
+    const double Nn = 4.0 * (double)(cmax > 4u ? cmax : 4u), Sw = Nn * (1.0 + 0x1p-20);
     const double Mtk = (double)__uint_as_float(tkb), Mnu = (double)__uint_as_float(lnb);
     const double Stk = Sw * Mtk, Snu = Sw * Mnu;
     const int ew = ilogb(Sw) + 1, etk = Stk > 0 ? ilogb(Stk) + 1 : 0, enu = Snu > 0 ? ilogb(Snu) + 1 : 0;
@@ -563,7 +588,7 @@ __device__ __forceinline__ QConst qconst_of(uint32_t cmax, uint32_t tkb, uint32_
     // is the relative error of the node value.
     const double qw = ldexp(1.0, ew - 52), qtk = ldexp(1.0, etk - 52), qnu = ldexp(1.0, enu - 52);
     Q.thr_w = Nn * qw / 2e-9;
-    Q.vtk = 4.0 * Nn * qtk / 2e-9;  // a corner's T term combines four quantized sums
+    Q.vtk = 4.0 * Nn * qtk / 2e-9;
     if (viscmod == 1) {
         Q.thr_nuw = Nn * (qnu + qw * Mnu) / 2e-9;
         Q.vnu = 0.0;
@@ -603,123 +628,212 @@ __device__ __forceinline__ QConst block_qconst(const FusedCounters *ctr, int vis
     return sq;
 }
 
-__device__ __forceinline__ double quant(double a, double b, double c) { return fma(a, b, c) - c; }
-
-// The sums of one cell.  A record's corner weights are the products X0 Y0,
-// X0 Y1, X1 Y0, X1 Y1 of its axis weights (X0 = 1 - X1, Y0 = 1 - Y1), so the
-// cell keeps, per type slot, the record count and the sums of X1, Y1 and X1 Y1
-// (quantized), and for the mobile records T, T X1, T Y1 and T X1 Y1
-// (quantized); acc_corners turns them into the four corner sums, exactly.  The
-// node viscosity goes to the nearest node with the quadrant weight, the
-// cell-centre one with the tent weight.
+// The sums of one cell.  With x = 2 X1 - 1, y = 2 Y1 - 1 in [-1, 1] a record's
+// corner weights are (1 -+ x)(1 -+ y) / 4, so a cell needs, per type slot, the record
+// count and the sums of x, y and x y, and for the mobile records T, T x, T y and
+// T x y; corner4 turns them into the sums at a corner.  The node viscosity goes to
+// the nearest node with the quadrant weight |x y|, the cell-centre one with the tent
+// weight (1 - |x|)(1 - |y|).
+//
+// No sum is picked per record (a predicated FP64 add became two selects): sums over a
+// part of the records come from sums with signs.  With s1, s2 = -1 where bit 0, 1 of
+// the slot is set, else 1, the sums of f, s1 f and s2 f (and s1 s2 f with four slots)
+// give every slot's, and those of t, sx t, sy t and sx sy t (sx, sy the signs of x, y)
+// every quadrant's, exactly, for quantized f and t.
 template <int NT>
 struct CellAcc {
-    int32_t n[NT];
-    double sx[NT], sy[NT], sxy[NT];
-    double t0, tx, ty, txy;
-    double nu[4], wnu[4];
-    double nd, wnd;
+    static constexpr int B = NT == 1 ? 0 : (NT == 2 ? 1 : (NT == 3 ? 2 : 3));  // signed copies of the slot sums
+    int32_t m[B + 1];                      // records with bit 0, bit 1, both bits set (B of them)
+    double x[B + 1], y[B + 1], p[B + 1];   // x, y, x y (quantized): plain, s1, s2, s1 s2
+    double w, wx, wy;                      // |x y| plain, sx, sy (sx sy: p[0])
+    double n[4];                           // log-viscosity x |x y| (quantized): plain, sx, sy, sx sy
+    double t0, tx, ty, txy, nd, wnd;       // sums of floors
 };
 
 template <int NT>
-__device__ __forceinline__ void acc_zero(CellAcc<NT> &a)
+__device__ __forceinline__ void acc_start(CellAcc<NT> &a, const QConst &Q)
 {
 #pragma unroll
-    for (int k = 0; k < NT; k++) {
-        a.n[k] = 0;
-        a.sx[k] = a.sy[k] = a.sxy[k] = 0.0;
+    for (int k = 0; k <= CellAcc<NT>::B; k++) {
+        a.m[k] = 0;
+        a.x[k] = a.y[k] = a.p[k] = 0.0;
     }
-    a.t0 = a.tx = a.ty = a.txy = 0.0;
+    a.w = a.wx = a.wy = 0.0;
 #pragma unroll
-    for (int q = 0; q < 4; q++) a.nu[q] = a.wnu[q] = 0.0;
-    a.nd = a.wnd = 0.0;
+    for (int k = 0; k < 4; k++) a.n[k] = 0.0;
+    a.t0 = a.tx = a.ty = a.txy = 0.5 * Q.ctk;
+    a.nd = 0.5 * Q.cnu;
+    a.wnd = 0.5 * Q.cw;
 }
 
-// One record into its cell's sums (markmart.c:859-913): weights from the
-// record's fixed-point X1, Y1 (exact in FP64, as are X1 - 1/2 and 1 - X1);
-// every product rounded to its sum's quantum.
-template <int NT>
-__device__ __forceinline__ void acc_rec(CellAcc<NT> &a, float4 r, const QConst &Q)
+// +-1.0 with the sign bit of word b
+__device__ __forceinline__ double unit_of(uint32_t b)
 {
-    const double lnu = rec_lnu(r);
-    const double X1 = weight_of(__float_as_uint(r.x)), Y1 = weight_of(__float_as_uint(r.y));
-    const double p = quant(X1, Y1, Q.cw);
-    const uint32_t tf = __float_as_uint(r.w);
-    const int slot = (int)(tf & 3u);
+    return __hiloint2double((int)((b & 0x80000000u) | 0x3FF00000u), 0);
+}
+
+// One record into its cell's sums (markmart.c:859-913): 33 FP64 operations with three
+// slots.
+template <int NT>
+__device__ __forceinline__ void acc_rec(CellAcc<NT> &a, uint4 u, const QConst &Q)
+{
+    constexpr int B = CellAcc<NT>::B;
+    // (2^52 + X) 2^-23 - 2^29 - 1 = 2 X1 - 1, exactly
+    const double x = fma(__hiloint2double(0x43300000, (int)(u.x & kWeightMask)), 0x1p-23, -(0x1p29 + 1.0));
+    const double y = fma(__hiloint2double(0x43300000, (int)(u.y & kWeightMask)), 0x1p-23, -(0x1p29 + 1.0));
+    const double xy = x * y;  // 24 x 24 bits: exact
+    const double p = (xy + Q.cw) - Q.cw;
+    a.x[0] += x;
+    a.y[0] += y;
+    a.p[0] += p;
 #pragma unroll
-    for (int k = 0; k < NT; k++) {
-        const double oh = (slot == k) ? 1.0 : 0.0;
-        a.n[k] += slot == k ? 1 : 0;
-        a.sx[k] = fma(oh, X1, a.sx[k]);
-        a.sy[k] = fma(oh, Y1, a.sy[k]);
-        a.sxy[k] = fma(oh, p, a.sxy[k]);
+    for (int k = 1; k <= B; k++) {
+        const uint32_t bit = k == 1 ? u.y << 1 : (k == 2 ? u.y : u.y & (u.y << 1));
+        a.m[k - 1] += (int32_t)(bit >> 31);
+        const double s = unit_of(k < 3 ? bit : u.y ^ (u.y << 1));
+        a.x[k] = fma(s, x, a.x[k]);
+        a.y[k] = fma(s, y, a.y[k]);
+        a.p[k] = fma(s, p, a.p[k]);
     }
-    if (!(tf & 4u)) {  // mobile type: temperature
-        const double tk = (double)r.z;
-        a.t0 += quant(tk, 1.0, Q.ctk);
-        a.tx += quant(tk, X1, Q.ctk);
-        a.ty += quant(tk, Y1, Q.ctk);
-        a.txy += quant(tk * X1, Y1, Q.ctk);
-    }
+    // the temperature of mobile types
+    const double tk = (double)__uint_as_float(u.y & kRecImmobile ? 0u : u.z), tkx = tk * x;  // 24 x 24 bits: exact
+    a.t0 = __dadd_rd(a.t0, tk);
+    a.tx = __dadd_rd(a.tx, tkx);
+    a.ty = __fma_rd(tk, y, a.ty);
+    a.txy = __fma_rd(tkx, y, a.txy);
     // the nearest node takes the viscosity with the quadrant weight
-    // 4 (wa - 1/2)(wb - 1/2), wa = max(X0, X1) = 1/2 + |X1 - 1/2| (both weights
-    // above one half: at most one corner)
-    const double ax = X1 - 0.5, ay = Y1 - 0.5, fx = fabs(ax), fy = fabs(ay);
-    if (fx > 0.0 && fy > 0.0) {
-        const double s2 = 4.0 * fx * fy;
-        const double t = quant(lnu, s2, Q.cnu), s2q = quant(s2, 1.0, Q.cw);
-        const int qq = (ax > 0.0 ? 2 : 0) | (ay > 0.0 ? 1 : 0);
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const double oh = (q == qq) ? 1.0 : 0.0;
-            a.nu[q] = fma(oh, t, a.nu[q]);
-            a.wnu[q] = fma(oh, s2q, a.wnu[q]);
-        }
-    }
+    // 4 (wa - 1/2)(wb - 1/2), wa = max(X0, X1) = (1 + |x|) / 2 (zero on a midline)
+    const double lnu = rec_lnu(u.x, u.y, u.w);
+    const uint32_t bx = (uint32_t)__double2hiint(x), by = (uint32_t)__double2hiint(y);
+    const double sx = unit_of(bx), sy = unit_of(by);
+    a.w += fabs(p);
+    a.wx = fma(p, sy, a.wx);  // |x y| sx = x y sy
+    a.wy = fma(p, sx, a.wy);
+    const double t = fma(lnu, fabs(xy), Q.cnu) - Q.cnu;
+    a.n[0] += t;
+    a.n[1] = fma(t, sx, a.n[1]);
+    a.n[2] = fma(t, sy, a.n[2]);
+    a.n[3] = fma(t, unit_of(bx ^ by), a.n[3]);
     // the cell centre takes it with the tent weight 4 (dx - 1/2)(dy - 1/2),
-    // dx = 1 - |X0 - 1/2|, so dx - 1/2 = 1/2 - |X1 - 1/2|
-    const double cx = 0.5 - fx, cy = 0.5 - fy;
-    if (cx > 0.0 && cy > 0.0) {
-        const double s2 = 4.0 * cx * cy;
-        a.nd += quant(lnu, s2, Q.cnu);
-        a.wnd += quant(s2, 1.0, Q.cw);
-    }
+    // dx = 1 - |X0 - 1/2| = 1 - |x| / 2
+    const double c = (1.0 - fabs(x)) * (1.0 - fabs(y));
+    a.nd = __fma_rd(lnu, c, a.nd);
+    a.wnd = __dadd_rd(a.wnd, c);
 }
 
-// The corner sums of a cell (corner q = 2a + b at node (m1 + a, m2 + b)): per
-// slot X0 Y0 = n - X1 - Y1 + X1 Y1, X0 Y1 = Y1 - X1 Y1, X1 Y0 = X1 - X1 Y1,
-// X1 Y1, likewise for T x weight; the mobile weight is the sum over the mobile
-// slots (mob: bit k set when slot k's type moves).  Every term is a multiple of
-// the sums' quanta and every partial sum stays below the quantum's range (the
-// counts are below 2^18), so each is exact.
+// a record whose terms are zero in every sum but wnd (there 1): x = y = T = 0, lnu = 0
+__device__ __forceinline__ uint4 rec_none() { return make_uint4(1u << 23, 1u << 23, 0u, 0u); }
+
+struct RecPair {
+    uint4 a, b;
+};
+__device__ __forceinline__ RecPair rec_pair(const uint4 *p)
+{
+    RecPair r;
+    r.a = __ldcs(p);
+    r.b = __ldcs(p + 1);
+    return r;
+}
+// the pair of records at p of which m (<= 0: none) are there
+__device__ __forceinline__ RecPair rec_pair(const uint4 *p, int m)
+{
+    RecPair r;
+    r.a = r.b = rec_none();
+    if (m > 0) r.a = __ldcs(p);
+    if (m > 1) r.b = __ldcs(p + 1);
+    return r;
+}
+
+// A cell's sums as k_cellnodes keeps them in shared memory: per slot {n, x, y, xy},
+// then {T, T x, T y, T x y}, nu[4], wnu[4], nd, wnd.
 template <int NT>
-__device__ __forceinline__ void acc_corners(const CellAcc<NT> &a, uint32_t mob, double (*wt)[4], double *w1,
-                                            double *tk)
+struct CellSums {
+    static constexpr int T = 4 * NT, NU = T + 4, WNU = NU + 4, ND = WNU + 4, WND = ND + 1, N = WND + 1;
+};
+
+// the sums of S neighbouring lanes, each lane of them the total
+template <int S, class V>
+__device__ __forceinline__ V lanes_sum(V v)
 {
 #pragma unroll
-    for (int q = 0; q < 4; q++) w1[q] = 0.0;
+    for (int o = 1; o < S; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// out(f, value) for every field f of CellSums from a cell's sums over S lanes; n: the
+// cell's records
+template <int NT, int S, class Out>
+__device__ __forceinline__ void acc_finish(CellAcc<NT> &a, const QConst &Q, int32_t n, Out &&out)
+{
+    using C = CellSums<NT>;
+    constexpr int B = CellAcc<NT>::B;
+    int32_t m[3] = {0, 0, 0};
 #pragma unroll
-    for (int k = 0; k < NT; k++) {
-        const double n = (double)a.n[k];
-        wt[k][3] = a.sxy[k];
-        wt[k][2] = a.sx[k] - a.sxy[k];
-        wt[k][1] = a.sy[k] - a.sxy[k];
-        wt[k][0] = ((n - a.sx[k]) - a.sy[k]) + a.sxy[k];
-        if ((mob >> k) & 1u) {
+    for (int k = 0; k < B; k++) m[k] = lanes_sum<S>(a.m[k]);
 #pragma unroll
-            for (int q = 0; q < 4; q++) w1[q] += wt[k][q];
+    for (int f = 0; f < 4; f++) {
+        double v[4] = {0.0, 0.0, 0.0, 0.0};  // the sum and its signed copies
+        if (f == 0) {
+            v[0] = (double)n;
+#pragma unroll
+            for (int k = 1; k <= B; k++) v[k] = k < 3 ? (double)(n - 2 * m[k - 1]) : (double)(n - 2 * (m[0] + m[1] - 2 * m[2]));
+        } else {
+#pragma unroll
+            for (int k = 0; k <= B; k++) v[k] = lanes_sum<S>(f == 1 ? a.x[k] : (f == 2 ? a.y[k] : a.p[k]));
         }
+        if (NT == 1) out(f, v[0]);
+        if (NT == 2) {
+            out(f, 0.5 * (v[0] + v[1]));
+            out(4 + f, 0.5 * (v[0] - v[1]));
+        }
+        if (NT == 3) {  // slots 0, 1, 2: (s1, s2) = (+, +), (-, +), (+, -)
+            out(f, 0.5 * (v[1] + v[2]));
+            out(4 + f, 0.5 * (v[0] - v[1]));
+            out(8 + f, 0.5 * (v[0] - v[2]));
+        }
+        if (NT == 4) {
+            out(f, 0.25 * ((v[0] + v[1]) + (v[2] + v[3])));
+            out(4 + f, 0.25 * ((v[0] - v[1]) + (v[2] - v[3])));
+            out(8 + f, 0.25 * ((v[0] + v[1]) - (v[2] + v[3])));
+            out(12 + f, 0.25 * ((v[0] - v[1]) - (v[2] - v[3])));
+        }
+        if (f == 3) a.p[0] = v[0];
     }
-    tk[3] = a.txy;
-    tk[2] = a.tx - a.txy;
-    tk[1] = a.ty - a.txy;
-    tk[0] = ((a.t0 - a.tx) - a.ty) + a.txy;
+    out(C::T, lanes_sum<S>(a.t0 - 0.5 * Q.ctk));
+    out(C::T + 1, lanes_sum<S>(a.tx - 0.5 * Q.ctk));
+    out(C::T + 2, lanes_sum<S>(a.ty - 0.5 * Q.ctk));
+    out(C::T + 3, lanes_sum<S>(a.txy - 0.5 * Q.ctk));
+    const double n0 = lanes_sum<S>(a.n[0]), n1 = lanes_sum<S>(a.n[1]), n2 = lanes_sum<S>(a.n[2]),
+                 n3 = lanes_sum<S>(a.n[3]);
+    out(C::NU + 0, 0.25 * ((n0 - n1) - (n2 - n3)));
+    out(C::NU + 1, 0.25 * ((n0 - n1) + (n2 - n3)));
+    out(C::NU + 2, 0.25 * ((n0 + n1) - (n2 + n3)));
+    out(C::NU + 3, 0.25 * ((n0 + n1) + (n2 + n3)));
+    const double w0 = lanes_sum<S>(a.w), w1 = lanes_sum<S>(a.wx), w2 = lanes_sum<S>(a.wy), w3 = a.p[0];
+    out(C::WNU + 0, 0.25 * ((w0 - w1) - (w2 - w3)));
+    out(C::WNU + 1, 0.25 * ((w0 - w1) + (w2 - w3)));
+    out(C::WNU + 2, 0.25 * ((w0 + w1) - (w2 + w3)));
+    out(C::WNU + 3, 0.25 * ((w0 + w1) + (w2 + w3)));
+    out(C::ND, lanes_sum<S>(a.nd - 0.5 * Q.cnu));
+    out(C::WND, lanes_sum<S>(a.wnd - 0.5 * Q.cw));
+}
+
+// 4 x the sum at corner q = 2a + b (node (m1 + a, m2 + b)) of a bilinear quadruple
+// {1, x, y, xy} sum; c: distance between the four in memory
+template <int q>
+__device__ __forceinline__ double corner4(const double *v, int c)
+{
+    const double s = v[0], x = v[c], y = v[2 * c], xy = v[3 * c];
+    if (q == 0) return ((s - x) - y) + xy;
+    if (q == 1) return ((s - x) + y) - xy;
+    if (q == 2) return ((s + x) - y) - xy;
+    return ((s + x) + y) + xy;
 }
 
 struct CellNodesArgs {
     int32_t nx, ny, nc1, nc2, cap;
     uint32_t mob;  // bit k set when type slot k's type is mobile (its T is averaged)
-    int32_t ncol;  // node columns per CTA: 8 * groups - 1
+    int32_t ncol;  // node columns per CTA: kCnCols * groups - 1
     int32_t ntx;   // CTAs along x
     const int32_t *count;
     const float4 *ra;
@@ -741,45 +855,11 @@ struct CellNodesArgs {
     unsigned long long *navg;  // averaged markers (the records of the cells a CTA owns)
 };
 
-// values of a node half (the corner sums of one cell column reaching a node column):
-// wt[NT], w1, tk, nu, wnu, then (right halves only) nd, wnd
+// The sums a node is made of: per-slot weights wt[NT], w1, tk, nu, wnu, nd, wnd
 template <int NT>
 struct NodeVals {
-    static constexpr int L = NT + 4, R = NT + 6;
+    static constexpr int N = NT + 6;
 };
-
-// uint4 per staged row: 4 records of 16 B.  Record t of row r sits at place
-// t ^ cn_swz(r): the 8 rows a quarter warp reads at once then fall on 8
-// distinct 16-byte bank groups
-constexpr int kCnRS = 4;
-__device__ __forceinline__ int cn_swz(int row) { return (row >> 1) & 3; }
-
-struct CnWarpBuf {
-    uint4 rec[2][32 * kCnRS];
-    int32_t cb[32], cn[32];
-};
-
-template <int NT>
-struct CnSmem {
-    CnWarpBuf w[8];
-    double hr[2][8][NodeVals<NT>::R][32];  // right halves, double buffered by group
-};
-
-// asynchronous copies of positions [P0, P0 + 4) of the strip's 32 buckets
-__device__ __forceinline__ void cn_stage(const CnWarpBuf &B, uint4 *dst, const float4 *__restrict__ ra, int P0,
-                                         int lane)
-{
-#pragma unroll
-    for (int it = 0; it < 4; it++) {
-        const int e = it * 32 + lane, row = e >> 2, piece = e & 3;
-        const int rec = P0 + piece;
-        const bool valid = rec < B.cn[row];
-        const uint4 *src = reinterpret_cast<const uint4 *>(ra);
-        if (valid) src = reinterpret_cast<const uint4 *>(ra + (int64_t)B.cb[row] + rec);
-        cp_async16(dst + row * kCnRS + (piece ^ cn_swz(row)), src, valid);
-    }
-    cp_async_commit();
-}
 
 __device__ __forceinline__ unsigned long long okey(double v)
 {
@@ -858,11 +938,12 @@ __device__ __forceinline__ void node_write(const CellNodesArgs &P, int64_t m3, c
             k += P.sv[s][2] * S[s];
             h += slot_heat()[s] * S[s];
         }
-        P.O.ro[m3] = r / W0;
-        P.O.et[m3] = 0.0 / W0;  // beta is zero on constant-property calls
-        P.O.cp[m3] = c / W0;
-        P.O.kt[m3] = k / W0;
-        P.O.ht[m3] = h / W0;
+        const double iw = 1.0 / W0;
+        P.O.ro[m3] = r * iw;
+        P.O.et[m3] = 0.0;  // beta is zero on constant-property calls
+        P.O.cp[m3] = c * iw;
+        P.O.kt[m3] = k * iw;
+        P.O.ht[m3] = h * iw;
         if (W1 != 0.0) P.O.tk[m3] = TK / W1;
     }
 }
@@ -923,100 +1004,136 @@ __device__ __forceinline__ void fold_minmax(double vmin, double vmax, int any, F
     }
 }
 
-// One CTA: node rows [d0, d0 + 31) x node columns [cs, cs + ncol).  Warp w of
-// group g sums cell column cc = cs - 1 + 8g + w, lane l cell row d0 - 1 + l; the
-// node column cc is finished by the same warp from its left half and the right
-// half of column cc - 1 (the warp before it, or the previous group's last).
-template <int NT>
-__global__ void __launch_bounds__(256, NT == 4 ? 2 : 3) k_cellnodes(const __grid_constant__ CellNodesArgs P)
+// One CTA: node rows [d0, d0 + ROWS - 1) x node columns [cs, cs + ncol).  In group g
+// warp w takes cell column cs - 1 + 8 g + w: its lanes S to a cell (lane s the pairs
+// of records s, s + S, ...), whose sums meet by shuffles and go to shared memory
+// (column w + 1; column 0 holds the last one of the group before); then a thread
+// finishes a node from its four cells.
+//
+// Bound by issue and the FP64 pipe: per record and lane 33 FP64 operations and
+// about 75 instructions in all, no branch; a cell and its node add about 500 once.
+// A lane to a cell reads whole kilobytes (rec_place) and needs no staging; S = 2
+// halves the serial chain where a grid leaves the device idle.  Per launch, with the
+// kernel that staged the records and picked slots and quadrants by one-hot factors
+// (226 instructions per record) before: 36M records, 1001^2 nodes 314 -> 207 us (DRAM
+// alone: 120); 2.56M, 401^2 41 -> 30; 160k, 101^2 24.5 -> 8.3; 6400, 21^2 21.7 -> 8.0.
+constexpr int kCnCols = 8, kCnThreads = 32 * kCnCols;
+constexpr int kCnBatch = 2;  // pairs of records per batch
+template <int NT, int S>
+struct CnShape {
+    static constexpr int ROWS = 32 / S;
+    using C = CellSums<NT>;
+    double v[C::N][kCnCols + 1][ROWS];
+};
+template <int NT, int S>
+__global__ void __launch_bounds__(kCnThreads, 2) k_cellnodes(const __grid_constant__ CellNodesArgs P)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    CnSmem<NT> &S = *reinterpret_cast<CnSmem<NT> *>(smraw);
-    constexpr int NL = NodeVals<NT>::L, NR = NodeVals<NT>::R;
+    using Shape = CnShape<NT, S>;
+    using C = CellSums<NT>;
+    Shape &M = *reinterpret_cast<Shape *>(smraw);
+    constexpr int ROWS = Shape::ROWS, CS = (kCnCols + 1) * ROWS;
     slot_heat_init(P);  // block_qconst syncs the block
     const QConst Q = block_qconst(P.ctr, P.viscmod);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int cs = (int)(blockIdx.x % P.ntx) * P.ncol, d0 = (int)(blockIdx.x / P.ntx) * 31;
-    const int groups = (P.ncol + 1) / 8;
-    CnWarpBuf &B = S.w[warp];
-    const int novf = P.ctr->novf;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % S;
+    const int cs = (int)(blockIdx.x % P.ntx) * P.ncol, d0 = (int)(blockIdx.x / P.ntx) * (ROWS - 1);
+    const int groups = (P.ncol + 1) / kCnCols;
+    const uint4 *recs = reinterpret_cast<const uint4 *>(P.ra);
     double vmin = 0.0, vmax = 0.0;
     int any = 0;
     unsigned owned = 0;
     for (int g = 0; g < groups; g++) {
-        const int cc = cs - 1 + 8 * g + warp, cr = d0 - 1 + lane;
+        const int cc = cs - 1 + kCnCols * g + warp;
+        const int row = lane / S, cr = d0 - 1 + row;
         const bool valid = cc >= 0 && cc < P.nc1 && cr >= 0 && cr < P.nc2;
         const int64_t cell = (int64_t)cc * P.nc2 + cr;
-        int32_t n = valid ? __ldg(P.count + cell) : 0;
-        if (lane >= 1 && !(g == 0 && warp == 0)) owned += (unsigned)n;  // each cell counted by one CTA
+        const int32_t n = valid ? __ldg(P.count + cell) : 0;
+        if (sub == 0 && row >= 1 && !(g == 0 && warp == 0)) owned += (unsigned)n;  // each cell counted by one CTA
         const int32_t nb = min(n, P.cap);
-        int maxc = nb;
-        for (int o = 16; o > 0; o >>= 1) maxc = max(maxc, __shfl_xor_sync(0xffffffffu, maxc, o));
-        __syncwarp();
-        B.cb[lane] = valid ? (int32_t)(cell * P.cap) : 0;
-        B.cn[lane] = nb;
-        __syncwarp();
+        // the lane's pairs of records: sub, sub + S, ...; every lane runs the warp's
+        // longest count in whole batches, with records that add nothing but 1 to
+        // wnd past its own
+        const uint4 *p = recs + (valid ? rec_place((int32_t)cell, 2 * sub, P.cap) : 0);
+        const int left = nb - 2 * sub, most = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(left, 0)),
+                  whole = (most + 2 * S * kCnBatch - 1) / (2 * S * kCnBatch),
+                  least = (int)__reduce_min_sync(0xffffffffu, (unsigned)max(left, 0));
         CellAcc<NT> a;
-        acc_zero(a);
-        if (maxc > 0) cn_stage(B, B.rec[0], P.ra, 0, lane);
-        for (int P0 = 0, k = 0; P0 < maxc; P0 += 4, k ^= 1) {
-            if (P0 + 4 < maxc) {
-                cn_stage(B, B.rec[k ^ 1], P.ra, P0 + 4, lane);
-                cp_async_wait<1>();
+        acc_start(a, Q);
+        RecPair r[kCnBatch];
+#pragma unroll
+        for (int k = 0; k < kCnBatch; k++) r[k] = rec_pair(p + k * S * 64, left - k * 2 * S);
+        for (int i = 1; i <= whole; i++) {
+            RecPair u[kCnBatch];
+            p += kCnBatch * S * 64;
+#pragma unroll
+            for (int k = 0; k < kCnBatch; k++) u[k] = r[k];
+            if ((i + 1) * kCnBatch * 2 * S <= least) {
+#pragma unroll
+                for (int k = 0; k < kCnBatch; k++) r[k] = rec_pair(p + k * S * 64);
             } else {
-                cp_async_wait<0>();
+#pragma unroll
+                for (int k = 0; k < kCnBatch; k++)
+                    r[k] = rec_pair(p + k * S * 64, left - (i * kCnBatch + k) * 2 * S);
             }
-            __syncwarp();
-            const uint4 *row = B.rec[k] + lane * kCnRS;
-            const int m = min(4, nb - P0);
-            for (int t = 0; t < m; t++) {
-                const uint4 u = row[t ^ cn_swz(lane)];
-                acc_rec<NT>(a, make_float4(__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z),
-                                           __uint_as_float(u.w)),
-                            Q);
+#pragma unroll
+            for (int k = 0; k < kCnBatch; k++) {
+                acc_rec<NT>(a, u[k].a, Q);
+                acc_rec<NT>(a, u[k].b, Q);
             }
-            __syncwarp();
         }
+        // (a lane's own records: its whole pairs, and the odd last one)
+        const int own = left <= 0 ? 0 : (left / (2 * S)) * 2 + min(left % (2 * S), 2);
+        a.wnd -= (double)(whole * kCnBatch * 2 - own);
         if (n > nb) {  // a full bucket: the rest of the cell's records are in the overflow list
-            for (int o = 0; o < novf; o++) {
-                const OvfRec r = P.ovf[o];
-                if (r.cell == (int32_t)cell) acc_rec<NT>(a, r.a, Q);
-            }
+            const int novf = P.ctr->novf;
+            for (int o = sub; o < novf; o += S)
+                if (P.ovf[o].cell == (int32_t)cell) acc_rec<NT>(a, *reinterpret_cast<const uint4 *>(&P.ovf[o].a), Q);
         }
-        // left half (corners 0 and 1 reach node column cc) and right half
-        // (corners 2, 3 and the centre reach node column cc + 1) of the node at
-        // row cr: corner 0 of this lane, corner 1 of the lane below
-        double L[NL];
-        double *hr = &S.hr[g & 1][warp][0][0];
-        double wt[NT][4], w1[4], tk[4];
-        acc_corners<NT>(a, P.mob, wt, w1, tk);
-#pragma unroll
-        for (int k = 0; k < NT; k++) {
-            L[k] = wt[k][0] + __shfl_up_sync(0xffffffffu, wt[k][1], 1);
-            hr[k * 32 + lane] = wt[k][2] + __shfl_up_sync(0xffffffffu, wt[k][3], 1);
-        }
-        L[NT + 0] = w1[0] + __shfl_up_sync(0xffffffffu, w1[1], 1);
-        L[NT + 1] = tk[0] + __shfl_up_sync(0xffffffffu, tk[1], 1);
-        L[NT + 2] = a.nu[0] + __shfl_up_sync(0xffffffffu, a.nu[1], 1);
-        L[NT + 3] = a.wnu[0] + __shfl_up_sync(0xffffffffu, a.wnu[1], 1);
-        hr[(NT + 0) * 32 + lane] = w1[2] + __shfl_up_sync(0xffffffffu, w1[3], 1);
-        hr[(NT + 1) * 32 + lane] = tk[2] + __shfl_up_sync(0xffffffffu, tk[3], 1);
-        hr[(NT + 2) * 32 + lane] = a.nu[2] + __shfl_up_sync(0xffffffffu, a.nu[3], 1);
-        hr[(NT + 3) * 32 + lane] = a.wnu[2] + __shfl_up_sync(0xffffffffu, a.wnu[3], 1);
-        hr[(NT + 4) * 32 + lane] = __shfl_up_sync(0xffffffffu, a.nd, 1);
-        hr[(NT + 5) * 32 + lane] = __shfl_up_sync(0xffffffffu, a.wnd, 1);
+        __syncwarp();
+        acc_finish<NT, S>(a, Q, n, [&](int f, double v) {
+            if (f % S == sub) M.v[f][warp + 1][row] = v;
+        });
         __syncthreads();
-        const int m1 = cc, m2 = cr;
-        if (lane >= 1 && m1 >= cs && m1 < cs + P.ncol && m1 < P.nx && m2 < P.ny && !(g == 0 && warp == 0)) {
-            const double *hp = warp > 0 ? &S.hr[g & 1][warp - 1][0][0] : &S.hr[(g - 1) & 1][7][0][0];
-            double Sv[NR];
+        for (int t = threadIdx.x; t < kCnCols * ROWS; t += kCnThreads) {
+            const int col = t / ROWS, row = t % ROWS, m1 = cs - 1 + kCnCols * g + col, m2 = d0 - 1 + row;
+            if (row < 1 || m1 < cs || m1 >= cs + P.ncol || m1 >= P.nx || m2 >= P.ny) continue;
+            // cells (m1, m2), (m1, m2 - 1), (m1 - 1, m2), (m1 - 1, m2 - 1): corners 0..3
+            const double *c0 = &M.v[0][col + 1][row], *c1 = c0 - 1, *c2 = c0 - ROWS, *c3 = c2 - 1;
+            double Sv[NodeVals<NT>::N];
+            double w1 = 0.0;
 #pragma unroll
-            for (int k = 0; k < NL; k++) Sv[k] = L[k] + hp[k * 32 + lane];
-            Sv[NT + 4] = hp[(NT + 4) * 32 + lane];
-            Sv[NT + 5] = hp[(NT + 5) * 32 + lane];
+            for (int k = 0; k <= NT; k++) {
+                const int at = 4 * k * CS;
+                const double w = 0.25 * ((corner4<0>(c0 + at, CS) + corner4<1>(c1 + at, CS)) +
+                                         (corner4<2>(c2 + at, CS) + corner4<3>(c3 + at, CS)));
+                if (k < NT) {
+                    Sv[k] = w;
+                    if ((P.mob >> k) & 1u) w1 += w;
+                } else {
+                    Sv[NT + 1] = w;  // T
+                }
+            }
+            Sv[NT] = w1;
+            Sv[NT + 2] = (c0[C::NU * CS] + c1[(C::NU + 1) * CS]) + (c2[(C::NU + 2) * CS] + c3[(C::NU + 3) * CS]);
+            Sv[NT + 3] = (c0[C::WNU * CS] + c1[(C::WNU + 1) * CS]) + (c2[(C::WNU + 2) * CS] + c3[(C::WNU + 3) * CS]);
+            Sv[NT + 4] = c3[C::ND * CS];
+            Sv[NT + 5] = c3[C::WND * CS];
             node_finish<NT>(P, Q, m1, m2, Sv, vmin, vmax, any);
         }
+        if (g + 1 == groups) break;
+        // the last column becomes the next group's column 0
+        double keep[(C::N * ROWS + kCnThreads - 1) / kCnThreads];
+#pragma unroll
+        for (int k = 0; k < (C::N * ROWS + kCnThreads - 1) / kCnThreads; k++) {
+            const int t = k * kCnThreads + threadIdx.x;
+            if (t < C::N * ROWS) keep[k] = M.v[t / ROWS][kCnCols][t % ROWS];
+        }
         __syncthreads();
+#pragma unroll
+        for (int k = 0; k < (C::N * ROWS + kCnThreads - 1) / kCnThreads; k++) {
+            const int t = k * kCnThreads + threadIdx.x;
+            if (t < C::N * ROWS) M.v[t / ROWS][0][t % ROWS] = keep[k];
+        }
     }
     fold_minmax(vmin, vmax, any, P.ctr, owned, P.navg);
 }
@@ -1071,7 +1188,7 @@ __global__ void __launch_bounds__(128) k_node_guard(const __grid_constant__ Cell
                 const int64_t cell = (int64_t)c1 * P.nc2 + c2;
                 const int32_t n = P.count[cell], nb = min(n, P.cap);
                 for (int t = lane; t < nb; t += 32) {
-                    const float4 r = P.ra[cell * P.cap + t];
+                    const float4 r = P.ra[rec_place((int32_t)cell, t, P.cap)];
                     fn(c, r, rec_lnu(r));
                 }
                 if (n > nb)
@@ -1102,11 +1219,10 @@ __global__ void __launch_bounds__(128) k_node_guard(const __grid_constant__ Cell
             double t[6];
             terms(c, r, lnu, t);
             const double wq = (t[0] + cq[0]) - cq[0];
-            const uint32_t tf = __float_as_uint(r.w);
-            const int slot = (int)(tf & 3u);
+            const int slot = rec_slot(r);
             for (int k = 0; k < NT; k++)
                 if (slot == k) S[k] += wq;
-            if (!(tf & 4u)) {
+            if (!rec_immobile(r)) {
                 S[NT] += wq;
                 S[NT + 1] += (t[1] + cq[1]) - cq[1];
             }

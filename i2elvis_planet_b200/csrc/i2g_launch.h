@@ -195,7 +195,7 @@ struct OvfRec;
 constexpr int kFusedSlots = 4;  // rock types (< 50) a fused call can average
 struct FusedLaunch {
     int32_t cap;          // places per cell bucket (even)
-    float4 *ra;           // [ncells * cap]
+    float4 *ra;           // [cells, whole strips of 32, * cap] (rec_place)
     OvfRec *ovf;          // [markers]
     int32_t *count;       // [ncells]
     FusedCounters *ctr;

@@ -156,7 +156,7 @@ static FusedMove fused_move_args(const GridView &G, const AvgArgsK &V, const Fus
     FusedMove M{};
     M.avg = V;
     M.avg.rad2 = radmax_sq_threshold(G.xsize);
-    for (int t = 0; t < kAvgTypes; t++) M.tinfo[t] = F.tinfo[t];
+    for (int t = 0; t < kAvgTypes; t++) M.type[t] = rec_type_byte(F.tinfo[t]);
     M.cap = F.cap;
     M.ra = F.ra;
     M.ovf = F.ovf;
@@ -201,47 +201,49 @@ int launch_move_fused(const StepLaunch &L, const MoveArgs &A, const AvgArgsK &V,
     return 2;
 }
 
-// Cell-column groups per k_cellnodes CTA (node columns 8 per group, less the one
-// it repeats): the CTAs of a grid take ceil(CTAs / resident) waves of 8 x groups
-// columns each, so the count with the fewest column-waves fills the device best
-// (at 1001 x 1001 nodes with 444 resident CTAs, 5 groups: 858 CTAs in 2 waves
-// of 40 columns, where 4 groups take 1089 CTAs in 3 waves of 32); ties go to more
-// groups (fewer repeated columns).
-static int cellnode_groups(int nx, int ny, int resident)
+template <int NT, int S>
+static void cellnodes_shape(const StepLaunch &L, CellNodesArgs P, int groups)
 {
-    const int64_t nty = (ny + 30) / 31;
-    int best = 4;
-    int64_t cost = INT64_MAX;
-    for (int g = 2; g <= 6; g++) {
-        const int64_t ctas = (nx + 8 * g - 2) / (8 * g - 1) * nty;
-        const int64_t c = (ctas + resident - 1) / resident * 8 * g;
-        if (c <= cost) {
-            cost = c;
-            best = g;
-        }
-    }
-    return best;
+    using Shape = CnShape<NT, S>;
+    static unsigned long long attr = 0;
+    allow_dynamic_smem((const void *)k_cellnodes<NT, S>, (int)sizeof(Shape), &attr);
+    P.ncol = kCnCols * groups - 1;
+    P.ntx = (P.nx + P.ncol - 1) / P.ncol;
+    const int nty = (P.ny + Shape::ROWS - 2) / (Shape::ROWS - 1);
+    k_cellnodes<NT, S><<<(unsigned)(P.ntx * nty), kCnThreads, sizeof(Shape), L.stream>>>(P);
 }
 
+// Two lanes to a cell while that leaves a CTA at most to an SM: there a launch lasts
+// as long as one CTA's chain (101^2 nodes 9.4 -> 8.3 us, 21^2 9.1 -> 8.0); with more CTAs
+// the shuffles cost more than they save (401^2: 30 -> 42).  Else cell-column groups
+// per CTA (node columns 8 per group, less the one it repeats): the CTAs of a grid
+// take ceil(CTAs / resident) waves of 8 x groups columns each, so the count with the
+// fewest column-waves fills the device best (at 1001 x 1001 nodes with 296 resident
+// CTAs 5 groups, 858 CTAs in 3 waves of 40 columns: 207 us; 4 groups, 4 waves of 32:
+// 219; 6 groups, 3 of 48: 232); ties go to more groups (fewer repeated columns).
 template <int NT>
-static int cellnodes(const StepLaunch &L, const CellNodesArgs &Pin)
+static int cellnodes(const StepLaunch &L, const CellNodesArgs &P)
 {
-    static unsigned long long attr = 0;
-    static unsigned resident = 0;
-    const int smem = (int)sizeof(CnSmem<NT>);
-    allow_dynamic_smem((const void *)k_cellnodes<NT>, smem, &attr);
-    if (!resident) {
-        // three CTAs of 72 KB per SM: prefer shared memory over L1 (the records are
-        // read once, through cp.async)
-        cudaFuncSetAttribute((const void *)k_cellnodes<NT>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-        resident = resident_ctas((const void *)k_cellnodes<NT>, 256, smem);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    auto ctas = [&](int rows, int g) {
+        return (int64_t)((P.nx + kCnCols * g - 2) / (kCnCols * g - 1)) * ((P.ny + rows - 2) / (rows - 1));
+    };
+    if (ctas(CnShape<NT, 2>::ROWS, 1) <= sms) {
+        cellnodes_shape<NT, 2>(L, P, 1);
+    } else {
+        const int64_t resident = 2 * (int64_t)sms;
+        int best = 1;
+        int64_t cost = INT64_MAX;
+        for (int g = 1; g <= 6; g++) {
+            const int64_t c = (ctas(CnShape<NT, 1>::ROWS, g) + resident - 1) / resident * g;
+            if (c <= cost) {
+                cost = c;
+                best = g;
+            }
+        }
+        cellnodes_shape<NT, 1>(L, P, best);
     }
-    CellNodesArgs P = Pin;
-    P.ncol = 8 * cellnode_groups(P.nx, P.ny, (int)resident) - 1;
-    P.ntx = (P.nx + P.ncol - 1) / P.ncol;
-    const int nty = (P.ny + 30) / 31;
-    k_cellnodes<NT><<<(unsigned)(P.ntx * nty), 256, smem, L.stream>>>(P);
     k_node_guard<NT><<<148, 128, 0, L.stream>>>(P);
     return 2;
 }
@@ -330,10 +332,14 @@ void preload_mixed()
     cudaFuncGetAttributes(&a, k_move_fused<false, false>);
     cudaFuncGetAttributes(&a, k_move_fused<true, true>);
     cudaFuncGetAttributes(&a, k_move_fused<true, false>);
-    cudaFuncGetAttributes(&a, k_cellnodes<1>);
-    cudaFuncGetAttributes(&a, k_cellnodes<2>);
-    cudaFuncGetAttributes(&a, k_cellnodes<3>);
-    cudaFuncGetAttributes(&a, k_cellnodes<4>);
+    cudaFuncGetAttributes(&a, k_cellnodes<1, 1>);
+    cudaFuncGetAttributes(&a, k_cellnodes<1, 2>);
+    cudaFuncGetAttributes(&a, k_cellnodes<2, 1>);
+    cudaFuncGetAttributes(&a, k_cellnodes<2, 2>);
+    cudaFuncGetAttributes(&a, k_cellnodes<3, 1>);
+    cudaFuncGetAttributes(&a, k_cellnodes<3, 2>);
+    cudaFuncGetAttributes(&a, k_cellnodes<4, 1>);
+    cudaFuncGetAttributes(&a, k_cellnodes<4, 2>);
     cudaFuncGetAttributes(&a, k_node_guard<3>);
     cudaFuncGetAttributes(&a, k_fused_deferred<true>);
     cudaFuncGetAttributes(&a, k_fused_begin);
