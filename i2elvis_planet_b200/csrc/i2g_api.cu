@@ -43,6 +43,9 @@ struct i2g_ctx {
     bool own_stream = false;
     int64_t nx = 0, ny = 0, nn = 0, ncells = 0;
     double *gx = nullptr, *gy = nullptr, *xmid = nullptr, *ymid = nullptr;
+    uint8_t *lines = nullptr;  // the axes' tables below, one block (line_tables)
+    LinePair *bpx = nullptr, *bpy = nullptr, *mpx = nullptr, *mpy = nullptr;
+    bool pairs = false;  // every width within div_by's range
     float *ixb = nullptr, *iyb = nullptr, *ixm = nullptr, *iym = nullptr;
     float4 *lx = nullptr, *ly = nullptr;
     double *g[G_N] = {};
@@ -263,6 +266,59 @@ struct PhaseTimer {
     }
 };
 
+// The tables of one axis of n lines, side by side in one block: pairs of lines and
+// of midpoints, {width, 1/width, 1/mid spacing} and its parts in FP32, lines,
+// midpoints, 1.0/d/d of the diffusion term (heatmart.c:592)
+struct AxisTables {
+    LinePair *bp, *mp;
+    float4 *l;
+    double *g, *mid, *id2;
+    float *ib, *im;
+};
+
+int64_t line_bytes(int64_t n) { return (n + 3) / 4 * 4 * (2 * sizeof(LinePair) + sizeof(float4) + 3 * sizeof(double) + 2 * sizeof(float)); }
+
+AxisTables axis_tables(uint8_t *at, int64_t n)
+{
+    n = (n + 3) / 4 * 4;
+    AxisTables t;
+    t.bp = reinterpret_cast<LinePair *>(at);
+    t.mp = t.bp + n;
+    t.l = reinterpret_cast<float4 *>(t.mp + n);
+    t.g = reinterpret_cast<double *>(t.l + n);
+    t.mid = t.g + n;
+    t.id2 = t.mid + n;
+    t.ib = reinterpret_cast<float *>(t.id2 + n);
+    t.im = t.ib + n;
+    return t;
+}
+
+// the tables (host memory, zeroed) from the lines g; whether every width is within
+// div_by's range
+bool fill_axis(const AxisTables &t, const double *g, int64_t n)
+{
+    bool ok = true;
+    auto pair = [&](double x0, double x1) {
+        const double h = x1 - x0;
+        ok = ok && h > 0x1p-400 && h < 0x1p400;
+        return LinePair{x0, x1, h, 1.0 / h};
+    };
+    for (int64_t i = 0; i < n; i++) t.g[i] = g[i];
+    for (int64_t i = 0; i + 1 < n; i++) {
+        const double w = g[i + 1] - g[i];
+        t.mid[i] = (g[i] + g[i + 1]) / 2.0;
+        t.ib[i] = (float)(1.0 / w);
+        t.id2[i] = 1.0 / w / w;
+        t.bp[i] = pair(g[i], g[i + 1]);
+    }
+    for (int64_t i = 0; i + 2 < n; i++) {
+        t.im[i] = (float)(1.0 / (t.mid[i + 1] - t.mid[i]));
+        t.mp[i] = pair(t.mid[i], t.mid[i + 1]);
+    }
+    for (int64_t i = 0; i + 1 < n; i++) t.l[i] = make_float4((float)(g[i + 1] - g[i]), t.ib[i], t.im[i], 0.f);
+    return ok;
+}
+
 GridView grid_view(const i2g_ctx *c)
 {
     GridView G{};
@@ -301,6 +357,12 @@ GridView grid_view(const i2g_ctx *c)
     G.sxxf = c->gpresent[G_SXX] ? c->ef[G_SXX] : nullptr;
     G.syyf = c->gpresent[G_SYY] ? c->ef[G_SYY] : nullptr;
     G.sxyf = c->gpresent[G_SXY] ? c->ef[G_SXY] : nullptr;
+    if (c->pairs) {
+        G.bpx = c->bpx;
+        G.bpy = c->bpy;
+        G.mpx = c->mpx;
+        G.mpy = c->mpy;
+    }
     G.ixb = c->ixb;
     G.iyb = c->iyb;
     G.ixm = c->ixm;
@@ -580,9 +642,12 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return bail(I2G_ECUDA);
     int r = I2G_OK;
 #define A(p, n) if ((r = dalloc(c, &(p), (n))) != I2G_OK) return bail(r)
-    A(c->gx, c->nx); A(c->gy, c->ny); A(c->xmid, c->nx); A(c->ymid, c->ny);
-    A(c->ixb, c->nx); A(c->iyb, c->ny); A(c->ixm, c->nx); A(c->iym, c->ny);
-    A(c->lx, c->nx); A(c->ly, c->ny);
+    A(c->lines, line_bytes(c->nx) + line_bytes(c->ny));
+    {
+        const AxisTables X = axis_tables(c->lines, c->nx), Y = axis_tables(c->lines + line_bytes(c->nx), c->ny);
+        c->bpx = X.bp; c->mpx = X.mp; c->lx = X.l; c->gx = X.g; c->xmid = X.mid; c->idx2 = X.id2; c->ixb = X.ib; c->ixm = X.im;
+        c->bpy = Y.bp; c->mpy = Y.mp; c->ly = Y.l; c->gy = Y.g; c->ymid = Y.mid; c->idy2 = Y.id2; c->iyb = Y.ib; c->iym = Y.im;
+    }
     for (int k = 0; k < G_N; k++) A(c->g[k], c->nn);
     if (P->precision == I2G_PREC_MIXED) {
         A(c->vxf, c->nn); A(c->vyf, c->nn); A(c->prf, c->nn); A(c->gaf, c->nn);
@@ -620,7 +685,6 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
     A(c->tconst, (int64_t)kTypeConstBytes);
     for (double *&p : c->tnode) A(p, c->nn);
     if (P->precision == I2G_PREC_MIXED) A(c->tnodef, 5 * c->nn);
-    A(c->idx2, c->nx); A(c->idy2, c->ny);
     A(c->td.melt, 12);
     A(c->sinter_stuck, 1);
 #undef A
@@ -680,21 +744,10 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
         if (!(gx[i] > gx[i - 1])) return fail(c, I2G_EINVAL, "gx must be strictly increasing");
     for (int64_t i = 1; i < ny; i++)
         if (!(gy[i] > gy[i - 1])) return fail(c, I2G_EINVAL, "gy must be strictly increasing");
-    std::vector<double> xm(nx, 0.0), ym(ny, 0.0);
-    std::vector<float> ixb(nx, 0.f), iyb(ny, 0.f), ixm(nx, 0.f), iym(ny, 0.f);
-    for (int64_t i = 0; i + 1 < nx; i++) xm[i] = (gx[i] + gx[i + 1]) / 2.0;
-    for (int64_t i = 0; i + 1 < ny; i++) ym[i] = (gy[i] + gy[i + 1]) / 2.0;
-    for (int64_t i = 0; i + 1 < nx; i++) ixb[i] = (float)(1.0 / (gx[i + 1] - gx[i]));
-    for (int64_t i = 0; i + 1 < ny; i++) iyb[i] = (float)(1.0 / (gy[i + 1] - gy[i]));
-    for (int64_t i = 0; i + 2 < nx; i++) ixm[i] = (float)(1.0 / (xm[i + 1] - xm[i]));
-    for (int64_t i = 0; i + 2 < ny; i++) iym[i] = (float)(1.0 / (ym[i + 1] - ym[i]));
-    // 1.0/celdx/celdx of the diffusion term (heatmart.c:592), the same operations
-    std::vector<double> idx2(nx, 0.0), idy2(ny, 0.0);
-    for (int64_t i = 0; i + 1 < nx; i++) idx2[i] = 1.0 / (gx[i + 1] - gx[i]) / (gx[i + 1] - gx[i]);
-    for (int64_t i = 0; i + 1 < ny; i++) idy2[i] = 1.0 / (gy[i + 1] - gy[i]) / (gy[i + 1] - gy[i]);
-    std::vector<float4> lx(nx, make_float4(0.f, 0.f, 0.f, 0.f)), ly(ny, make_float4(0.f, 0.f, 0.f, 0.f));
-    for (int64_t i = 0; i + 1 < nx; i++) lx[i] = make_float4((float)(gx[i + 1] - gx[i]), ixb[i], ixm[i], 0.f);
-    for (int64_t i = 0; i + 1 < ny; i++) ly[i] = make_float4((float)(gy[i + 1] - gy[i]), iyb[i], iym[i], 0.f);
+    std::vector<double> host((size_t)(line_bytes(nx) + line_bytes(ny)) / sizeof(double), 0.0);
+    uint8_t *hl = reinterpret_cast<uint8_t *>(host.data());
+    const bool px = fill_axis(axis_tables(hl, nx), gx, nx), py = fill_axis(axis_tables(hl + line_bytes(nx), ny), gy, ny);
+    c->pairs = px && py;
     c->inv_x = (double)(nx - 1) / (gx[nx - 1] - gx[0]);
     c->inv_y = (double)(ny - 1) / (gy[ny - 1] - gy[0]);
     // uniform axes: every line within 1e-9 of a width of g[0] + i w
@@ -712,18 +765,7 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
     c->uwx = uwx;
     c->uwy = uwy;
     c->fz.ready = false;
-    CK(cudaMemcpyAsync(c->gx, gx, sizeof(double) * nx, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->gy, gy, sizeof(double) * ny, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->xmid, xm.data(), sizeof(double) * nx, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->ymid, ym.data(), sizeof(double) * ny, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->ixb, ixb.data(), sizeof(float) * nx, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->iyb, iyb.data(), sizeof(float) * ny, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->ixm, ixm.data(), sizeof(float) * nx, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->iym, iym.data(), sizeof(float) * ny, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->lx, lx.data(), sizeof(float4) * nx, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->ly, ly.data(), sizeof(float4) * ny, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->idx2, idx2.data(), sizeof(double) * nx, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->idy2, idy2.data(), sizeof(double) * ny, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->lines, hl, (size_t)(line_bytes(nx) + line_bytes(ny)), cudaMemcpyHostToDevice, c->stream));
     const double *src[G_N] = {vx, vy, pr, exx, eyy, exy, sxx, syy, sxy, ga, mu};
     for (int k = 0; k < G_N; k++) {
         c->gpresent[k] = src[k] != nullptr;

@@ -331,8 +331,13 @@ __global__ void __launch_bounds__(256) k_contrib_const(const __grid_constant__ G
             const int32_t m10 = k / nc2, m20 = k - m10 * nc2;
             if constexpr (!MIXED) {
                 double a0, a1, b0, b1;
-                fdw64(__ldg(G.gx + m10), __ldg(G.gx + m10 + 1), x, a0, a1);
-                fdw64(__ldg(G.gy + m20), __ldg(G.gy + m20 + 1), y, b0, b1);
+                if (G.bpx) {
+                    fdw_pair(G.bpx, m10, x, a0, a1);
+                    fdw_pair(G.bpy, m20, y, b0, b1);
+                } else {
+                    fdw64(__ldg(G.gx + m10), __ldg(G.gx + m10 + 1), x, a0, a1);
+                    fdw64(__ldg(G.gy + m20), __ldg(G.gy + m20 + 1), y, b0, b1);
+                }
                 u.r.wx0 = a0;
                 u.r.wx1 = a1;
                 u.r.wy0 = b0;

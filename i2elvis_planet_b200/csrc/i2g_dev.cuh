@@ -28,6 +28,12 @@ namespace i2g {
 
 constexpr int kTypes = I2G_MAXTYPES;
 
+// Two neighbouring lines of an axis (basic lines g, or the midpoints of the
+// staggered nodes): their coordinates, h = x1 - x0 and r = 1 / h, both rounded once
+struct __align__(16) LinePair {
+    double x0, x1, h, r;
+};
+
 // grid fields and derived lookup tables, all in device memory
 struct GridView {
     int64_t nx, ny;  // xnumx, ynumy (grid lines)
@@ -35,6 +41,9 @@ struct GridView {
     double inv_x, inv_y;  // (n-1)/(g[n-1]-g[0]): first guess of the cell search
     const double *gx, *gy;
     const double *xmid, *ymid;  // (g[i]+g[i+1])/2.0, i < n-1: staggered node coordinates
+    // pairs of basic lines (i, i + 1) and of midpoints, per i (of the last midpoint
+    // x0 alone); NULL where a width is too small or large for div_by
+    const LinePair *bpx, *bpy, *mpx, *mpy;
     const double *vx, *vy, *pr, *ga;
     const double *exx, *eyy, *exy, *sxx, *syy, *sxy;  // NULL when absent (all zero)
     const double *mu;                                  // NULL when absent
@@ -208,6 +217,43 @@ __device__ __forceinline__ void fdw64(double x0, double x1, double xi, double &w
     w0 = c4 / c3;
 }
 
+// a / h to the nearest, as the IEEE division gives it, from r = 1 / h to the nearest
+// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000,
+// 1990: with r correctly rounded and q within one unit of a / h, the remainder
+// a - q h is exact and q + remainder x r rounds to the quotient; a first correction
+// of a r makes q that close).  For h and r in the normal range and a not below
+// 2^-900 in magnitude, where no product underflows.
+__device__ __forceinline__ double div_by(double a, double h, double r)
+{
+    double q = a * r;
+    q = __fma_rn(__fma_rn(-q, h, a), r, q);
+    return __fma_rn(__fma_rn(-q, h, a), r, q);
+}
+constexpr uint32_t kDivTiny = (1023u - 900u) << 20;  // high word of 2^-900
+__device__ __forceinline__ uint32_t abs_hi(double a) { return (uint32_t)__double2hiint(a) & 0x7fffffffu; }
+
+// fdw64 on the pair P[i]: the same two quotients (a zero or tiny numerator, a
+// marker on a line, takes the division itself)
+__device__ __forceinline__ void fdw_pair(const LinePair *__restrict__ P, int i, double xi, double &w0, double &w1)
+{
+    const double2 *p = reinterpret_cast<const double2 *>(P + i);
+    const double2 u = __ldg(p), v = __ldg(p + 1);
+    const double c5 = u.x - xi, c4 = u.y - xi;
+    if (min(abs_hi(c5), abs_hi(c4)) < kDivTiny) {
+        w1 = (-c5) / v.x;
+        w0 = c4 / v.x;
+    } else {
+        w1 = div_by(-c5, v.x, v.y);
+        w0 = div_by(c4, v.x, v.y);
+    }
+}
+
+// v / 6.0
+__device__ __forceinline__ double sixth_of(double v)
+{
+    return abs_hi(v) < kDivTiny ? v / 6.0 : div_by(v, 6.0, 1.0 / 6.0);
+}
+
 // FP32 weights from an FP64 offset and a precomputed FP32 reciprocal spacing.
 __device__ __forceinline__ void fdw32(double x0, float inv_h, double xi, float &w0, float &w1)
 {
@@ -274,6 +320,48 @@ __device__ __forceinline__ void interp_v(const GridView &G, double x, double y, 
         fdw32(__ldg(G.gy + m20), __ldg(G.iyb + m20), y, wy0, wy1);
         vyo = (double)bil32(G.vyf, ny, m1, m20, wx0, wx1, wy0, wy1);
     }
+}
+
+// allinterv() of the FP64 form on the line pairs: the same cells, stencils and sums
+// as interp_v<false>, the weights' divisions by div_by, the search from a nearby
+// cell (hx, hy; -1: none), which becomes the point's
+__device__ __forceinline__ void interp_v_pairs(const GridView &G, double x, double y, int &hx, int &hy, double &vxo,
+                                               double &vyo)
+{
+    clampxy(G, x, y);
+    const int nx = (int)G.nx, ny = (int)G.ny;
+    hx = hx >= 0 ? cell_walk(G.gx, nx, hx, x) : (int)cell_search(G.gx, G.nx, G.inv_x, x);
+    hy = hy >= 0 ? cell_walk(G.gy, ny, hy, y) : (int)cell_search(G.gy, G.ny, G.inv_y, y);
+    int m2 = hy, m1 = hx;
+    if (y < __ldg(G.ymid + hy)) m2 -= 1;
+    m2 = min(max(m2, 0), ny - 3);
+    if (x < __ldg(G.xmid + hx)) m1 -= 1;
+    m1 = min(max(m1, 0), nx - 3);
+    double wx0, wx1, wy0, wy1;
+    fdw_pair(G.bpx, hx, x, wx0, wx1);
+    fdw_pair(G.mpy, m2, y, wy0, wy1);
+    vxo = bil64(G.vx, ny, hx, m2, wx0, wx1, wy0, wy1);
+    fdw_pair(G.mpx, m1, x, wx0, wx1);
+    fdw_pair(G.bpy, hy, y, wy0, wy1);
+    vyo = bil64(G.vy, ny, m1, hy, wx0, wx1, wy0, wy1);
+}
+
+// the pressure of allintere() likewise (interp_e<false> without the other fields)
+__device__ __forceinline__ double interp_p_pairs(const GridView &G, double x, double y, int &hx, int &hy)
+{
+    clampxy(G, x, y);
+    const int nx = (int)G.nx, ny = (int)G.ny;
+    hx = hx >= 0 ? cell_walk(G.gx, nx, hx, x) : (int)cell_search(G.gx, G.nx, G.inv_x, x);
+    hy = hy >= 0 ? cell_walk(G.gy, ny, hy, y) : (int)cell_search(G.gy, G.ny, G.inv_y, y);
+    int a = hx, b = hy;
+    if (x > __ldg(G.xmid + hx)) a += 1;
+    a = min(max(a, 1), nx - 2);
+    if (y > __ldg(G.ymid + hy)) b += 1;
+    b = min(max(b, 1), ny - 2);
+    double wx0, wx1, wy0, wy1;
+    fdw_pair(G.mpx, a - 1, x, wx0, wx1);
+    fdw_pair(G.mpy, b - 1, y, wy0, wy1);
+    return bil64(G.pr, ny, a, b, wx0, wx1, wy0, wy1);
 }
 
 // cell-centre stencil of allintere() (markmart.c:1514-1522): lower index a, b >= 1

@@ -86,20 +86,33 @@ __device__ __forceinline__ int32_t move_marker(const GridView &G, const MarkerVi
         } else {
             double ga, e[6];
             int64_t c1, c2;
-            interp_e<MIXED>(G, x, y, pr, ga, false, VISC, e, c1, c2);
+            const bool pairs = G.bpx != nullptr;
+            if (!VISC && pairs) pr = interp_p_pairs(G, x, y, hx, hy);
+            else interp_e<MIXED>(G, x, y, pr, ga, false, VISC, e, c1, c2);
             M.p[i] = pr;
             if (VISC) visc_update(M, T, A, i, mt, pr, e);
-            if (A.markmod == 1) {
-                interp_v<MIXED>(G, x, y, vx0, vy0);
-            } else {
-                double vx1, vy1, vx2, vy2, vx3, vy3, vx4, vy4;
-                interp_v<MIXED>(G, x, y, vx1, vy1);
-                interp_v<MIXED>(G, x + vx1 * dt / 2.0, y + vy1 * dt / 2.0, vx2, vy2);
-                interp_v<MIXED>(G, x + vx2 * dt / 2.0, y + vy2 * dt / 2.0, vx3, vy3);
-                interp_v<MIXED>(G, x + vx3 * dt, y + vy3 * dt, vx4, vy4);
-                vx0 = (vx1 + 2.0 * vx2 + 2.0 * vx3 + vx4) / 6.0;
-                vy0 = (vy1 + 2.0 * vy2 + 2.0 * vy3 + vy4) / 6.0;
+            // the stages as a loop: one copy of the gather's code
+            double sx = 0.0, sy = 0.0, vx = 0.0, vy = 0.0;
+            const int nst = A.markmod == 1 ? 1 : 4;
+#pragma unroll 1
+            for (int st = 0; st < nst; st++) {
+                double px = x, py = y;
+                if (st == 1 || st == 2) {
+                    px = x + vx * dt / 2.0;
+                    py = y + vy * dt / 2.0;
+                } else if (st == 3) {
+                    px = x + vx * dt;
+                    py = y + vy * dt;
+                }
+                if (pairs) interp_v_pairs(G, px, py, hx, hy, vx, vy);
+                else interp_v<MIXED>(G, px, py, vx, vy);
+                // vx1 + 2 vx2 + 2 vx3 + vx4, in that order
+                const double c = st == 1 || st == 2 ? 2.0 : 1.0;
+                sx = st == 0 ? vx : sx + c * vx;
+                sy = st == 0 ? vy : sy + c * vy;
             }
+            vx0 = nst == 1 ? vx : sixth_of(sx);
+            vy0 = nst == 1 ? vy : sixth_of(sy);
         }
         if (A.outgrid == 2) {
             if (x < 0 || x > G.xsize) vy0 = 0;
@@ -118,8 +131,11 @@ __device__ __forceinline__ int32_t move_marker(const GridView &G, const MarkerVi
 
 // sub: the marker's arrival index in its new cell (the count before it), so the
 // sort places it at cstart[key] + sub without atomics of its own
+// The FP64 form is bound by the latency of its gathers and quotients: four CTAs per SM
+// and the stages as a loop (2.56M markers, 401^2 nodes: 187 us; three CTAs 227; with a
+// division per weight and the stages unrolled 218, five CTAs of that 207).
 template <bool MIXED, bool VISC>
-__global__ void __launch_bounds__(256) k_move(const __grid_constant__ GridView G, const __grid_constant__ MarkerView M,
+__global__ void __launch_bounds__(256, MIXED || VISC ? 0 : 4) k_move(const __grid_constant__ GridView G, const __grid_constant__ MarkerView M,
                                               const DevTypes *__restrict__ Ty, const __grid_constant__ MoveArgs A,
                                               int32_t *__restrict__ key, int32_t *__restrict__ count,
                                               int32_t *__restrict__ sub)

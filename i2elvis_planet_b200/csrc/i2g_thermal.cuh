@@ -30,8 +30,13 @@ __device__ __forceinline__ void tweights(const GridView &G, double x, double y, 
 {
     m10 = cell_search(G.gx, G.nx, G.inv_x, x);
     m20 = cell_search(G.gy, G.ny, G.inv_y, y);
-    fdw64(__ldg(G.gx + m10), __ldg(G.gx + m10 + 1), x, wx0, wx1);
-    fdw64(__ldg(G.gy + m20), __ldg(G.gy + m20 + 1), y, wy0, wy1);
+    if (G.bpx) {
+        fdw_pair(G.bpx, (int)m10, x, wx0, wx1);
+        fdw_pair(G.bpy, (int)m20, y, wy0, wy1);
+    } else {
+        fdw64(__ldg(G.gx + m10), __ldg(G.gx + m10 + 1), x, wx0, wx1);
+        fdw64(__ldg(G.gy + m20), __ldg(G.gy + m20 + 1), y, wy0, wy1);
+    }
 }
 
 __device__ __forceinline__ bool inside_box(const GridView &G, double x, double y)

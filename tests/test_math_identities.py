@@ -44,3 +44,31 @@ def test_sqrt_within_one_ulp_of_pow_half():
     for v in (0.0, -0.0, np.inf, -np.inf, np.nan, -1.0, 1.0, 4.0, 5e-324):
         assert ulps(pow_half(v), libm.pow(v, 0.5)) == 0, v
         assert np.signbit(pow_half(v)) == np.signbit(libm.pow(v, 0.5)) or np.isnan(v) or v < 0, v
+
+
+def test_div_by_is_the_division():
+    """div_by (i2g_dev.cuh): a / h from r = 1 / h by two corrections, every result
+    the IEEE quotient: random numerators, and ones whose quotient lies next to a
+    double or halfway between two, for widths of grids and extreme ones."""
+    libm.fma.restype = C.c_double
+    libm.fma.argtypes = [C.c_double] * 3
+    rng = np.random.default_rng(7)
+    n = 40000
+    h = np.concatenate([rng.random(n) * 10.0 ** rng.integers(-3, 7, n), 500.0 * (1 + 2.0 ** -52 * rng.integers(0, 4000, n)),
+                        np.ldexp(1 + rng.random(n), rng.integers(-390, 390, n)), np.full(n, 6.0)])
+    q = rng.random(h.size)
+    half = np.nextafter(q, 1) * 0.5 + q * 0.5
+    with np.errstate(under="ignore"):
+        a = np.where(rng.random(h.size) < 0.3, q * h, np.where(rng.random(h.size) < 0.5, half * h, rng.random(h.size) * h))
+        a = np.where(rng.random(h.size) < 0.5, a, np.nextafter(a, np.where(rng.random(h.size) < 0.5, np.inf, -np.inf)))
+    a = a * np.where(rng.random(h.size) < 0.5, 1.0, -1.0)
+    a = a[np.abs(a) >= 2.0 ** -900][: h.size]
+    h = h[: a.size]
+    bad = 0
+    for x, w in zip(a.tolist(), h.tolist()):
+        r = 1.0 / w
+        v = x * r
+        v = libm.fma(libm.fma(-v, w, x), r, v)
+        v = libm.fma(libm.fma(-v, w, x), r, v)
+        bad += v != x / w
+    assert bad == 0
