@@ -1470,8 +1470,8 @@ int i2g_ronurecalc(i2g_ctx *c, double timesum, uint32_t flags)
         D.melt_out = c->td.melt + 6 * (1 - c->td.cur);
         CK(cudaMemcpyAsync(D.melt_out, D.melt_in, 6 * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
         const StepLaunch L0{c->stream, G, M, c->dtypes};
-        c->launches += mixed ? launch_td_melt_mixed(L0, D, c->P.gridmod, c->td.flag, c->td.si)
-                             : launch_td_melt_fp64(L0, D, c->P.gridmod, c->td.flag, c->td.si);
+        c->launches += mixed ? launch_td_melt_mixed(L0, D, c->P.gridmod, c->sb.key, c->td.flag, c->td.si)
+                             : launch_td_melt_fp64(L0, D, c->P.gridmod, c->sb.key, c->td.flag, c->td.si);
         size_t bytes = c->td.scan_bytes;
         const int rs = td_prev_scan(c->stream, c->td.scan, &bytes, c->td.flag, c->td.prev, c->n);
         if (rs < 0) return fail(c, I2G_ECUDA, "melt-state scan");
@@ -1629,6 +1629,8 @@ int i2g_set_td_table(i2g_ctx *c, const i2g_td_table *t)
     a.pbmin = t->pbmin;
     a.tkstp = t->tkstp;
     a.pbstp = t->pbstp;
+    a.itkstp = 1.0 / t->tkstp;
+    a.ipbstp = 1.0 / t->pbstp;
     a.tknum = t->tknum;
     a.pbnum = t->pbnum;
     a.si_melting = t->si_melting;

@@ -248,8 +248,46 @@ __device__ __forceinline__ void contrib_inplace(const GridView &G, const MarkerV
     for (int q = 0; q < PayVec<MIXED, CONST>::R4; q++) d[q] = u.v[q];
 }
 
+// The class of a rock type whose property model takes its own path with densimod 2:
+// outside the table, solid, wet, molten
+__device__ __forceinline__ int table_class(int t)
+{
+    if (!td_type(t)) return 0;
+    return t > 20 ? 3 : (t == 6 ? 2 : 1);
+}
+
+// A block's 256 markers with densimod 2 in the order of their classes, so that most
+// warps follow one path of the property model (mixed types of a cell otherwise send
+// every warp down all of them); the markers stay the block's own 256 neighbours, whose
+// fields and grid nodes are in L1.  Table path, 6.25M markers, 501^2 nodes: 852 us in
+// storage order with the reference's expressions, 495 with the classes and
+// td_props_mixed / molten_k_mixed, 427 with five CTAs per SM (four: 436, two: 616;
+// the registers of the rare branches spill, the latency they hide is worth more).
+__device__ __forceinline__ int class_order(int t, bool valid, uint8_t *order, int (*cnt)[4])
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int c = valid ? table_class(t) : 0;
+    unsigned mine = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const unsigned m = __ballot_sync(0xffffffffu, c == k);
+        if (c == k) mine = m;
+        if (lane == 0) cnt[w][k] = __popc(m);
+    }
+    __syncthreads();
+    int at = __popc(mine & ((1u << lane) - 1u));
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+        for (int v = 0; v < 8; v++)
+            if (k < c || (k == c && v < w)) at += cnt[v][k];
+    order[at] = (uint8_t)threadIdx.x;
+    __syncthreads();
+    return order[threadIdx.x];
+}
+
 template <bool MIXED>
-__global__ void __launch_bounds__(256, 3) k_contrib_inplace(const __grid_constant__ GridView G,
+__global__ void __launch_bounds__(256, MIXED ? 5 : 3) k_contrib_inplace(const __grid_constant__ GridView G,
                                                             const __grid_constant__ MarkerView A,
                                                             const int32_t *__restrict__ rank,
                                                             const int32_t *__restrict__ key,
@@ -257,11 +295,14 @@ __global__ void __launch_bounds__(256, 3) k_contrib_inplace(const __grid_constan
                                                             const __grid_constant__ AvgArgsK args,
                                                             const double *__restrict__ T0p, void *payload)
 {
+    __shared__ uint8_t order[256];
+    __shared__ int cnt[8][4];
     uint4 *P = reinterpret_cast<uint4 *>(payload);
     const double T0 = *T0p;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += stride)
-        contrib_inplace<MIXED>(G, A, rank, key, Ty->t, args, T0, P, i);
+    int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (args.densimod == 2)
+        i = (int64_t)blockIdx.x * 256 + class_order(i < A.n ? A.type[i] : 0, i < A.n, order, cnt);
+    if (i < A.n) contrib_inplace<MIXED>(G, A, rank, key, Ty->t, args, T0, P, i);
 }
 
 // The in-place contributions of such a call (k_contrib_inplace's results): a

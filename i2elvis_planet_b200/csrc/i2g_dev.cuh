@@ -110,6 +110,7 @@ struct TdArgs {
     // (markmart.c:2147-2154), products formed once on the host in that order
     const double2 *rh;
     double tkmin, pbmin, tkstp, pbstp;
+    double itkstp, ipbstp;  // 1 / tkstp, 1 / pbstp (mixed form)
     int32_t tknum, pbnum;
     int32_t si_melting, ice_melting;
     // 1 (FP64 form): the reference's own expressions, libm pow included; 0 (mixed

@@ -172,6 +172,22 @@ __device__ __forceinline__ double molten_k(const i2g_types &T, int mm2, double m
 // occupancy): the pressure gather with viscalc, the molten-material
 // conductivity and the porous-silicate conductivity.
 
+// molten_k in the mixed form: with X = ro^2 bb ga cp / eta_fluid and Y = bb ga cp / nu
+// the flux's powers cancel, (kt^(2/3) dT^(4/3) X^(1/3))^(3/2) / (dT^2 ro) Y^(-1/2) =
+// kt sqrt(nu / eta_fluid) (ro > 0), and the flux's threshold is tested on its cube:
+// no pow (five of them took most of a molten marker's time)
+__device__ __forceinline__ double molten_k_mixed(const i2g_types &T, int mm2, double mkt, double Tm, double T0,
+                                                 double mro, double mga, double mcp, double mnu, double eta_fluid)
+{
+    const double kt = T.markkt[mm2], dT = Tm - T0, b = T.markbb[mm2] * mga * mcp, X = mro * mro * b / eta_fluid;
+    if (!(X >= 0.0) || !(kt >= 0.0)) return mkt;  // a negative power base: NaN flux
+    const double d2 = dT * dT;
+    const double cube = (0.089 * 0.089 * 0.089) * (kt * kt) * (d2 * d2) * X;
+    if (!(cube > 0.0001 * 0.0001 * 0.0001)) return cube == cube ? kt : mkt;
+    const double r = mnu / eta_fluid;
+    return r >= 0.0 ? copysign(kt * sqrt(r), mro) : r * 0.0 + sqrt(r);
+}
+
 // allintere() (markmart.c:281) and, for markers without a viscosity, viscalc()
 template <bool MIXED>
 __device__ __noinline__ void pressure_visc(const GridView &G, const i2g_types &T, const AvgArgsK &A, double x,
@@ -188,21 +204,76 @@ __device__ __noinline__ void pressure_visc(const GridView &G, const i2g_types &T
     }
 }
 
+// the pressure (and gravity) of pressure_visc alone, for a marker strictly inside the
+// box whose cell (c1, c2) is known
+template <bool MIXED>
+__device__ __forceinline__ void pressure_at(const GridView &G, double x, double y, int64_t c1, int64_t c2, bool want_ga,
+                                            double &pr, double &mga)
+{
+    int64_t a, b;
+    centre_stencil(G, c1, c2, x, y, a, b);
+    if constexpr (!MIXED) {
+        double wx0, wx1, wy0, wy1;
+        fdw64(__ldg(G.xmid + a - 1), __ldg(G.xmid + a), x, wx0, wx1);
+        fdw64(__ldg(G.ymid + b - 1), __ldg(G.ymid + b), y, wy0, wy1);
+        pr = bil64(G.pr, G.ny, a, b, wx0, wx1, wy0, wy1);
+        mga = (want_ga && G.ga) ? bil64(G.ga, G.ny, a, b, wx0, wx1, wy0, wy1) : 0.0;
+    } else {
+        float fx0, fx1, fy0, fy1;
+        fdw32(__ldg(G.xmid + a - 1), __ldg(G.ixm + a - 1), x, fx0, fx1);
+        fdw32(__ldg(G.ymid + b - 1), __ldg(G.iym + b - 1), y, fy0, fy1);
+        pr = (double)bil32(G.prf, G.ny, a, b, fx0, fx1, fy0, fy1);
+        mga = (want_ga && G.gaf) ? (double)bil32(G.gaf, G.ny, a, b, fx0, fx1, fy0, fy1) : 0.0;
+    }
+}
+
+// The table markers of a call, one thread per storage slot: flag[id] = id for a
+// table marker (the filter of markmart.c:277 and the types of markmart.c:482),
+// else -1; si[id] = the eps[21] it leaves (td_last_melt) at the pressure the
+// averaging interpolates for it (allintere, markmart.c:281), in the cell its key names.
+template <bool MIXED>
+__global__ void __launch_bounds__(256) k_td_melt(const __grid_constant__ GridView G,
+                                                 const __grid_constant__ MarkerView A,
+                                                 const __grid_constant__ TdArgs D, int32_t gridmod,
+                                                 const int32_t *__restrict__ key, int32_t *__restrict__ flag,
+                                                 double *__restrict__ si)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= A.n) return;
+    const int32_t id = A.id[i];
+    const int mt = A.type[i];
+    const double x = A.x[i], y = A.y[i], Tm = A.T[i];
+    const bool ok = (gridmod <= 1 || (id % gridmod) == 0) && td_type(mt) && x > 0 && y > 0 && x < G.xsize &&
+                    y < G.ysize && Tm > 0;
+    if (ok) {
+        double pr, ga;
+        const int32_t k = __ldg(key + i), nc2 = (int32_t)(G.ny - 1), m10 = k / nc2;
+        pressure_at<MIXED>(G, x, y, m10, k - m10 * nc2, false, pr, ga);
+        si[id] = td_last_melt(D, Tm, pr * 1.0000e-5, mt, nullptr);
+    }
+    flag[id] = ok ? id : -1;
+}
+
 // conductivity of molten silicate / iron by melt fraction (markmart.c:509-610);
 // the melt fractions are eps[21] / eps[50] as the marker reads them (markmart.c:287-288)
+template <bool MIXED>
 static __device__ __noinline__ double molten_branch(const i2g_types &T, const AvgArgsK &A, int32_t id, int mm2,
                                                     double mkt, double mtk, double T0, double mro, double mga,
                                                     double mcp, double mnu)
 {
     double xm = A.xmelt_si, xfe = A.xmelt_fe;
     if (A.densimod == 2) td_prev_melt(A.td, id, xm, xfe);
+    auto molten_k = [&](double eta) {
+        return MIXED ? molten_k_mixed(T, mm2, mkt, mtk, T0, mro, mga, mcp, mnu, eta)
+                     : i2g::molten_k(T, mm2, mkt, mtk, T0, mro, mga, mcp, mnu, eta);
+    };
     if (mm2 == 25 || mm2 == 26) {
         if (xm >= 0.4000 && xm <= 0.6000)
-            mkt = molten_k(T, mm2, mkt, mtk, T0, mro, mga, mcp, mnu, T.markn0[mm2] * exp((-172.690) * (xm - 0.400)));
-        if (xm > 0.6000) mkt = molten_k(T, mm2, mkt, mtk, T0, mro, mga, mcp, mnu, 100.0000);
+            mkt = molten_k(T.markn0[mm2] * exp((-172.690) * (xm - 0.400)));
+        if (xm > 0.6000) mkt = molten_k(100.0000);
     } else {
-        if (xfe < 1.0000) mkt = molten_k(T, mm2, mkt, mtk, T0, mro, mga, mcp, mnu, 1.0000e12);
-        if (xfe == 1.0000) mkt = molten_k(T, mm2, mkt, mtk, T0, mro, mga, mcp, mnu, 0.010);
+        if (xfe < 1.0000) mkt = molten_k(1.0000e12);
+        if (xfe == 1.0000) mkt = molten_k(0.010);
     }
     return mkt;
 }
@@ -211,11 +282,13 @@ static __device__ __noinline__ double molten_branch(const i2g_types &T, const Av
 // the density, heat capacity, expansion term, conductivity and viscosity; the
 // marker's type flips with its melt; the call's last table marker leaves the
 // melt state
-static __device__ __noinline__ int td_branch(const i2g_types &T, const AvgArgsK &A, int32_t id, int mm2,
+template <bool MIXED>
+static __device__ __forceinline__ int td_branch(const i2g_types &T, const AvgArgsK &A, int32_t id, int mm2,
                                              double mtk, double mpb, double &mro, double &mcp, double &mbb,
                                              double &mkt, double &mnu)
 {
-    const int nt = td_props(A.td, T, A.nubeg, A.nuend, mtk, mpb, mm2, mro, mcp, mbb, mkt, mnu);
+    const int nt = MIXED ? td_props_mixed(A.td, T, A.nubeg, A.nuend, mtk, mpb, mm2, mro, mcp, mbb, mkt, mnu)
+                         : td_props(A.td, T, A.nubeg, A.nuend, mtk, mpb, mm2, mro, mcp, mbb, mkt, mnu);
     if (id == __ldg(A.td.last)) td_write_state(A.td, mtk, mpb, mm2);
     return nt;
 }
@@ -356,7 +429,8 @@ __device__ __forceinline__ bool marker_contrib(const GridView &G, const i2g_type
     const double mtk = Tm;
     double pr = 0.0, mga = 0.0, mnu = eta;
     int64_t m10 = c1, m20 = c2;
-    if (need_p) pressure_visc<MIXED>(G, T, A, x, y, mtk, r.hi, mt, molten, needvisc, pr, mga, mnu, m10, m20);
+    if (needvisc) pressure_visc<MIXED>(G, T, A, x, y, mtk, r.hi, mt, molten, needvisc, pr, mga, mnu, m10, m20);
+    else if (need_p) pressure_at<MIXED>(G, x, y, c1, c2, molten, pr, mga);
     const double mpb = pr * 1.0000e-5;
     if (outside_radmax(G, A, x, y)) mnu = 1.000e+22;
     // porosity and maximum temperature (markmart.c:347-360, 462-472)
@@ -368,20 +442,23 @@ __device__ __forceinline__ bool marker_contrib(const GridView &G, const i2g_type
     if (mpor > 1.000) mpor = 1.000;
     if (has_por) r.por = mpor;
     // density (dencalc, markmart.c:1024-1046), heat capacity, conductivity (markmart.c:475-478)
-    double mro, mbb = 0;
-    if (A.densimod == 0) {
-        mro = T.markro[mm2];
+    double mro, mbb = 0, mcp, mkt;
+    if (A.densimod == 2 && td_type(mm2)) {
+        r.type = td_branch<MIXED>(T, A, r.id, mm2, mtk, mpb, mro, mcp, mbb, mkt, mnu);
     } else {
-        mro = T.markro[mm2] * (1.0 - T.markbb[mm2] * (mtk - 298.15)) * (1.0 + T.markaa[mm2] * (mpb - 1.0) * 1e-3) *
-              (1.000 - mpor);
-        mbb = T.markbb[mm2] / (1.0 - T.markbb[mm2] * (mtk - 298.15));
+        if (A.densimod == 0) {
+            mro = T.markro[mm2];
+        } else {
+            mro = T.markro[mm2] * (1.0 - T.markbb[mm2] * (mtk - 298.15)) *
+                  (1.0 + T.markaa[mm2] * (mpb - 1.0) * 1e-3) * (1.000 - mpor);
+            mbb = T.markbb[mm2] / (1.0 - T.markbb[mm2] * (mtk - 298.15));
+        }
+        mcp = T.markcp[mm2];
+        mkt = T.markkt[mm2];
+        if (T.markkf[mm2] != 0.0) mkt += T.markkf[mm2] / (mtk + 77.0);  // 0/(T+77) adds exactly 0
+        if (T.markkp[mm2] != 0.0) mkt *= exp(T.markkp[mm2] * mpb);  // exp(0) == 1 exactly
     }
-    double mcp = T.markcp[mm2];
-    double mkt = T.markkt[mm2];
-    if (T.markkf[mm2] != 0.0) mkt += T.markkf[mm2] / (mtk + 77.0);  // 0/(T+77) adds exactly 0
-    if (T.markkp[mm2] != 0.0) mkt *= exp(T.markkp[mm2] * mpb);  // exp(0) == 1 exactly
-    if (A.densimod == 2 && td_type(mm2)) r.type = td_branch(T, A, r.id, mm2, mtk, mpb, mro, mcp, mbb, mkt, mnu);
-    if (molten) mkt = molten_branch(T, A, r.id, mm2, mkt, mtk, T0, mro, mga, mcp, mnu);
+    if (molten) mkt = molten_branch<MIXED>(T, A, r.id, mm2, mkt, mtk, T0, mro, mga, mcp, mnu);
     // porosity-dependent conductivity of solid silicates (markmart.c:614-638)
     if (mm2 == 5 || mm2 == 6) mkt = (mpor == 0.0) ? T.markkt[mm2] : porous_k(T, mm2, mpor, mkt);
     if (mkt <= 0.0010) mkt = 0.0010;

@@ -282,6 +282,125 @@ static __device__ __noinline__ int td_props(const TdArgs &D, const i2g_types &T,
     return nt;
 }
 
+// td_props of the mixed form: the same model with the same arithmetic up to the
+// rounding of FP64 operations (a few 1e-16 of a value; the expansion term's central
+// difference over 0.1% of the pressure grows that to 1e-11).  Each curve is found
+// once per pressure, quotients with one denominator share its reciprocal, and
+// pow(r, 0.48) is exp(0.48 log r).
+static __device__ __noinline__ int td_props_mixed(const TdArgs &D, const i2g_types &T, double nubeg, double nuend,
+                                                  double mtk, double mpb, int mm2, double &mro_o, double &mcp_o,
+                                                  double &mbb_o, double &mkt_o, double &mnu)
+{
+    const bool low = mpb < 235000.0, crust = mm2 == 11 || mm2 == 12 || mm2 == 31 || mm2 == 32;
+    const double cap = low ? 1200.0 : 2100.0, iT = 1.0 / mtk;
+    const double t = mtk * (low ? 1.0 / 1774.0 : 1.0 / 2117.0);
+    // (770.9, 1157) / min(mtk, cap)
+    const double mkt1 = ((low ? 1.878 : 1.291) + (mtk <= cap ? (low ? 770.9 : 1157.0) * iT
+                                                             : (low ? 770.9 / 1200.0 : 1157.0 / 2100.0))) *
+                        (1.0 + (low ? 4.26e-6 : 2.50e-6) * mpb);
+    double mkt = mkt1 + t * t * t;
+    double e = (mtk - D.tkmin) * D.itkstp;
+    if (e < 0) e = 0;
+    if (e > (double)(D.tknum - 1)) e = (double)(D.tknum - 1);
+    double n = (mpb - D.pbmin) * D.ipbstp;
+    if (n < 0) n = 0;
+    if (n > (double)(D.pbnum - 1)) n = (double)(D.pbnum - 1);
+    int n1 = (e == e) ? (int)e : 0;
+    if (n1 > D.tknum - 2) n1 = D.tknum - 2;
+    int n2 = (n == n) ? (int)n : 0;
+    if (n2 > D.pbnum - 2) n2 = D.pbnum - 2;
+    e = e - (double)n1;
+    n = n - (double)n2;
+    const double2 *q = D.rh + ((crust ? D.tknum : 0) + n1) * D.pbnum + n2;
+    const double2 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + D.pbnum), q3 = __ldg(q + D.pbnum + 1);
+    const double r0 = q0.x + n * (q1.x - q0.x), r1 = q2.x + n * (q3.x - q2.x);
+    double mro = r0 + e * (r1 - r0);
+    const double hT0 = q2.y - q0.y, hT1 = q3.y - q1.y;
+    double mcp = (hT0 + n * (hT1 - hT0)) * D.itkstp;
+    if (mcp < 1e+2) mcp = 1e+2;
+    else if (mcp > 5e+4) mcp = 5e+4;
+    // 2 / (R1 + R0) and 2 / (R3 + R2) over one denominator
+    const double s0 = q1.x + q0.x, s1 = q3.x + q2.x, hP0 = q1.y - q0.y, hP1 = q3.y - q2.y;
+    double mbb = 2.0 * (s1 + e * (s0 - s1)) / (s0 * s1) - (hP0 + e * (hP1 - hP0)) * (D.ipbstp * 1e-5);
+    mbb *= mro * iT;
+    if (mbb < -1e-2) mbb = -1e-2;
+    else if (mbb > 1e-2) mbb = 1e-2;
+    // partially molten rock (markmart.c:2178-2235)
+    double ts, tl, hl;
+    si_curve(mpb, mm2, D.si_melting, false, ts, tl, hl);
+    const bool melts = tl != 0.0;
+    if (ts >= tl - 100.0) ts = tl - 100.0;
+    const double iw = 1.0 / (tl - ts);
+    auto clamp01 = [](double v) {
+        if (v < 0.0) v = 0.0;
+        if (v > 1.0) v = 1.0;
+        return v;
+    };
+    const double xm = melts ? clamp01((mtk - ts) * iw) : 0.0;
+    int nt = mm2;
+    if (xm > 0 && mm2 < 20) nt = mm2 + 20;
+    if (xm <= 0 && mm2 > 20) nt = mm2 - 20;
+    if (nt > 20) {
+        mro = mro * (1.0 - xm) +
+              xm * T.markro[nt] * (1.0 - T.markbb[nt] * (mtk - 298.15)) * (1.0 + T.markaa[nt] * (mpb - 1.0) * 1e-3);
+        if (xm > 0.1) {
+            // Pinkerton & Stevenson (1992) eq. 5, clamped
+            const double r = (1.0 - xm) / xm;
+            double nueff = T.marknu[nt] * exp((2.5 + (r > 0.0 ? exp(0.48 * log(r)) : 0.0)) * (1.0 - xm));
+            if (nueff < T.markn0[nt]) nueff = T.markn0[nt];
+            if (nueff > T.markn1[nt]) nueff = T.markn1[nt];
+            if (nueff < nubeg) nueff = nubeg;
+            if (nueff > nuend) nueff = nuend;
+            mnu = nueff;
+        }
+        const bool fin = isfinite(mpb);
+        const double k1 = T.markkp[nt], k0 = T.markkp[nt - 20], i77 = 1.0 / (mtk + 77.0);
+        const double e1 = (k1 == 0.0 && fin) ? 1.0 : exp(k1 * mpb);
+        const double e0 = k0 == k1 ? e1 : ((k0 == 0.0 && fin) ? 1.0 : exp(k0 * mpb));
+        mkt = ((T.markkt[nt] + T.markkf[nt] * i77) * e1) * xm +
+              ((T.markkt[nt - 20] + T.markkf[nt - 20] * i77) * e0) * (1.0 - xm);
+        if (xm > 0 && xm < 1.0) {
+            // latent heat by central differences: -ro dH/dP / T and dH/dT
+            const double dmpb = mpb * 0.001;
+            double lat[2];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                double a, b, h;
+                si_curve(k ? mpb + dmpb : mpb - dmpb, nt, D.si_melting, false, a, b, h);
+                lat[k] = b != 0.0 ? h * si_frac(mtk, a, b) : 0.0;
+            }
+            mbb += (lat[0] - lat[1]) * (mro * iT) / (2.0 * dmpb * 1e+5);
+            if (melts) mcp += hl * (clamp01((mtk + 1.0 - ts) * iw) - clamp01((mtk - 1.0 - ts) * iw)) * 0.5;
+        }
+    }
+    // water ice of type 6 (markmart.c:2237-2268)
+    if (nt == 6 && D.ice_melting == 1) {
+        double is, il;
+        ice_curve(mpb, false, is, il);
+        if (il != 0.0) {
+            const double lat = (284000.0 + 233000.0) * 0.3, iiw = 1.0 / (il - is);
+            const double xi = clamp01((mtk - is) * iiw);
+            if (xi > 0 && xi < 1.0) {
+                const double dmpb = mpb * 0.001;
+                double x[2];
+#pragma unroll 1
+                for (int k = 0; k < 2; k++) {
+                    double a, b;
+                    ice_curve(k ? mpb + dmpb : mpb - dmpb, false, a, b);
+                    x[k] = b != 0.0 ? clamp01((mtk - a) / (b - a)) : 0.0;
+                }
+                mbb += lat * (x[0] - x[1]) * (mro * iT) / (2.0 * dmpb * 1e+5);
+                mcp += lat * (clamp01((mtk + 1.0 - is) * iiw) - clamp01((mtk - 1.0 - is) * iiw)) * 0.5;
+            }
+        }
+    }
+    mro_o = mro;
+    mcp_o = mcp;
+    mbb_o = mbb;
+    mkt_o = mkt;
+    return nt;
+}
+
 // The eps[] state tdbasecalc leaves for the table marker at (mtk, mpb, type mm2):
 // its last meltpart1 call is at (mtk - 1, mpb) when a type-6 marker's ice is
 // partly molten (markmart.c:2263), else at (mtk, mpb) with the new type
@@ -321,32 +440,6 @@ __device__ __forceinline__ void td_prev_melt(const TdArgs &D, int32_t id, double
         xsi = __ldg(D.melt_in + 0);
         xfe = __ldg(D.melt_in + 2);
     }
-}
-
-// The table markers of a call, one thread per storage slot: flag[id] = id for a
-// table marker (the filter of markmart.c:277 and the types of markmart.c:482),
-// else -1; si[id] = the eps[21] it leaves (td_last_melt) at the pressure the
-// averaging interpolates for it (allintere, markmart.c:281).
-template <bool MIXED>
-__global__ void __launch_bounds__(256) k_td_melt(const __grid_constant__ GridView G,
-                                                 const __grid_constant__ MarkerView A,
-                                                 const __grid_constant__ TdArgs D, int32_t gridmod,
-                                                 int32_t *__restrict__ flag, double *__restrict__ si)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.n) return;
-    const int32_t id = A.id[i];
-    const int mt = A.type[i];
-    const double x = A.x[i], y = A.y[i], Tm = A.T[i];
-    const bool ok = (gridmod <= 1 || (id % gridmod) == 0) && td_type(mt) && x > 0 && y > 0 && x < G.xsize &&
-                    y < G.ysize && Tm > 0;
-    if (ok) {
-        double pr, ga, e[6];
-        int64_t m10, m20;
-        interp_e<MIXED>(G, x, y, pr, ga, false, false, e, m10, m20);
-        si[id] = td_last_melt(D, Tm, pr * 1.0000e-5, mt, nullptr);
-    }
-    flag[id] = ok ? id : -1;
 }
 
 // the eps[] state after the call, from the last table marker (markmart.c:2237-2275)
