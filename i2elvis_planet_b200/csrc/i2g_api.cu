@@ -46,6 +46,9 @@ struct i2g_ctx {
     uint8_t *lines = nullptr;  // the axes' tables below, one block (line_tables)
     LinePair *bpx = nullptr, *bpy = nullptr, *mpx = nullptr, *mpy = nullptr;
     bool pairs = false;  // every width within div_by's range
+    int32_t *binx = nullptr, *biny = nullptr;  // GridView.binx, biny (nonuniform axes)
+    bool xuni = false, yuni = false;
+    double bsx = 0, bsy = 0;
     float *ixb = nullptr, *iyb = nullptr, *ixm = nullptr, *iym = nullptr;
     float4 *lx = nullptr, *ly = nullptr;
     double *g[G_N] = {};
@@ -274,9 +277,14 @@ struct AxisTables {
     float4 *l;
     double *g, *mid, *id2;
     float *ib, *im;
+    int32_t *bin;  // axis_bins(n) + 1 entries (GridView.binx)
 };
 
-int64_t line_bytes(int64_t n) { return (n + 3) / 4 * 4 * (2 * sizeof(LinePair) + sizeof(float4) + 3 * sizeof(double) + 2 * sizeof(float)); }
+int64_t line_bytes(int64_t n)
+{
+    return (n + 3) / 4 * 4 * (2 * sizeof(LinePair) + sizeof(float4) + 3 * sizeof(double) + 2 * sizeof(float) + 4 * sizeof(int32_t));
+}
+int32_t axis_bins(int64_t n) { return (int32_t)(4 * n - 1); }
 
 AxisTables axis_tables(uint8_t *at, int64_t n)
 {
@@ -290,6 +298,7 @@ AxisTables axis_tables(uint8_t *at, int64_t n)
     t.id2 = t.mid + n;
     t.ib = reinterpret_cast<float *>(t.id2 + n);
     t.im = t.ib + n;
+    t.bin = reinterpret_cast<int32_t *>(t.im + n);
     return t;
 }
 
@@ -316,6 +325,13 @@ bool fill_axis(const AxisTables &t, const double *g, int64_t n)
         t.mp[i] = pair(t.mid[i], t.mid[i + 1]);
     }
     for (int64_t i = 0; i + 1 < n; i++) t.l[i] = make_float4((float)(g[i + 1] - g[i]), t.ib[i], t.im[i], 0.f);
+    const int32_t nb = axis_bins(n);
+    int64_t m = 0;
+    for (int32_t j = 0; j <= nb; j++) {
+        const double e = g[0] + (g[n - 1] - g[0]) * ((double)j / nb);
+        while (m < n - 2 && g[m + 1] <= e) m++;
+        t.bin[j] = (int32_t)m;
+    }
     return ok;
 }
 
@@ -363,6 +379,12 @@ GridView grid_view(const i2g_ctx *c)
         G.mpx = c->mpx;
         G.mpy = c->mpy;
     }
+    G.binx = c->xuni ? nullptr : c->binx;
+    G.biny = c->yuni ? nullptr : c->biny;
+    G.nbx = axis_bins(c->nx);
+    G.nby = axis_bins(c->ny);
+    G.bsx = c->bsx;
+    G.bsy = c->bsy;
     G.ixb = c->ixb;
     G.iyb = c->iyb;
     G.ixm = c->ixm;
@@ -645,8 +667,8 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
     A(c->lines, line_bytes(c->nx) + line_bytes(c->ny));
     {
         const AxisTables X = axis_tables(c->lines, c->nx), Y = axis_tables(c->lines + line_bytes(c->nx), c->ny);
-        c->bpx = X.bp; c->mpx = X.mp; c->lx = X.l; c->gx = X.g; c->xmid = X.mid; c->idx2 = X.id2; c->ixb = X.ib; c->ixm = X.im;
-        c->bpy = Y.bp; c->mpy = Y.mp; c->ly = Y.l; c->gy = Y.g; c->ymid = Y.mid; c->idy2 = Y.id2; c->iyb = Y.ib; c->iym = Y.im;
+        c->bpx = X.bp; c->mpx = X.mp; c->lx = X.l; c->gx = X.g; c->xmid = X.mid; c->idx2 = X.id2; c->ixb = X.ib; c->ixm = X.im; c->binx = X.bin;
+        c->bpy = Y.bp; c->mpy = Y.mp; c->ly = Y.l; c->gy = Y.g; c->ymid = Y.mid; c->idy2 = Y.id2; c->iyb = Y.ib; c->iym = Y.im; c->biny = Y.bin;
     }
     for (int k = 0; k < G_N; k++) A(c->g[k], c->nn);
     if (P->precision == I2G_PREC_MIXED) {
@@ -760,6 +782,10 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
     double uwx = 0, uwy = 0;
     const bool ux = uniform(gx, nx, uwx), uy = uniform(gy, ny, uwy);
     c->uni = ux && uy;
+    c->xuni = ux;
+    c->yuni = uy;
+    c->bsx = axis_bins(nx) / (gx[nx - 1] - gx[0]);
+    c->bsy = axis_bins(ny) / (gy[ny - 1] - gy[0]);
     c->ux0 = gx[0];
     c->uy0 = gy[0];
     c->uwx = uwx;

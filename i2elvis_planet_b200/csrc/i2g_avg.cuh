@@ -263,10 +263,9 @@ __device__ __forceinline__ int table_class(int t)
 // storage order with the reference's expressions, 495 with the classes and
 // td_props_mixed / molten_k_mixed, 427 with five CTAs per SM (four: 436, two: 616;
 // the registers of the rare branches spill, the latency they hide is worth more).
-__device__ __forceinline__ int class_order(int t, bool valid, uint8_t *order, int (*cnt)[4])
+__device__ __forceinline__ int class_order(int c, uint8_t *order, int (*cnt)[4])
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int c = valid ? table_class(t) : 0;
     unsigned mine = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -275,12 +274,15 @@ __device__ __forceinline__ int class_order(int t, bool valid, uint8_t *order, in
         if (lane == 0) cnt[w][k] = __popc(m);
     }
     __syncthreads();
-    int at = __popc(mine & ((1u << lane) - 1u));
+    // where the warp's part of each class starts: lane 8 k + v holds warp v's class k
+    const int own = cnt[lane & 7][lane >> 3];
+    int sum = own;
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-        for (int v = 0; v < 8; v++)
-            if (k < c || (k == c && v < w)) at += cnt[v][k];
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += u;
+    }
+    const int at = __shfl_sync(0xffffffffu, sum - own, 8 * c + w) + __popc(mine & ((1u << lane) - 1u));
     order[at] = (uint8_t)threadIdx.x;
     __syncthreads();
     return order[threadIdx.x];
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(256, MIXED ? 5 : 3) k_contrib_inplace(const __
     const double T0 = *T0p;
     int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (args.densimod == 2)
-        i = (int64_t)blockIdx.x * 256 + class_order(i < A.n ? A.type[i] : 0, i < A.n, order, cnt);
+        i = (int64_t)blockIdx.x * 256 + class_order(i < A.n ? table_class(A.type[i]) : 0, order, cnt);
     if (i < A.n) contrib_inplace<MIXED>(G, A, rank, key, Ty->t, args, T0, P, i);
 }
 

@@ -58,6 +58,11 @@ struct GridView {
     // index (2 i + qx) * 2 (ny - 1) + 2 j + qy) the bilinear forms of vx and vy in
     // the quarter's own coordinates, two float4; NULL when absent
     const float4 *vq4;
+    // nonuniform axis: per bin of a uniform division of [g[0], g[n-1]] the cell its
+    // left edge lies in (one entry more than bins); NULL: none.  bsx, bsy: bins per metre
+    const int32_t *binx, *biny;
+    double bsx, bsy;
+    int32_t nbx, nby;
     const float *ixb, *iyb;  // 1/(g[i+1]-g[i])
     const float *ixm, *iym;  // 1/(mid[i+1]-mid[i])
     const float4 *lx, *ly;   // per grid line: {width, 1/width, 1/mid spacing, 0}
@@ -209,6 +214,31 @@ __device__ __forceinline__ int cell_walk(const double *__restrict__ g, int n, in
     return m;
 }
 
+// cell_search through an axis' bins: the bin's two cells bound a bisection of a few
+// steps where the guess from the mean spacing lands many cells off and the search
+// bisects the whole axis.  The cell found is checked; anything else is searched.
+__device__ __forceinline__ int cell_bins(const double *__restrict__ g, int64_t n, double inv,
+                                         const int32_t *__restrict__ bin, int nb, double scale, double x)
+{
+    if (!bin) return (int)cell_search(g, n, inv, x);
+    const int j = min(max(__double2int_rd((x - __ldg(g)) * scale), 0), nb - 1);
+    int lo = __ldg(bin + j), hi = __ldg(bin + j + 1);
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(g + mid) <= x) lo = mid; else hi = mid - 1;
+    }
+    if (__ldg(g + lo) <= x && x < __ldg(g + lo + 1)) return lo;
+    return (int)cell_search(g, n, inv, x);
+}
+__device__ __forceinline__ int cell_x(const GridView &G, double x)
+{
+    return cell_bins(G.gx, G.nx, G.inv_x, G.binx, G.nbx, G.bsx, x);
+}
+__device__ __forceinline__ int cell_y(const GridView &G, double y)
+{
+    return cell_bins(G.gy, G.ny, G.inv_y, G.biny, G.nby, G.bsy, y);
+}
+
 // ------------------------------------------------------------------ weights
 // Two-point order-0 Fornberg weights in the reference's operation order.
 __device__ __forceinline__ void fdw64(double x0, double x1, double xi, double &w0, double &w1)
@@ -331,8 +361,8 @@ __device__ __forceinline__ void interp_v_pairs(const GridView &G, double x, doub
 {
     clampxy(G, x, y);
     const int nx = (int)G.nx, ny = (int)G.ny;
-    hx = hx >= 0 ? cell_walk(G.gx, nx, hx, x) : (int)cell_search(G.gx, G.nx, G.inv_x, x);
-    hy = hy >= 0 ? cell_walk(G.gy, ny, hy, y) : (int)cell_search(G.gy, G.ny, G.inv_y, y);
+    hx = hx >= 0 ? cell_walk(G.gx, nx, hx, x) : cell_x(G, x);
+    hy = hy >= 0 ? cell_walk(G.gy, ny, hy, y) : cell_y(G, y);
     int m2 = hy, m1 = hx;
     if (y < __ldg(G.ymid + hy)) m2 -= 1;
     m2 = min(max(m2, 0), ny - 3);
@@ -352,8 +382,8 @@ __device__ __forceinline__ double interp_p_pairs(const GridView &G, double x, do
 {
     clampxy(G, x, y);
     const int nx = (int)G.nx, ny = (int)G.ny;
-    hx = hx >= 0 ? cell_walk(G.gx, nx, hx, x) : (int)cell_search(G.gx, G.nx, G.inv_x, x);
-    hy = hy >= 0 ? cell_walk(G.gy, ny, hy, y) : (int)cell_search(G.gy, G.ny, G.inv_y, y);
+    hx = hx >= 0 ? cell_walk(G.gx, nx, hx, x) : cell_x(G, x);
+    hy = hy >= 0 ? cell_walk(G.gy, ny, hy, y) : cell_y(G, y);
     int a = hx, b = hy;
     if (x > __ldg(G.xmid + hx)) a += 1;
     a = min(max(a, 1), nx - 2);
@@ -515,6 +545,100 @@ __device__ inline double viscalc(const i2g_types &T, double mtk, double mpb, dou
     return nueff;
 }
 
+// The per-type constants viscalc forms again for every marker: 2 / k1 with
+// k1 = marknu / markss^(markmm - 1) of the power law, and 1 / markmm.
+struct ViscType {
+    double two_k1, imm;
+    int cls;  // which of viscalc's paths the type takes: bit 0 power law, bit 1 Peierls creep
+};
+__device__ __forceinline__ ViscType visc_type(const i2g_types &T, int m)
+{
+    ViscType V{0.0, 1.0, 0};
+    const double ss = T.markss[m], mm = T.markmm[m];
+    if (ss != 0 && mm != 1.0) {
+        V.two_k1 = 2.0 / (T.marknu[m] / pow(ss, mm - 1.0));
+        V.imm = 1.0 / mm;
+        V.cls = 1;
+    }
+    if (T.marks0[m] > 0) V.cls |= 2;
+    return V;
+}
+
+// viscalc() of the mixed form: the same model and branches in FP64, its powers as
+// exp and log of what they multiply and its chains of quotients over one
+// denominator (results within a few 1e-14 of viscalc's).  et: the viscosity before
+// (the strength's factor rii = (0.5 sii / eii / et)^0.87 when positive,
+// markmart.c:52-56), evaluated where the brittle strength reads it.
+__device__ __forceinline__ double viscalc_mixed(const i2g_types &T, const ViscType &V, double mtk, double mpb, double hi,
+                                                double epsin, double sigin, double et, double timesum,
+                                                double relax_time, double nubeg, double nuend, int mm2)
+{
+    if (mm2 > 20) return T.markn0[mm2];
+    const double lamb = T.markll[mm2], abrit = T.marka0[mm2], bbrit = T.markb0[mm2], s0 = T.marks0[mm2];
+    const double dh = T.markdh[mm2], dv = T.markdv[mm2], nu0 = T.marknu[mm2], act = dh + dv * mpb;
+    double nubrit = 0;
+    if (epsin > 0 && (bbrit > 0 || abrit * lamb > 0)) {
+        double sbrit = abrit + bbrit * mpb * 1e+5 * lamb;
+        if (s0 <= 0 && sbrit > T.marks1[mm2]) sbrit = T.marks1[mm2];
+        if (sbrit > 0 && hi > 0 &&
+            ((timesum - (hi * 1.000e+6 * 365.250 * 24.000 * 3600.000)) <
+             (relax_time * 1.000e+6 * 365.250 * 24.000 * 3600.000)))
+            sbrit = 1.000e+6;
+        if (sbrit > 0) {
+            const double rii = et > 0 ? exp(0.87 * log(0.5 * sigin / (epsin * et))) : 1.0;
+            nubrit = 2.0 * epsin * rii / sbrit;
+        } else {
+            nubrit = 1.0 / T.markn0[mm2];
+        }
+    }
+    double nupeierls = 0;
+    if (s0 > 0 && sigin > 1e+7 && epsin > 0) {
+        const double sig0 = T.marks1[mm2], c = -(8.314 * mtk) / act, l0 = log(epsin / s0);
+        double s = sig0 * 0.95;
+#pragma unroll 1
+        for (int n2 = 0; n2 < 5; n2++) {
+            s = pow_half(c * (l0 - 2.0 * log(s)));
+            if (s > 1.0) s = -s;
+            s = (1.0 - s) * sig0;
+        }
+        if (s > sig0) s = sig0;
+        nupeierls = 2.0 * epsin / s;
+    }
+    double nueff = 0;  // nunewt + nupowl
+    if (nu0) {
+        double e1 = 0.0;
+        const bool arrhenius = dh != 0 || dv != 0;
+        if (arrhenius) {
+            e1 = act / (8.314 * mtk);
+            if (e1 > 150.0) e1 = 150.0;
+            if (V.cls & 1) {
+            } else if (dh < 0 && dv > 0) {
+                e1 = dh * (mtk - dv);
+                if (e1 < -150.0) e1 = -150.0;
+            } else if (dh < 0 && dv < 0) {
+                e1 = (-dh) * (1.0 - (mtk - (-dv)) / (-dv)) / 8.314 / (-dv);
+                if (e1 > 150.0) e1 = 150.0;
+            }
+        }
+        const double ie = arrhenius ? exp(-e1) : 1.0;
+        if (V.cls & 1) {
+            nueff = V.two_k1 * ie;
+            // 1 / (0.5 (nu0 e^e1 epsin)^(1/mm) / epsin)
+            if (epsin > 0) nueff += 2.0 * epsin * exp(-(log(nu0 * epsin) + e1) * V.imm);
+        } else {
+            nueff = ie / nu0;
+        }
+    }
+    if (nubrit > nueff) nueff = nubrit;
+    if (nupeierls > nueff) nueff = nupeierls;
+    nueff = nueff <= 0 ? T.markn1[mm2] : 1.0 / nueff;
+    if (nueff < T.markn0[mm2]) nueff = T.markn0[mm2];
+    if (nueff > T.markn1[mm2]) nueff = T.markn1[mm2];
+    if (nueff < nubeg) nueff = nubeg;
+    if (nueff > nuend) nueff = nuend;
+    return nueff;
+}
+
 // strain-rate and stress invariants (markmart.c:47-48)
 __device__ __forceinline__ void invariants(const double *e, double &eii, double &sii)
 {
@@ -537,26 +661,25 @@ struct AxisF {
 };
 
 // the tail of axis_fast: weights of the basic cell b at FP32 offset d from g[b],
-// and the staggered stencil with its weights
-__device__ __forceinline__ void axis_tail(const float4 *__restrict__ L, int64_t n, int b, float d, AxisF &A)
+// and the staggered stencil with its weights; lb, lp: the lines b and b - 1
+__device__ __forceinline__ void axis_tail2(const float4 lb, const float4 lp, int64_t n, int b, float d, AxisF &A)
 {
-    const float4 lb = __ldg(L + b);
     A.b = b;
     A.b1 = d * lb.y;
     A.b0 = 1.0f - A.b1;
     int m = (A.b1 < 0.5f) ? b - 1 : b;
     if (m < 0) m = 0;
     if (m > (int)n - 3) m = (int)n - 3;
-    float t;
-    if (m == b) {
-        t = (d - 0.5f * lb.x) * lb.z;
-    } else {
-        const float4 lp = __ldg(L + b - 1);
-        t = (d + 0.5f * lp.x) * lp.z;
-    }
+    const bool same = m == b;  // else b - 1
+    const float t = (d + (same ? -0.5f * lb.x : 0.5f * lp.x)) * (same ? lb.z : lp.z);
     A.m = m;
     A.m1 = t;
     A.m0 = 1.0f - t;
+}
+
+__device__ __forceinline__ void axis_tail(const float4 *__restrict__ L, int64_t n, int b, float d, AxisF &A)
+{
+    axis_tail2(__ldg(L + b), __ldg(L + max(b - 1, 0)), n, b, d, A);
 }
 
 __device__ __forceinline__ void axis_fast(const double *__restrict__ g, const float4 *__restrict__ L, int64_t n,
@@ -574,6 +697,7 @@ __device__ __forceinline__ void axis_fast(const double *__restrict__ g, const fl
 struct AxisRK {
     int b;
     float du, lo, hi;
+    float w, wp;  // FP32 widths of cells b and b - 1 (line tables only)
 };
 
 __device__ __forceinline__ void axis_stage(const float4 *__restrict__ L, int64_t n, const AxisRK &R, float e,
@@ -581,18 +705,27 @@ __device__ __forceinline__ void axis_stage(const float4 *__restrict__ L, int64_t
 {
     if (e < R.lo) e = R.lo;
     if (e > R.hi) e = R.hi;
+    // a step to a neighbour without a branch; where the point is not in that cell
+    // either, the walk goes on
     int b = R.b;
-    while (e < 0.0f && b > 0) {
-        --b;
-        e += __ldg(L + b).x;
+    const bool down = e < 0.0f && b > 0, up = !down && e >= R.w && b < (int)n - 2;
+    e = down ? e + R.wp : (up ? e - R.w : e);
+    b += up - down;
+    float4 lb = __ldg(L + b);
+    if ((e < 0.0f && b > 0) || (e >= lb.x && b < (int)n - 2)) {
+        while (e < 0.0f && b > 0) {
+            --b;
+            e += __ldg(L + b).x;
+        }
+        while (b < (int)n - 2) {
+            const float w = __ldg(L + b).x;
+            if (!(e >= w)) break;
+            e -= w;
+            ++b;
+        }
+        lb = __ldg(L + b);
     }
-    while (b < (int)n - 2) {
-        const float w = __ldg(L + b).x;
-        if (!(e >= w)) break;
-        e -= w;
-        ++b;
-    }
-    axis_tail(L, n, b, e, A);
+    axis_tail2(lb, __ldg(L + max(b - 1, 0)), n, b, e, A);
 }
 
 __device__ __forceinline__ float bil32i(const float *__restrict__ f, int ny, int m1, int m2, float wx0, float wx1,
@@ -619,11 +752,17 @@ __device__ __forceinline__ void stage1_fast(const GridView &G, double x, double 
 {
     double xc = x, yc = y;
     clampxy(G, xc, yc);
-    const int bx = (int)cell_search(G.gx, G.nx, G.inv_x, xc), by = (int)cell_search(G.gy, G.ny, G.inv_y, yc);
+    const int bx = cell_x(G, xc), by = cell_y(G, yc);
     const double gbx = __ldg(G.gx + bx), gby = __ldg(G.gy + by);
     AxisF X, Y;
-    axis_tail(G.lx, G.nx, bx, (float)(xc - gbx), X);
-    axis_tail(G.ly, G.ny, by, (float)(yc - gby), Y);
+    const float4 lx = __ldg(G.lx + bx), ly = __ldg(G.ly + by);
+    const float4 lxp = __ldg(G.lx + max(bx - 1, 0)), lyp = __ldg(G.ly + max(by - 1, 0));
+    axis_tail2(lx, lxp, G.nx, bx, (float)(xc - gbx), X);
+    axis_tail2(ly, lyp, G.ny, by, (float)(yc - gby), Y);
+    RX.w = lx.x;
+    RX.wp = lxp.x;
+    RY.w = ly.x;
+    RY.wp = lyp.x;
     RX.b = bx;
     RX.du = (float)(x - gbx);
     RX.lo = (float)(0.0 - gbx);
@@ -716,8 +855,8 @@ __device__ __forceinline__ void strain_mixed(const GridView &G, double x, double
 __device__ __forceinline__ int32_t cell_key(const GridView &G, double x, double y, int cx = -1, int cy = -1)
 {
     clampxy(G, x, y);
-    const int64_t m10 = cx >= 0 ? cell_walk(G.gx, (int)G.nx, cx, x) : cell_search(G.gx, G.nx, G.inv_x, x);
-    const int64_t m20 = cy >= 0 ? cell_walk(G.gy, (int)G.ny, cy, y) : cell_search(G.gy, G.ny, G.inv_y, y);
+    const int64_t m10 = cx >= 0 ? cell_walk(G.gx, (int)G.nx, cx, x) : cell_x(G, x);
+    const int64_t m20 = cy >= 0 ? cell_walk(G.gy, (int)G.ny, cy, y) : cell_y(G, y);
     return (int32_t)(m10 * (G.ny - 1) + m20);
 }
 

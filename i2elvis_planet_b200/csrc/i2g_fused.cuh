@@ -306,8 +306,9 @@ struct FusedStat {
 // the warp calls it together (the bucket places are claimed per warp).
 template <bool VISC, bool UNI>
 __device__ __forceinline__ void move_record(const GridView &G, const MarkerView &M, const i2g_types &T,
-                                            const MoveArgs &A, const FusedMove &F, int64_t i, bool live, int mt,
-                                            double x, double y, const double Tm, double eta, FusedStat &st)
+                                            const MoveArgs &A, const FusedMove &F, const ViscType *VT, int64_t i,
+                                            bool live, int mt, double x, double y, const double Tm, double eta,
+                                            FusedStat &st)
 {
     const int lane = threadIdx.x & 31;
     bool ok = false, defer = false;
@@ -337,8 +338,7 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
             if (VISC) {
                 double e[6];
                 strain_mixed(G, x, y, X1, Y1, e);
-                visc_update(M, T, A, i, mt, pr, e);
-                eta = M.eta[i];
+                eta = visc_update_mixed(M, T, VT[mt < 20 ? mt : min(mt - 20, kAvgTypes - 1)], A, i, mt, Tm, eta, pr, e);
             }
             if (A.outgrid == 2) {
                 if (x < 0 || x > G.xsize) vy0 = 0;
@@ -474,15 +474,28 @@ __device__ __forceinline__ void move_stage_issue(const MarkerView &M, MoveStage 
 // Persistent: CTA b takes tiles b, b + gridDim.x, ... (the grid is the resident
 // CTAs of the device, one wave), so the loads of the next tile are in flight
 // while the current tile computes.  Each thread copies and reads only its own
-// marker's fields: the cp.async group wait orders them, no CTA barrier.
+// marker's fields: the cp.async group wait orders them, no CTA barrier.  With the
+// viscosity update a thread reads the marker its class order gives it, behind the
+// order's barriers.  Viscosity update, nonuniform grid, 4M markers: 564 us with
+// viscalc's own expressions and searches and walks by the whole axis, 348 with
+// viscalc_mixed and the class order, 284 with the axis bins and branch-free stage steps
+// (235 -> 170 of it without the update); two or three CTAs per SM 401, five 350.
 template <bool VISC, bool UNI>
-__global__ void __launch_bounds__(kMoveTile, VISC ? 2 : 4) k_move_fused(const __grid_constant__ GridView G,
+__global__ void __launch_bounds__(kMoveTile, VISC ? 4 : 4) k_move_fused(const __grid_constant__ GridView G,
                                                     const __grid_constant__ MarkerView M,
                                                     const DevTypes *__restrict__ Ty, const __grid_constant__ MoveArgs A,
                                                     const __grid_constant__ FusedMove F)
 {
     __shared__ MoveStage S[2];
     __shared__ FusedStat wst[kMoveTile / 32];
+    // the rheology's per-type constants, and the tile's order by the path it takes
+    __shared__ ViscType VT[VISC ? kAvgTypes : 1];
+    __shared__ uint8_t order[kMoveTile], types[kMoveTile];
+    __shared__ int cnt[kMoveTile / 32][4];
+    if (VISC) {
+        if (threadIdx.x < kAvgTypes) VT[threadIdx.x] = visc_type(Ty->t, threadIdx.x);
+        __syncthreads();
+    }
     const i2g_types &T = Ty->t;
     const int tid = threadIdx.x;
     const int ntiles = (int)((M.n + kMoveTile - 1) / kMoveTile);
@@ -496,18 +509,26 @@ __global__ void __launch_bounds__(kMoveTile, VISC ? 2 : 4) k_move_fused(const __
         i = (int64_t)tile * kMoveTile + tid;
         const int64_t inext = i + (int64_t)gridDim.x * kMoveTile;
         move_stage_issue(M, S[b ^ 1], inext);
-        const int mt = mt_next;
+        int mt = mt_next, mine = tid;
         mt_next = inext < M.n ? M.type[inext] : 0;
         cp_async_wait<1>();  // this tile's copies
+        if (VISC) {
+            // a thread takes a marker of the tile by its rheology's path
+            types[tid] = (uint8_t)mt;
+            mine = class_order(i < M.n && mt < kAvgTypes ? VT[mt < 20 ? mt : mt - 20].cls : 0, order, cnt);
+            mt = (int8_t)types[mine];
+            i = (int64_t)tile * kMoveTile + mine;
+        }
         const bool live = i < M.n;
         double x = 0.0, y = 0.0, Tm = 0.0, eta = 0.0;
         if (live) {
-            x = S[b].v[0][tid];
-            y = S[b].v[1][tid];
-            Tm = S[b].v[2][tid];
-            eta = S[b].v[3][tid];
+            x = S[b].v[0][mine];
+            y = S[b].v[1][mine];
+            Tm = S[b].v[2][mine];
+            eta = S[b].v[3][mine];
         }
-        move_record<VISC, UNI>(G, M, T, A, F, i, live, mt, x, y, Tm, eta, st);
+        move_record<VISC, UNI>(G, M, T, A, F, VT, i, live, mt, x, y, Tm, eta, st);
+        if (VISC) __syncthreads();  // the tile's stage and order are done with
     }
     cp_async_wait<0>();
     fused_stat_flush(st, F.ctr);

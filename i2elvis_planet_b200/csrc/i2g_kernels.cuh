@@ -58,6 +58,21 @@ __device__ __forceinline__ void visc_update(const MarkerView &M, const i2g_types
     }
 }
 
+// visc_update in the mixed form from the marker's loaded T and viscosity; returns the
+// viscosity it stores
+__device__ __forceinline__ double visc_update_mixed(const MarkerView &M, const i2g_types &T, const ViscType &V,
+                                                    const MoveArgs &A, int64_t i, int mt, double Tm, double eta,
+                                                    double pr, const double *e)
+{
+    if (!(mt < 50 && Tm > 0)) return eta;
+    double eii, sii;
+    invariants(e, eii, sii);
+    eta = viscalc_mixed(T, V, Tm, pr * 1e-5, M.hi ? M.hi[i] : 0.0, eii, sii, eta, A.timesum, A.relax_time, A.nubeg,
+                        A.nuend, mt < 20 ? mt : mt - 20);
+    M.eta[i] = eta;
+    return eta;
+}
+
 // One marker of movemark() (markmart.c:23-155); returns the marker's new cell.
 template <bool MIXED, bool VISC>
 __device__ __forceinline__ int32_t move_marker(const GridView &G, const MarkerView &M, const i2g_types &T,
@@ -81,7 +96,7 @@ __device__ __forceinline__ int32_t move_marker(const GridView &G, const MarkerVi
             if (VISC) {
                 double e[6];
                 strain_mixed(G, x, y, X1, Y1, e);
-                visc_update(M, T, A, i, mt, pr, e);
+                visc_update_mixed(M, T, visc_type(T, mt < 20 ? mt : mt - 20), A, i, mt, M.T[i], M.eta[i], pr, e);
             }
         } else {
             double ga, e[6];
