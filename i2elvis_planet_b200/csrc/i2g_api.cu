@@ -120,13 +120,13 @@ struct i2g_ctx {
         FusedCounters *ctr = nullptr;
         int32_t *treset = nullptr;   // [max_markers]
         int2 *defer = nullptr;       // [max_markers]
-        int32_t *guard = nullptr;    // [nodes]
         int32_t *cmax = nullptr;     // device scratch: largest cell count
         int32_t *count = nullptr;    // [ncells] records per cell
         bool resets_done = false;    // the sticky-air resets of the records are applied
-        void *host = nullptr;        // pinned copy of the counters of the last fused movemark
-        cudaEvent_t host_ev = nullptr;
-        bool host_pending = false;
+        uint8_t *zero = nullptr;     // ctr and count, one block, zeroed by every movemark
+        int64_t zero_bytes = 0;
+        int32_t *spilled = nullptr;  // mapped host memory: set by a movemark that overflowed a bucket
+        int32_t *spilled_dev = nullptr;
         bool ready = false;          // the buckets hold the records of the markers as they are
         double timesum = 0.0;        // the movemark's timesum
         int32_t nt = 0;              // type slots in use (averaged types present); 0 = none
@@ -602,8 +602,7 @@ int i2g_destroy(i2g_ctx *c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (void *p : c->allocs) cudaFree(p);
     if (c->fz.ra) cudaFree(c->fz.ra);
-    if (c->fz.host) cudaFreeHost(c->fz.host);
-    if (c->fz.host_ev) cudaEventDestroy(c->fz.host_ev);
+    if (c->fz.spilled) cudaFreeHost(c->fz.spilled);
     if (c->typecheck_host) cudaFreeHost(c->typecheck_host);
     for (auto &p : c->pending) {
         cudaEventDestroy(p.a);
@@ -693,16 +692,17 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
     A(c->typecheck, 8);
     A(c->ndeferred, 1);
     if (P->precision == I2G_PREC_MIXED) {
-        uint8_t *ovf = nullptr, *ctr = nullptr;
+        uint8_t *ovf = nullptr;
+        const int64_t cb = ((int64_t)fused_counters_bytes() + 255) / 256 * 256;
         A(ovf, (int64_t)fused_ovf_bytes() * (c->cap > 0 ? c->cap : 1));
-        A(ctr, (int64_t)fused_counters_bytes());
+        c->fz.zero_bytes = cb + (int64_t)sizeof(int32_t) * c->ncells;
+        A(c->fz.zero, c->fz.zero_bytes);
         c->fz.ovf = reinterpret_cast<OvfRec *>(ovf);
-        c->fz.ctr = reinterpret_cast<FusedCounters *>(ctr);
+        c->fz.ctr = reinterpret_cast<FusedCounters *>(c->fz.zero);
+        c->fz.count = reinterpret_cast<int32_t *>(c->fz.zero + cb);
         A(c->fz.treset, c->cap);
         A(c->fz.defer, c->cap);
-        A(c->fz.guard, c->nn);
         A(c->fz.cmax, 1);
-        A(c->fz.count, c->ncells);
     }
     A(c->tconst, (int64_t)kTypeConstBytes);
     for (double *&p : c->tnode) A(p, c->nn);
@@ -716,12 +716,13 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
         return bail(I2G_ENOMEM);
     }
     if (P->precision == I2G_PREC_MIXED) {
-        if (cudaHostAlloc(&c->fz.host, fused_counters_bytes(), cudaHostAllocDefault) != cudaSuccess) {
+        if (cudaHostAlloc((void **)&c->fz.spilled, sizeof(int32_t), cudaHostAllocMapped) != cudaSuccess) {
             cudaGetLastError();
-            c->fz.host = nullptr;
+            c->fz.spilled = nullptr;
             return bail(I2G_ENOMEM);
         }
-        if (cudaEventCreateWithFlags(&c->fz.host_ev, cudaEventDisableTiming) != cudaSuccess) return bail(I2G_ECUDA);
+        *c->fz.spilled = 0;
+        if (cudaHostGetDevicePointer((void **)&c->fz.spilled_dev, c->fz.spilled, 0) != cudaSuccess) return bail(I2G_ECUDA);
     }
     for (int k = 0; k < N_N; k++)
         if (cudaMemsetAsync(c->node[k], 0, sizeof(double) * (size_t)c->nn, c->stream) != cudaSuccess) return bail(I2G_ECUDA);
@@ -1246,21 +1247,20 @@ static bool fused_call(const i2g_ctx *c, double timesum)
            const_properties_call(c, timesum);
 }
 
-// the host copy of the last fused movemark's counters: grow the buckets when a
-// cell overflowed its bucket (the overflow list kept the results exact)
+// A fused movemark that overflowed a bucket has set the flag in host memory: read the
+// last one's counters and enlarge the buckets (the overflow list kept the results
+// exact).  The flag costs the other calls no copy and no query.
 static int fused_check_overflow(i2g_ctx *c)
 {
-    if (!c->fz.host_pending || c->in_graph) return I2G_OK;
-    if (cudaEventQuery(c->fz.host_ev) != cudaSuccess) {
-        cudaGetLastError();
-        return I2G_OK;
-    }
-    c->fz.host_pending = false;
+    if (c->in_graph || !*(volatile int32_t *)c->fz.spilled) return I2G_OK;
+    CK(cudaStreamSynchronize(c->stream));
+    *(volatile int32_t *)c->fz.spilled = 0;
+    std::vector<uint8_t> ctr(fused_counters_bytes());
+    CK(cudaMemcpy(ctr.data(), c->fz.ctr, ctr.size(), cudaMemcpyDeviceToHost));
     int32_t cmax = 0, novf = 0;
-    fused_host_stats(c->fz.host, &cmax, &novf);
+    fused_host_stats(ctr.data(), &cmax, &novf);
     if (novf > 0 && cmax > c->fz.cap) {
         c->fz.overflows++;
-        CK(cudaStreamSynchronize(c->stream));
         TRY(fused_buckets(c, cmax));
     }
     return I2G_OK;
@@ -1295,22 +1295,17 @@ int i2g_movemark(i2g_ctx *c, double timestep, double timesum, uint32_t flags)
         F.ctr = c->fz.ctr;
         F.treset = c->fz.treset;
         F.defer = c->fz.defer;
+        F.spilled = c->fz.spilled_dev;
         F.stepc = c->g_stepc;
         F.stepi = c->g_stepi;
         for (int t = 0; t < kAvgTypes; t++) F.tinfo[t] = c->fz.tinfo[t];
         const AvgArgsK V = avg_args(c, timesum, 0);
         {
             PhaseTimer t(c, 0);
-            CK(cudaMemsetAsync(c->fz.count, 0, sizeof(int32_t) * (size_t)c->ncells, c->stream));
-            CK(cudaMemsetAsync(c->fz.ctr, 0, fused_move_counters_bytes(), c->stream));
+            CK(cudaMemsetAsync(c->fz.zero, 0, (size_t)c->fz.zero_bytes, c->stream));
             c->launches += launch_move_fused(L, A, V, F);
         }
         CKL();
-        if (!c->fz.host_pending) {
-            CK(cudaMemcpyAsync(c->fz.host, c->fz.ctr, fused_counters_bytes(), cudaMemcpyDeviceToHost, c->stream));
-            CK(cudaEventRecord(c->fz.host_ev, c->stream));
-            c->fz.host_pending = true;
-        }
         c->fz.ready = true;
         c->fz.resets_done = false;
         c->fz.timesum = timesum;
@@ -1412,8 +1407,10 @@ static int fused_ronurecalc(i2g_ctx *c, double timesum, uint32_t flags)
     F.ovf = c->fz.ovf;
     F.count = c->fz.count;
     F.ctr = c->fz.ctr;
-    F.treset = c->fz.resets_done ? nullptr : c->fz.treset;  // marker indices of the storage at movemark
-    F.guard = c->fz.guard;
+    F.treset = c->fz.treset;  // marker indices of the storage at movemark
+    F.defer = c->fz.defer;
+    F.spilled = c->fz.spilled_dev;
+    F.first = !c->fz.resets_done;
     F.nt = c->fz.nt;
     for (int t = 0; t < kAvgTypes; t++) F.tinfo[t] = c->fz.tinfo[t];  // slots and immobile bits
     for (int k = 0; k < c->fz.nt; k++) {
@@ -2379,7 +2376,6 @@ int batch_run_streams_graph(i2g_batch *b, const double *timestep, double *timesu
             c->g_stepc = b->dstepc + (size_t)k * i2g_batch::kMaxSteps * 4;
             c->g_stepi = b->dstep;
             c->in_graph = true;
-            c->fz.host_pending = false;  // every replay copies the counters out
         }
         int r = I2G_OK;
         cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed);

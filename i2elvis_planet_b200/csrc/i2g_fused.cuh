@@ -31,7 +31,7 @@
 // The node values are therefore bitwise the same for every run, launch shape and
 // marker storage order.  A node whose temperature or viscosity weight sum is so
 // small that the quantum would cost more than 1e-9 of the value is recomputed by
-// k_node_guard with quanta of its own.
+// node_guard with quanta of its own.
 #pragma once
 
 #include "i2g_avg.cuh"
@@ -46,8 +46,8 @@ struct FusedCounters {
     // and |log-viscosity| (FP32 bit patterns of upper bounds), averaged markers
     uint32_t part[kFusedParts][4];
     int32_t novf, ntreset;  // overflow records, pending sticky-air resets
-    int32_t ndefer, pad0;   // records whose log-viscosity k_fused_deferred writes
-    int32_t nguard, any;    // nodes for k_node_guard; any node viscosity written
+    int32_t ndefer;         // records whose log-viscosity k_fused_begin writes
+    int32_t any;            // any node viscosity written
     unsigned long long kmin, kmax;  // ordered keys of the smallest / largest node viscosity
 };
 
@@ -64,7 +64,8 @@ struct FusedMove {
     float4 *ra;                  // [cells, whole strips of 32, * cap] the records (rec_pack, rec_place)
     OvfRec *ovf;                 // [markers]
     int32_t *count;              // [ncells] records per cell (zeroed before the launch)
-    FusedCounters *ctr;          // part/novf/ntreset zeroed before the launch
+    FusedCounters *ctr;          // zeroed before the launch
+    int32_t *spilled;            // host memory: set to 1 by a call that overflows a bucket
     int32_t *treset;             // [markers] markers whose T the averaging resets
     int2 *defer;                 // [markers] {marker, record place} of markers without a viscosity
     // a step replayed from a CUDA graph: the step's timesum from a device table
@@ -392,7 +393,7 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
             if (Tm != mtk) F.treset[atomicAdd(&F.ctr->ntreset, 1)] = (int32_t)i;
         }
         // a marker without a viscosity of its own (eta <= 0) gets it from
-        // viscalc in k_fused_deferred (a place is kept for it here)
+        // viscalc in k_fused_begin (a place is kept for it here)
         lnu = eta > 0 ? record_lnu(G, V, x, y, eta) : 0.0;
         defer = !(eta > 0);
         rec = rec_pack(weight_fix(wx1), weight_fix(wy1), (float)mtk, (uint32_t)F.type[mt], lnu);
@@ -408,6 +409,7 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
             F.ra[place] = rec;
         } else {
             const int32_t o = atomicAdd(&F.ctr->novf, 1);
+            if (o == 0) *(volatile int32_t *)F.spilled = 1;
             OvfRec r;
             r.a = rec;
             r.lnu = lnu;
@@ -534,41 +536,6 @@ __global__ void __launch_bounds__(kMoveTile, VISC ? 4 : 4) k_move_fused(const __
     fused_stat_flush(st, F.ctr);
 }
 
-// The markers k_move_fused kept a place for: viscosity from the rheology at the
-// marker's new position (allintere + viscalc, markmart.c:281, 320-332), then the
-// record's log-viscosity and the call's |log-viscosity| bound.
-template <bool MIXED>
-__global__ void __launch_bounds__(128) k_fused_deferred(const __grid_constant__ GridView G,
-                                                        const __grid_constant__ MarkerView M,
-                                                        const DevTypes *__restrict__ Ty,
-                                                        const __grid_constant__ FusedMove F)
-{
-    const int32_t m = F.ctr->ndefer;
-    if (m == 0) return;
-    AvgArgsK V = F.avg;  // viscalc's impact weakening reads timesum (markmart.c:1886-1889)
-    if (F.stepc) V.timesum = F.stepc[4 * *F.stepi];
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < m; q += stride) {
-        const int2 d = F.defer[q];
-        const int64_t i = d.x;
-        const double x = M.x[i], y = M.y[i];
-        const int mt = M.type[i];
-        const double mtk = mt < 2 ? V.tmp_ambient : M.T[i];
-        double pr = 0.0, mga = 0.0, mnu = 0.0;
-        int64_t m10, m20;
-        pressure_visc<MIXED>(G, Ty->t, V, x, y, mtk, M.hi ? M.hi[i] : 0.0, mt, false, true, pr, mga, mnu, m10, m20);
-        const double lnu = record_lnu(G, V, x, y, mnu);
-        if (d.y >= 0) {
-            F.ra[d.y] = rec_with_lnu(F.ra[d.y], lnu);
-        } else {
-            OvfRec &r = F.ovf[-d.y - 1];
-            r.a = rec_with_lnu(r.a, lnu);
-            r.lnu = lnu;
-        }
-        atomicMax(&F.ctr->part[q % kFusedParts][2], __float_as_uint(__double2float_ru(fabs(lnu))));
-    }
-}
-
 // ----------------------------------------------------------------- sums and nodes
 // The rounding of one averaging call, derived from the counters: two ways to add
 // terms in FP64 so that the sum does not depend on their order.
@@ -584,7 +551,7 @@ __global__ void __launch_bounds__(128) k_fused_deferred(const __grid_constant__ 
 //           operation per term.
 struct QConst {
     double cw, ctk, cnu;  // weights, temperature x weight, log-viscosity x weight
-    // a node goes to k_node_guard where a weight sum is below thr_w (thr_nuw for
+    // a node goes to node_guard where a weight sum is below thr_w (thr_nuw for
     // the viscosity weights), or |TK| below vtk, or |NU|, |ND| below vnu: there
     // the quanta could move its value by more than 1e-9 of the value
     double thr_w, thr_nuw, vtk, vnu;
@@ -872,7 +839,6 @@ struct CellNodesArgs {
     double nubeg, nuend;
     const double *mu;
     NodeOut O;
-    int32_t *guard;
     unsigned long long *navg;  // averaged markers (the records of the cells a CTA owns)
 };
 
@@ -970,9 +936,9 @@ __device__ __forceinline__ void node_write(const CellNodesArgs &P, int64_t m3, c
 }
 
 // A node whose sums are so small that the call's quanta would cost more than
-// 1e-9 of a value is listed for k_node_guard instead of written.
+// 1e-9 of a value is left to node_guard (true).
 template <int NT>
-__device__ __forceinline__ void node_finish(const CellNodesArgs &P, const QConst &Q, int m1, int m2, const double *S,
+__device__ __forceinline__ bool node_finish(const CellNodesArgs &P, const QConst &Q, int m1, int m2, const double *S,
                                             double &vmin, double &vmax, int &any)
 {
     const int64_t m3 = (int64_t)m1 * P.ny + m2;
@@ -983,8 +949,8 @@ __device__ __forceinline__ void node_finish(const CellNodesArgs &P, const QConst
     const bool flag = (W0 > 0 && W0 < Q.thr_w) || (W1 > 0 && (W1 < Q.thr_w || fabs(TK) < Q.vtk)) ||
                       (WNU > 0 && (WNU < Q.thr_nuw || fabs(NU) < Q.vnu)) ||
                       (WND > 0 && (WND < Q.thr_nuw || fabs(ND) < Q.vnu));
-    if (flag) P.guard[atomicAdd(&P.ctr->nguard, 1)] = (int32_t)m3;
-    else node_write<NT>(P, m3, S, vmin, vmax, any);
+    if (!flag) node_write<NT>(P, m3, S, vmin, vmax, any);
+    return flag;
 }
 
 // {min, max, any} of the CTA into the call's ordered-key atomics
@@ -1023,6 +989,102 @@ __device__ __forceinline__ void fold_minmax(double vmin, double vmax, int any, F
             if (!ctr->any) atomicExch(&ctr->any, 1);
         }
     }
+}
+
+// The viscosity range of the nodes a thread wrote
+struct ViscRange {
+    double lo, hi;
+    int any;
+};
+
+// A node whose sums are small against the call's quanta, by a warp: the records of
+// the node's four cells once for the largest terms, once more with quanta fitted to
+// this node (so the sums are exact again, at a resolution of 2^-52 of the node's own
+// largest terms), then the node as node_write makes it.
+template <int NT>
+static __device__ __noinline__ void node_guard(const CellNodesArgs &P, int m1, int m2, ViscRange *range)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t m3 = (int64_t)m1 * P.ny + m2;
+    const int novf = P.ctr->novf;
+    constexpr int NV = NT + 6;
+    // the terms of a record of cell c (c = 0..3: cells (m1-1, m2-1), (m1-1, m2),
+    // (m1, m2-1), (m1, m2)), which reaches the node through its corner 3 - c:
+    // t[0] weight, t[1] T x weight, t[2] quadrant weight, t[3] its
+    // log-viscosity term, t[4] centre weight, t[5] its term
+    auto terms = [&](int c, float4 r, double lnu, double *t) {
+        const int q = 3 - c;
+        const double X1 = weight_of(__float_as_uint(r.x)), Y1 = weight_of(__float_as_uint(r.y));
+        const double X0 = 1.0 - X1, Y0 = 1.0 - Y1;
+        const double wx = (q >> 1) ? X1 : X0, wy = (q & 1) ? Y1 : Y0;
+        t[0] = wx * wy;
+        t[1] = (double)r.z * t[0];
+        t[2] = t[3] = t[4] = t[5] = 0.0;
+        if (wx > 0.5 && wy > 0.5) {
+            t[2] = 4.0 * (wx - 0.5) * (wy - 0.5);
+            t[3] = lnu * t[2];
+        }
+        if (c == 0) {
+            const double dx = 1.0 - fabs(X0 - 0.5), dy = 1.0 - fabs(Y0 - 0.5);
+            if (dx > 0.5 && dy > 0.5) {
+                t[4] = 4.0 * (dx - 0.5) * (dy - 0.5);
+                t[5] = lnu * t[4];
+            }
+        }
+    };
+    auto each = [&](auto &&fn) {
+        for (int c = 0; c < 4; c++) {
+            const int c1 = m1 - 1 + (c >> 1), c2 = m2 - 1 + (c & 1);
+            if (c1 < 0 || c2 < 0 || c1 >= P.nc1 || c2 >= P.nc2) continue;
+            const int64_t cell = (int64_t)c1 * P.nc2 + c2;
+            const int32_t n = P.count[cell], nb = min(n, P.cap);
+            for (int t = lane; t < nb; t += 32) {
+                const float4 r = P.ra[rec_place((int32_t)cell, t, P.cap)];
+                fn(c, r, rec_lnu(r));
+            }
+            if (n > nb)
+                for (int o = lane; o < novf; o += 32)
+                    if (P.ovf[o].cell == (int32_t)cell) fn(c, P.ovf[o].a, rec_lnu(P.ovf[o].a));
+        }
+    };
+    double mx[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    int nrec = 0;
+    each([&](int c, float4 r, double lnu) {
+        double t[6];
+        terms(c, r, lnu, t);
+        for (int k = 0; k < 6; k++) mx[k] = fmax(mx[k], fabs(t[k]));
+        nrec++;
+    });
+    for (int o = 16; o > 0; o >>= 1) {
+        for (int k = 0; k < 6; k++) mx[k] = fmax(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+        nrec += __shfl_xor_sync(0xffffffffu, nrec, o);
+    }
+    double cq[6];
+    for (int k = 0; k < 6; k++) {
+        const double b = (double)(nrec > 0 ? nrec : 1) * mx[k];
+        cq[k] = ldexp(1.5, b > 0 ? ilogb(b) + 1 : 0);
+    }
+    double S[NV];
+    for (int k = 0; k < NV; k++) S[k] = 0.0;
+    each([&](int c, float4 r, double lnu) {
+        double t[6];
+        terms(c, r, lnu, t);
+        const double wq = (t[0] + cq[0]) - cq[0];
+        const int slot = rec_slot(r);
+        for (int k = 0; k < NT; k++)
+            if (slot == k) S[k] += wq;
+        if (!rec_immobile(r)) {
+            S[NT] += wq;
+            S[NT + 1] += (t[1] + cq[1]) - cq[1];
+        }
+        S[NT + 2] += (t[3] + cq[3]) - cq[3];
+        S[NT + 3] += (t[2] + cq[2]) - cq[2];
+        S[NT + 4] += (t[5] + cq[5]) - cq[5];
+        S[NT + 5] += (t[4] + cq[4]) - cq[4];
+    });
+    for (int o = 16; o > 0; o >>= 1)
+        for (int k = 0; k < NV; k++) S[k] += __shfl_xor_sync(0xffffffffu, S[k], o);
+    if (lane == 0) node_write<NT>(P, m3, S, range->lo, range->hi, range->any);
 }
 
 // One CTA: node rows [d0, d0 + ROWS - 1) x node columns [cs, cs + ncol).  In group g
@@ -1117,29 +1179,42 @@ __global__ void __launch_bounds__(kCnThreads, 2) k_cellnodes(const __grid_consta
         __syncthreads();
         for (int t = threadIdx.x; t < kCnCols * ROWS; t += kCnThreads) {
             const int col = t / ROWS, row = t % ROWS, m1 = cs - 1 + kCnCols * g + col, m2 = d0 - 1 + row;
-            if (row < 1 || m1 < cs || m1 >= cs + P.ncol || m1 >= P.nx || m2 >= P.ny) continue;
-            // cells (m1, m2), (m1, m2 - 1), (m1 - 1, m2), (m1 - 1, m2 - 1): corners 0..3
-            const double *c0 = &M.v[0][col + 1][row], *c1 = c0 - 1, *c2 = c0 - ROWS, *c3 = c2 - 1;
-            double Sv[NodeVals<NT>::N];
-            double w1 = 0.0;
+            bool small = false;
+            if (row >= 1 && m1 >= cs && m1 < cs + P.ncol && m1 < P.nx && m2 < P.ny) {
+                // cells (m1, m2), (m1, m2 - 1), (m1 - 1, m2), (m1 - 1, m2 - 1): corners 0..3
+                const double *c0 = &M.v[0][col + 1][row], *c1 = c0 - 1, *c2 = c0 - ROWS, *c3 = c2 - 1;
+                double Sv[NodeVals<NT>::N];
+                double w1 = 0.0;
 #pragma unroll
-            for (int k = 0; k <= NT; k++) {
-                const int at = 4 * k * CS;
-                const double w = 0.25 * ((corner4<0>(c0 + at, CS) + corner4<1>(c1 + at, CS)) +
-                                         (corner4<2>(c2 + at, CS) + corner4<3>(c3 + at, CS)));
-                if (k < NT) {
-                    Sv[k] = w;
-                    if ((P.mob >> k) & 1u) w1 += w;
-                } else {
-                    Sv[NT + 1] = w;  // T
+                for (int k = 0; k <= NT; k++) {
+                    const int at = 4 * k * CS;
+                    const double w = 0.25 * ((corner4<0>(c0 + at, CS) + corner4<1>(c1 + at, CS)) +
+                                             (corner4<2>(c2 + at, CS) + corner4<3>(c3 + at, CS)));
+                    if (k < NT) {
+                        Sv[k] = w;
+                        if ((P.mob >> k) & 1u) w1 += w;
+                    } else {
+                        Sv[NT + 1] = w;  // T
+                    }
+                }
+                Sv[NT] = w1;
+                Sv[NT + 2] = (c0[C::NU * CS] + c1[(C::NU + 1) * CS]) + (c2[(C::NU + 2) * CS] + c3[(C::NU + 3) * CS]);
+                Sv[NT + 3] = (c0[C::WNU * CS] + c1[(C::WNU + 1) * CS]) + (c2[(C::WNU + 2) * CS] + c3[(C::WNU + 3) * CS]);
+                Sv[NT + 4] = c3[C::ND * CS];
+                Sv[NT + 5] = c3[C::WND * CS];
+                small = node_finish<NT>(P, Q, m1, m2, Sv, vmin, vmax, any);
+            }
+            // the warp's nodes with small sums, one after the other
+            for (unsigned f = __ballot_sync(0xffffffffu, small); f; f &= f - 1) {
+                const int from = __ffs(f) - 1;
+                ViscRange r{0.0, 0.0, 0};
+                node_guard<NT>(P, __shfl_sync(0xffffffffu, m1, from), __shfl_sync(0xffffffffu, m2, from), &r);
+                if (r.any) {
+                    vmin = any ? fmin(vmin, r.lo) : r.lo;
+                    vmax = any ? fmax(vmax, r.hi) : r.hi;
+                    any = 1;
                 }
             }
-            Sv[NT] = w1;
-            Sv[NT + 2] = (c0[C::NU * CS] + c1[(C::NU + 1) * CS]) + (c2[(C::NU + 2) * CS] + c3[(C::NU + 3) * CS]);
-            Sv[NT + 3] = (c0[C::WNU * CS] + c1[(C::WNU + 1) * CS]) + (c2[(C::WNU + 2) * CS] + c3[(C::WNU + 3) * CS]);
-            Sv[NT + 4] = c3[C::ND * CS];
-            Sv[NT + 5] = c3[C::WND * CS];
-            node_finish<NT>(P, Q, m1, m2, Sv, vmin, vmax, any);
         }
         if (g + 1 == groups) break;
         // the last column becomes the next group's column 0
@@ -1159,122 +1234,50 @@ __global__ void __launch_bounds__(kCnThreads, 2) k_cellnodes(const __grid_consta
     fold_minmax(vmin, vmax, any, P.ctr, owned, P.navg);
 }
 
-// Nodes listed by k_cellnodes, a warp each: the records of the node's four cells
-// once for the largest terms, once more with quanta fitted to this node (so the
-// sums are exact again, at a resolution of 2^-52 of the node's own largest
-// terms), then the node as node_write makes it.
-template <int NT>
-__global__ void __launch_bounds__(128) k_node_guard(const __grid_constant__ CellNodesArgs P)
-{
-    slot_heat_init(P);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int ng = P.ctr->nguard, novf = P.ctr->novf;
-    const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    double vmin = 0.0, vmax = 0.0;
-    int any = 0;
-    constexpr int NV = NT + 6;
-    for (int64_t gi = warp0; gi < ng; gi += nwarps) {
-        const int64_t m3 = P.guard[gi];
-        const int m1 = (int)(m3 / P.ny), m2 = (int)(m3 - (int64_t)m1 * P.ny);
-        // the terms of a record of cell c (c = 0..3: cells (m1-1, m2-1), (m1-1, m2),
-        // (m1, m2-1), (m1, m2)), which reaches the node through its corner 3 - c:
-        // t[0] weight, t[1] T x weight, t[2] quadrant weight, t[3] its
-        // log-viscosity term, t[4] centre weight, t[5] its term
-        auto terms = [&](int c, float4 r, double lnu, double *t) {
-            const int q = 3 - c;
-            const double X1 = weight_of(__float_as_uint(r.x)), Y1 = weight_of(__float_as_uint(r.y));
-            const double X0 = 1.0 - X1, Y0 = 1.0 - Y1;
-            const double wx = (q >> 1) ? X1 : X0, wy = (q & 1) ? Y1 : Y0;
-            t[0] = wx * wy;
-            t[1] = (double)r.z * t[0];
-            t[2] = t[3] = t[4] = t[5] = 0.0;
-            if (wx > 0.5 && wy > 0.5) {
-                t[2] = 4.0 * (wx - 0.5) * (wy - 0.5);
-                t[3] = lnu * t[2];
-            }
-            if (c == 0) {
-                const double dx = 1.0 - fabs(X0 - 0.5), dy = 1.0 - fabs(Y0 - 0.5);
-                if (dx > 0.5 && dy > 0.5) {
-                    t[4] = 4.0 * (dx - 0.5) * (dy - 0.5);
-                    t[5] = lnu * t[4];
-                }
-            }
-        };
-        auto each = [&](auto &&fn) {
-            for (int c = 0; c < 4; c++) {
-                const int c1 = m1 - 1 + (c >> 1), c2 = m2 - 1 + (c & 1);
-                if (c1 < 0 || c2 < 0 || c1 >= P.nc1 || c2 >= P.nc2) continue;
-                const int64_t cell = (int64_t)c1 * P.nc2 + c2;
-                const int32_t n = P.count[cell], nb = min(n, P.cap);
-                for (int t = lane; t < nb; t += 32) {
-                    const float4 r = P.ra[rec_place((int32_t)cell, t, P.cap)];
-                    fn(c, r, rec_lnu(r));
-                }
-                if (n > nb)
-                    for (int o = lane; o < novf; o += 32)
-                        if (P.ovf[o].cell == (int32_t)cell) fn(c, P.ovf[o].a, rec_lnu(P.ovf[o].a));
-            }
-        };
-        double mx[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        int nrec = 0;
-        each([&](int c, float4 r, double lnu) {
-            double t[6];
-            terms(c, r, lnu, t);
-            for (int k = 0; k < 6; k++) mx[k] = fmax(mx[k], fabs(t[k]));
-            nrec++;
-        });
-        for (int o = 16; o > 0; o >>= 1) {
-            for (int k = 0; k < 6; k++) mx[k] = fmax(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-            nrec += __shfl_xor_sync(0xffffffffu, nrec, o);
-        }
-        double cq[6];
-        for (int k = 0; k < 6; k++) {
-            const double b = (double)(nrec > 0 ? nrec : 1) * mx[k];
-            cq[k] = ldexp(1.5, b > 0 ? ilogb(b) + 1 : 0);
-        }
-        double S[NV];
-        for (int k = 0; k < NV; k++) S[k] = 0.0;
-        each([&](int c, float4 r, double lnu) {
-            double t[6];
-            terms(c, r, lnu, t);
-            const double wq = (t[0] + cq[0]) - cq[0];
-            const int slot = rec_slot(r);
-            for (int k = 0; k < NT; k++)
-                if (slot == k) S[k] += wq;
-            if (!rec_immobile(r)) {
-                S[NT] += wq;
-                S[NT + 1] += (t[1] + cq[1]) - cq[1];
-            }
-            S[NT + 2] += (t[3] + cq[3]) - cq[3];
-            S[NT + 3] += (t[2] + cq[2]) - cq[2];
-            S[NT + 4] += (t[5] + cq[5]) - cq[5];
-            S[NT + 5] += (t[4] + cq[4]) - cq[4];
-        });
-        for (int o = 16; o > 0; o >>= 1)
-            for (int k = 0; k < NV; k++) S[k] += __shfl_xor_sync(0xffffffffu, S[k], o);
-        if (lane == 0) node_write<NT>(P, m3, S, vmin, vmax, any);
-    }
-    fold_minmax(vmin, vmax, any, P.ctr);
-}
-
-// Start of a fused averaging call: the call's counters, the markers' averaged
-// count, and the sticky-air temperature resets k_move_fused recorded.
-static __global__ void k_fused_begin(MarkerView M, FusedCounters *ctr, const int32_t *__restrict__ treset, double tmp_ambient,
-                              unsigned long long *navg)
+// Start of a fused averaging call: the call's counters, and the work k_move_fused left
+// for it (first: not done by an earlier call on the same records): the sticky-air
+// temperature resets, and the markers it kept a place for, whose viscosity comes
+// from the rheology at the new position (allintere + viscalc, markmart.c:281,
+// 320-332) into their records' log-viscosity and the call's |log-viscosity| bound.
+template <bool MIXED>
+__global__ void __launch_bounds__(256) k_fused_begin(const __grid_constant__ GridView G,
+                                                     const __grid_constant__ MarkerView M,
+                                                     const DevTypes *__restrict__ Ty,
+                                                     const __grid_constant__ FusedMove F, int32_t first,
+                                                     unsigned long long *navg)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ctr->nguard = 0;
-        ctr->any = 0;
-        ctr->kmin = ~0ull;
-        ctr->kmax = 0ull;
+        F.ctr->any = 0;
+        F.ctr->kmin = ~0ull;
+        F.ctr->kmax = 0ull;
         if (navg) *navg = 0ull;  // k_cellnodes counts the averaged markers
     }
-    if (!treset) return;  // applied by an earlier call on the same records
-    const int32_t m = ctr->ntreset;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x)
-        M.T[treset[q]] = tmp_ambient;
+    if (!first) return;
+    const int32_t resets = F.ctr->ntreset, m = F.ctr->ndefer;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, q0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t q = q0; q < resets; q += stride) M.T[F.treset[q]] = F.avg.tmp_ambient;
+    if (m == 0) return;
+    AvgArgsK V = F.avg;  // viscalc's impact weakening reads timesum (markmart.c:1886-1889)
+    if (F.stepc) V.timesum = F.stepc[4 * *F.stepi];
+    for (int64_t q = q0; q < m; q += stride) {
+        const int2 d = F.defer[q];
+        const int64_t i = d.x;
+        const double x = M.x[i], y = M.y[i];
+        const int mt = M.type[i];
+        const double mtk = mt < 2 ? V.tmp_ambient : M.T[i];
+        double pr = 0.0, mga = 0.0, mnu = 0.0;
+        int64_t m10, m20;
+        pressure_visc<MIXED>(G, Ty->t, V, x, y, mtk, M.hi ? M.hi[i] : 0.0, mt, false, true, pr, mga, mnu, m10, m20);
+        const double lnu = record_lnu(G, V, x, y, mnu);
+        if (d.y >= 0) {
+            F.ra[d.y] = rec_with_lnu(F.ra[d.y], lnu);
+        } else {
+            OvfRec &r = F.ovf[-d.y - 1];
+            r.a = rec_with_lnu(r.a, lnu);
+            r.lnu = lnu;
+        }
+        atomicMax(&F.ctr->part[q % kFusedParts][2], __float_as_uint(__double2float_ru(fabs(lnu))));
+    }
 }
 
 // marktmax (markmart.c:354-360) on a fused averaging call

@@ -203,7 +203,8 @@ struct FusedLaunch {
     FusedCounters *ctr;
     int32_t *treset;      // [markers]
     int2 *defer;          // [markers]
-    int32_t *guard;       // [nodes]
+    int32_t *spilled;     // mapped host memory: a call overflowed a bucket
+    bool first;           // averaging: the first call on these records
     uint8_t tinfo[50];    // per rock type < 50: slot | immobile << 2
     int32_t nt;           // slots in use, 1..kFusedSlots
     double sv[kFusedSlots][4];  // per slot: ro, cp, kt, ht of this call
@@ -221,7 +222,6 @@ struct FusedLaunch {
     bool track_tmax;
 };
 size_t fused_counters_bytes();
-size_t fused_move_counters_bytes();  // the leading part k_move_fused needs zeroed
 size_t fused_ovf_bytes();            // bytes of one overflow record
 // largest cell count and overflow count from a host copy of the counters
 void fused_host_stats(const void *counters, int32_t *count_max, int32_t *novf);

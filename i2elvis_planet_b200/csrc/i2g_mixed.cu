@@ -140,7 +140,6 @@ int launch_tanti_mixed(const StepLaunch &L, const double *sol1)
 
 // ----------------------------------------------------------------- fused step
 size_t fused_counters_bytes() { return sizeof(FusedCounters); }
-size_t fused_move_counters_bytes() { return offsetof(FusedCounters, nguard); }
 size_t fused_ovf_bytes() { return sizeof(OvfRec); }
 
 void fused_host_stats(const void *counters, int32_t *count_max, int32_t *novf)
@@ -163,6 +162,7 @@ static FusedMove fused_move_args(const GridView &G, const AvgArgsK &V, const Fus
     M.ovf = F.ovf;
     M.count = F.count;
     M.ctr = F.ctr;
+    M.spilled = F.spilled;
     M.treset = F.treset;
     M.defer = F.defer;
     M.stepc = F.stepc;
@@ -198,8 +198,7 @@ int launch_move_fused(const StepLaunch &L, const MoveArgs &A, const AvgArgsK &V,
     else if (visc) move_fused<true, false>(L, A, M);
     else if (uni) move_fused<false, true>(L, A, M);
     else move_fused<false, false>(L, A, M);
-    k_fused_deferred<true><<<148, 128, 0, L.stream>>>(L.G, L.M, L.types, M);
-    return 2;
+    return 1;
 }
 
 template <int NT, int S>
@@ -245,15 +244,14 @@ static int cellnodes(const StepLaunch &L, const CellNodesArgs &P)
         }
         cellnodes_shape<NT, 1>(L, P, best);
     }
-    k_node_guard<NT><<<148, 128, 0, L.stream>>>(P);
-    return 2;
+    return 1;
 }
 
 int launch_avg_fused(const StepLaunch &L, const AvgArgsK &V, const FusedLaunch &F, const NodeOut &O)
 {
     int nl = 0;
     const int64_t nn = L.G.nx * L.G.ny;
-    k_fused_begin<<<148, 256, 0, L.stream>>>(L.M, F.ctr, F.treset, V.tmp_ambient, F.navg);
+    k_fused_begin<true><<<148, 256, 0, L.stream>>>(L.G, L.M, L.types, fused_move_args(L.G, V, F), F.first ? 1 : 0, F.navg);
     nl++;
     if (F.track_tmax && L.M.tmax && L.M.n > 0) {
         AvgArgsK V2 = V;
@@ -286,7 +284,6 @@ int launch_avg_fused(const StepLaunch &L, const AvgArgsK &V, const FusedLaunch &
     P.nuend = V.nuend;
     P.mu = L.G.mu;
     P.O = O;
-    P.guard = F.guard;
     P.navg = F.navg;
     switch (F.nt) {
     case 1: nl += cellnodes<1>(L, P); break;
@@ -341,9 +338,7 @@ void preload_mixed()
     cudaFuncGetAttributes(&a, k_cellnodes<3, 2>);
     cudaFuncGetAttributes(&a, k_cellnodes<4, 1>);
     cudaFuncGetAttributes(&a, k_cellnodes<4, 2>);
-    cudaFuncGetAttributes(&a, k_node_guard<3>);
-    cudaFuncGetAttributes(&a, k_fused_deferred<true>);
-    cudaFuncGetAttributes(&a, k_fused_begin);
+    cudaFuncGetAttributes(&a, k_fused_begin<true>);
     cudaFuncGetAttributes(&a, k_fused_clamp);
 }
 
