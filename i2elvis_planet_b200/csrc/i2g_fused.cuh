@@ -92,6 +92,19 @@ __device__ __forceinline__ int floor_fm(float u, float &fl)
     return __float_as_int(s) - 0x4B400000;
 }
 __device__ __forceinline__ float flt_of(int d) { return __int_as_float(0x4B400000 + d) - kF32Magic; }  // |d| < 2^22
+// max and min that pass a NaN on, as "if (e < lo) e = lo" does, in one instruction
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float min_nan(float a, float b)
+{
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
 // The stencil choice and weights of one axis (AxisF) on a uniform axis: b1 is the
 // coordinate inside basic cell b in cells; the staggered stencil is the lower or
 // upper neighbour by the half-cell, clamped to [0, n-3], with its weight
@@ -143,14 +156,14 @@ __device__ __forceinline__ void uni_stage(const AxisRK &R, float e, float fiw, i
 // cell.  fiw2 = 2 / width.
 __device__ __forceinline__ void uni_half(const AxisRK &R, float e, float fiw2, int nh, int &h, float &f)
 {
-    if (e < R.lo) e = R.lo;
-    if (e > R.hi) e = R.hi;
+    e = min_nan(max_nan(e, R.lo), R.hi);
     const float s = e * fiw2;
     float fl;
     const int k0 = 2 * R.b + floor_fm(s, fl);
     const int k = min(max(k0, 0), nh - 1);
     h = k;
-    f = s - (fl - flt_of(k0 - k));  // s - (float)(k - 2 R.b)
+    f = s - fl;
+    if (k != k0) f = s - (fl - flt_of(k0 - k));  // s - (float)(k - 2 R.b); at the box's edge
 }
 
 // vx and vy at a point of quarter cell (hx, hy) with coordinates (fx, fy) in it,
@@ -240,6 +253,9 @@ __device__ __forceinline__ unsigned lane_lt()
 constexpr uint32_t kWeightMask = 0x1FFFFFFu;
 constexpr uint32_t kRecImmobile = 1u << 29;
 constexpr int kRecSlotShift = 30;
+// What k_move_fused reads per rock type, a byte: rec_type_byte of an averaged type, and
+// bit 0 for a type that movemark leaves where it is (markim)
+constexpr int kMoveTypes = 128;
 // tinfo[] of a rock type (slot | immobile << 2) as the y word's top byte has it
 __host__ __device__ constexpr uint8_t rec_type_byte(uint8_t tinfo)
 {
@@ -247,9 +263,9 @@ __host__ __device__ constexpr uint8_t rec_type_byte(uint8_t tinfo)
 }
 __device__ __forceinline__ uint32_t weight_fix(double w)
 {
-    w = w < 0.0 ? 0.0 : (w > 1.0 ? 1.0 : w);
-    // w 2^24 + 2^52 rounds to nearest-even at unit resolution: __double2uint_rn(w 2^24)
-    return (uint32_t)__double2loint(fma(w, 0x1p24, 0x1p52));
+    // w 2^24 + 1.5 x 2^52 rounds to nearest-even at unit resolution, its low word the
+    // signed result: __double2int_rn(w 2^24), held to [0, 2^24]
+    return (uint32_t)min(max(__double2loint(fma(w, 0x1p24, 0x1.8p52)), 0), 1 << 24);
 }
 __device__ __forceinline__ double weight_of(uint32_t word)
 {
@@ -307,9 +323,9 @@ struct FusedStat {
 // the warp calls it together (the bucket places are claimed per warp).
 template <bool VISC, bool UNI>
 __device__ __forceinline__ void move_record(const GridView &G, const MarkerView &M, const i2g_types &T,
-                                            const MoveArgs &A, const FusedMove &F, const ViscType *VT, int64_t i,
-                                            bool live, int mt, double x, double y, const double Tm, double eta,
-                                            FusedStat &st)
+                                            const MoveArgs &A, const FusedMove &F, const ViscType *VT,
+                                            const uint8_t *type, int64_t i, bool live, int mt, double x, double y,
+                                            const double Tm, double eta, FusedStat &st)
 {
     const int lane = threadIdx.x & 31;
     bool ok = false, defer = false;
@@ -323,7 +339,8 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
         // again)
         const bool inbox = (x >= 0 && y >= 0 && x <= G.xsize && y <= G.ysize);
         int hx = -1, hy = -1;
-        if ((inbox || A.outgrid != 1) && !T.markim[mt]) {
+        bool moved = false;
+        if ((inbox || A.outgrid != 1) && !(type[mt] & 1u)) {
             double pr, vx0, vy0;
             AxisF X1, Y1;
             if (UNI) {
@@ -341,7 +358,7 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
                 strain_mixed(G, x, y, X1, Y1, e);
                 eta = visc_update_mixed(M, T, VT[mt < 20 ? mt : min(mt - 20, kAvgTypes - 1)], A, i, mt, Tm, eta, pr, e);
             }
-            if (A.outgrid == 2) {
+            if (A.outgrid == 2 && !inbox) {
                 if (x < 0 || x > G.xsize) vy0 = 0;
                 if (y < 0 || y > G.ysize) vx0 = 0;
             }
@@ -349,12 +366,13 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
             y = advance(y, A.timestep, vy0, A.f32pos);
             M.x[i] = x;
             M.y[i] = y;
-            if (x < 0 || y < 0 || x > G.xsize || y > G.ysize) M.T[i] = 0;
+            moved = true;
         }
         // the averaging's filter at the new position (markmart.c:277)
         const AvgArgsK &V = F.avg;
-        ok = x > 0 && y > 0 && x < G.xsize && y < G.ysize && Tm > 0 && mt < kAvgTypes &&
-             (V.gridmod <= 1 || (M.id[i] % V.gridmod) == 0);
+        const bool inner = x > 0 && y > 0 && x < G.xsize && y < G.ysize;
+        if (!inner && moved && (x < 0 || y < 0 || x > G.xsize || y > G.ysize)) M.T[i] = 0;
+        ok = inner && Tm > 0 && mt < kAvgTypes && (V.gridmod <= 1 || (M.id[i] % V.gridmod) == 0);
         if (ok) {
             if (UNI) {
                 bx = min(max(floor_dm((x - G.gx0) * G.iwx), 0), (int)G.nx - 2);
@@ -396,7 +414,7 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
         // viscalc in k_fused_begin (a place is kept for it here)
         lnu = eta > 0 ? record_lnu(G, V, x, y, eta) : 0.0;
         defer = !(eta > 0);
-        rec = rec_pack(weight_fix(wx1), weight_fix(wy1), (float)mtk, (uint32_t)F.type[mt], lnu);
+        rec = rec_pack(weight_fix(wx1), weight_fix(wy1), (float)mtk, (uint32_t)(type[mt] & 0xFEu), lnu);
     }
     uint32_t cnt = 0;
     if (ok) {
@@ -480,8 +498,10 @@ __device__ __forceinline__ void move_stage_issue(const MarkerView &M, MoveStage 
 // viscosity update a thread reads the marker its class order gives it, behind the
 // order's barriers.  Viscosity update, nonuniform grid, 4M markers: 564 us with
 // viscalc's own expressions and searches and walks by the whole axis, 348 with
-// viscalc_mixed and the class order, 284 with the axis bins and branch-free stage steps
-// (235 -> 170 of it without the update); two or three CTAs per SM 401, five 350.
+// viscalc_mixed and the class order, 284 with the axis bins and branch-free stage steps;
+// two or three CTAs per SM 401, five 350.  Uniform grid without the update, 401^2 nodes,
+// 642k markers: 69.0 -> 67.0 us and 624 -> 604 instructions per warp and tile with the
+// types' flags in shared memory, the box tests shared, and clamps of one instruction.
 template <bool VISC, bool UNI>
 __global__ void __launch_bounds__(kMoveTile, VISC ? 4 : 4) k_move_fused(const __grid_constant__ GridView G,
                                                     const __grid_constant__ MarkerView M,
@@ -494,10 +514,11 @@ __global__ void __launch_bounds__(kMoveTile, VISC ? 4 : 4) k_move_fused(const __
     __shared__ ViscType VT[VISC ? kAvgTypes : 1];
     __shared__ uint8_t order[kMoveTile], types[kMoveTile];
     __shared__ int cnt[kMoveTile / 32][4];
-    if (VISC) {
-        if (threadIdx.x < kAvgTypes) VT[threadIdx.x] = visc_type(Ty->t, threadIdx.x);
-        __syncthreads();
-    }
+    __shared__ uint8_t type[kMoveTypes];
+    if (VISC && threadIdx.x < kAvgTypes) VT[threadIdx.x] = visc_type(Ty->t, threadIdx.x);
+    if (threadIdx.x < kMoveTypes)
+        type[threadIdx.x] = (threadIdx.x < kAvgTypes ? F.type[threadIdx.x] : 0) | (Ty->t.markim[threadIdx.x] ? 1 : 0);
+    __syncthreads();
     const i2g_types &T = Ty->t;
     const int tid = threadIdx.x;
     const int ntiles = (int)((M.n + kMoveTile - 1) / kMoveTile);
@@ -529,7 +550,7 @@ __global__ void __launch_bounds__(kMoveTile, VISC ? 4 : 4) k_move_fused(const __
             Tm = S[b].v[2][mine];
             eta = S[b].v[3][mine];
         }
-        move_record<VISC, UNI>(G, M, T, A, F, VT, i, live, mt, x, y, Tm, eta, st);
+        move_record<VISC, UNI>(G, M, T, A, F, VT, type, i, live, mt, x, y, Tm, eta, st);
         if (VISC) __syncthreads();  // the tile's stage and order are done with
     }
     cp_async_wait<0>();
