@@ -81,7 +81,7 @@ struct i2g_ctx {
     int32_t *ndeferred = nullptr;   // device: markers deferred to the general property model
     uint8_t *tconst = nullptr;      // device: per-type table of a constant-property averaging call
     int *typecheck_host = nullptr;  // pinned mirror, read after the set call's final sync
-    int32_t TX = 16;  // averaging tile: cell columns (x 32 cell rows)
+    int32_t TX = 16;  // averaging tile: cell columns (x 32 cell rows), cellsum_cols()
     unsigned long long *navg = nullptr;
     DevTypes *dtypes = nullptr;
     int64_t nsorts = 0;
@@ -268,6 +268,27 @@ struct PhaseTimer {
         c->pending.push_back({phase, a, b});
     }
 };
+
+// Cell columns per tile of k_cellsums (8 warps, a column each at a time; two CTAs per
+// SM): the tiles take ceil(tiles / resident) waves of that many columns, so the
+// width with the fewest column-waves; ties go to the wider.  401^2 nodes, FP64 form:
+// 16 columns, 325 tiles in two waves, 62.8 us; 8 columns, 650 in three, 53.2.  201^2,
+// one wave of either: FP64 form 27.0 -> 20.0 us, mixed 21.0 -> 16.0.  Any width gives
+// the same sums.
+int32_t cellsum_cols(int64_t nc1, int64_t nc2, int sms)
+{
+    int32_t best = 8;
+    int64_t cost = INT64_MAX;
+    for (int32_t tx : {8, 16, 32}) {
+        const int64_t tiles = ((nc1 + tx - 1) / tx) * ((nc2 + 31) / 32), resident = 2 * (int64_t)sms;
+        const int64_t c = (tiles + resident - 1) / resident * tx;
+        if (c <= cost) {
+            cost = c;
+            best = tx;
+        }
+    }
+    return best;
+}
 
 // The tables of one axis of n lines, side by side in one block: pairs of lines and
 // of midpoints, {width, 1/width, 1/mid spacing} and its parts in FP32, lines,
@@ -656,6 +677,9 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
         return r;
     };
     if (cudaSetDevice(c->dev) != cudaSuccess) return bail(I2G_ECUDA);
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
+    c->TX = cellsum_cols(c->nx - 1, c->ny - 1, sms);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(I2G_ECUDA);
     c->own_stream = true;
     if (cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess) return bail(I2G_ECUDA);
