@@ -42,6 +42,7 @@ struct i2g_ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int64_t nx = 0, ny = 0, nn = 0, ncells = 0;
+    int64_t pitch = 0;  // doubles from one grid or node field to the next
     double *gx = nullptr, *gy = nullptr, *xmid = nullptr, *ymid = nullptr;
     uint8_t *lines = nullptr;  // the axes' tables below, one block (line_tables)
     LinePair *bpx = nullptr, *bpy = nullptr, *mpx = nullptr, *mpy = nullptr;
@@ -80,7 +81,13 @@ struct i2g_ctx {
     int *typecheck = nullptr;       // device: {bad-type bits, first bad marker}
     int32_t *ndeferred = nullptr;   // device: markers deferred to the general property model
     uint8_t *tconst = nullptr;      // device: per-type table of a constant-property averaging call
-    int *typecheck_host = nullptr;  // pinned mirror, read after the set call's final sync
+    // pinned host memory, one block: the set call's mirror of typecheck, the fused
+    // step's overflow flag, and room for small grids' tables and fields (kStageBytes)
+    uint8_t *pinned = nullptr;
+    uint8_t *stage = nullptr;
+    int64_t stage_bytes = 0;
+    int *typecheck_host = nullptr;
+    bool gzero[G_N] = {};  // the field is zero on the device
     int32_t TX = 16;  // averaging tile: cell columns (x 32 cell rows), cellsum_cols()
     unsigned long long *navg = nullptr;
     DevTypes *dtypes = nullptr;
@@ -300,6 +307,15 @@ struct AxisTables {
     float *ib, *im;
     int32_t *bin;  // axis_bins(n) + 1 entries (GridView.binx)
 };
+
+// Grids whose tables and fields take this much or less cross through pinned memory of
+// the context in one copy each way: a coupled step (grid up, move, average, nodes back)
+// of 21^2 nodes 235 -> 104 us, 101^2 340 -> 167, 201^2 (4.1 MB) 540 -> 424.  At 301^2
+// (9.2 MB) the host's copies cost what the calls save: 821 -> 808, not worth the memory.
+constexpr int64_t kStageBytes = 5 << 20;
+// Fields in the caller's own pinned memory cross at full rate by themselves; theirs
+// are staged only while a field is this small, where the call costs more than its bytes
+constexpr int64_t kStagePinned = 64 << 10;
 
 int64_t line_bytes(int64_t n)
 {
@@ -623,8 +639,7 @@ int i2g_destroy(i2g_ctx *c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (void *p : c->allocs) cudaFree(p);
     if (c->fz.ra) cudaFree(c->fz.ra);
-    if (c->fz.spilled) cudaFreeHost(c->fz.spilled);
-    if (c->typecheck_host) cudaFreeHost(c->typecheck_host);
+    if (c->pinned) cudaFreeHost(c->pinned);
     for (auto &p : c->pending) {
         cudaEventDestroy(p.a);
         cudaEventDestroy(p.b);
@@ -668,6 +683,7 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
     c->nx = P->xnumx;
     c->ny = P->ynumy;
     c->nn = c->nx * c->ny;
+    c->pitch = (c->nn + 31) / 32 * 32;
     c->ncells = (c->nx - 1) * (c->ny - 1);
     c->cap = P->max_markers;
     c->fail_alloc_at = env_long("I2G_FAIL_ALLOC_AT");
@@ -687,19 +703,23 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return bail(I2G_ECUDA);
     int r = I2G_OK;
 #define A(p, n) if ((r = dalloc(c, &(p), (n))) != I2G_OK) return bail(r)
-    A(c->lines, line_bytes(c->nx) + line_bytes(c->ny));
+    // the axes' tables and the fields in one block, the node fields in another: a
+    // small grid crosses in one copy
+    const int64_t lb = (line_bytes(c->nx) + line_bytes(c->ny) + 255) / 256 * 256;
+    A(c->lines, lb + (int64_t)sizeof(double) * G_N * c->pitch);
+    for (int k = 0; k < G_N; k++) c->g[k] = reinterpret_cast<double *>(c->lines + lb) + k * c->pitch;
+    A(c->node[0], N_N * c->pitch);
+    for (int k = 1; k < N_N; k++) c->node[k] = c->node[0] + k * c->pitch;
     {
         const AxisTables X = axis_tables(c->lines, c->nx), Y = axis_tables(c->lines + line_bytes(c->nx), c->ny);
         c->bpx = X.bp; c->mpx = X.mp; c->lx = X.l; c->gx = X.g; c->xmid = X.mid; c->idx2 = X.id2; c->ixb = X.ib; c->ixm = X.im; c->binx = X.bin;
         c->bpy = Y.bp; c->mpy = Y.mp; c->ly = Y.l; c->gy = Y.g; c->ymid = Y.mid; c->idy2 = Y.id2; c->iyb = Y.ib; c->iym = Y.im; c->biny = Y.bin;
     }
-    for (int k = 0; k < G_N; k++) A(c->g[k], c->nn);
     if (P->precision == I2G_PREC_MIXED) {
         A(c->vxf, c->nn); A(c->vyf, c->nn); A(c->prf, c->nn); A(c->gaf, c->nn);
         A(c->vxq, c->nn); A(c->vyq, c->nn); A(c->prq, c->nn);
         for (int k = G_EXX; k <= G_SXY; k++) A(c->ef[k], c->nn);
     }
-    for (int k = 0; k < N_N; k++) A(c->node[k], c->nn);
     for (int b = 0; b < 2; b++) {
         MarkerBuf &m = c->mb[b];
         A(m.x, c->cap); A(m.y, c->cap); A(m.T, c->cap); A(m.eta, c->cap); A(m.p, c->cap);
@@ -734,22 +754,21 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
     A(c->td.melt, 12);
     A(c->sinter_stuck, 1);
 #undef A
-    if (cudaHostAlloc((void **)&c->typecheck_host, 8 * sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+    c->stage_bytes = lb + (int64_t)sizeof(double) * G_N * c->pitch;
+    if (c->stage_bytes > kStageBytes) c->stage_bytes = 0;
+    if (cudaHostAlloc((void **)&c->pinned, 256 + (size_t)c->stage_bytes, cudaHostAllocMapped) != cudaSuccess) {
         cudaGetLastError();
-        c->typecheck_host = nullptr;
+        c->pinned = nullptr;
         return bail(I2G_ENOMEM);
     }
-    if (P->precision == I2G_PREC_MIXED) {
-        if (cudaHostAlloc((void **)&c->fz.spilled, sizeof(int32_t), cudaHostAllocMapped) != cudaSuccess) {
-            cudaGetLastError();
-            c->fz.spilled = nullptr;
-            return bail(I2G_ENOMEM);
-        }
-        *c->fz.spilled = 0;
-        if (cudaHostGetDevicePointer((void **)&c->fz.spilled_dev, c->fz.spilled, 0) != cudaSuccess) return bail(I2G_ECUDA);
-    }
-    for (int k = 0; k < N_N; k++)
-        if (cudaMemsetAsync(c->node[k], 0, sizeof(double) * (size_t)c->nn, c->stream) != cudaSuccess) return bail(I2G_ECUDA);
+    c->typecheck_host = reinterpret_cast<int *>(c->pinned);
+    c->fz.spilled = reinterpret_cast<int32_t *>(c->pinned + 128);
+    c->stage = c->stage_bytes ? c->pinned + 256 : nullptr;
+    *c->fz.spilled = 0;
+    uint8_t *pinned_dev = nullptr;
+    if (cudaHostGetDevicePointer((void **)&pinned_dev, c->pinned, 0) != cudaSuccess) return bail(I2G_ECUDA);
+    c->fz.spilled_dev = reinterpret_cast<int32_t *>(pinned_dev + 128);
+    if (cudaMemsetAsync(c->node[0], 0, sizeof(double) * N_N * (size_t)c->pitch, c->stream) != cudaSuccess) return bail(I2G_ECUDA);
     if (cudaMemcpyAsync(&c->dtypes->t, T, sizeof(i2g_types), cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
         return bail(I2G_ECUDA);
     if (cudaMemsetAsync(c->stats, 0, 4 * sizeof(double), c->stream) != cudaSuccess) return bail(I2G_ECUDA);
@@ -780,6 +799,49 @@ int i2g_set_types(i2g_ctx *c, const i2g_types *T)
     return I2G_OK;
 }
 
+// Whether the caller's arrays go through the context's pinned memory: a small grid, every
+// non-NULL p[k] host memory (device memory is left to cudaMemcpy, which refuses it as
+// it always did), pinned only while small
+static bool staged_arrays(const i2g_ctx *c, const double *const *p, int k)
+{
+    if (!c->stage) return false;
+    const bool small = (int64_t)sizeof(double) * c->nn <= kStagePinned;
+    for (int a = 0; a < k; a++) {
+        if (!p[a]) continue;
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, p[a]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeUnregistered && !(at.type == cudaMemoryTypeHost && small)) return false;
+    }
+    return true;
+}
+
+// the mixed form's copies of the context's grid fields
+static GridForms grid_forms(const i2g_ctx *c)
+{
+    GridForms F{};
+    F.nx = c->nx;
+    F.ny = c->ny;
+    const int field[4] = {G_VX, G_VY, G_PR, G_GA};
+    float *out[4] = {c->vxf, c->vyf, c->prf, c->gaf};
+    int m = 0;
+    for (int k = 0; k < 4; k++, m++) {
+        F.in[m] = c->g[field[k]];
+        F.out[m] = out[k];
+    }
+    for (int k = G_EXX; k <= G_SXY; k++, m++) {
+        F.in[m] = c->g[k];
+        F.out[m] = c->gpresent[k] ? c->ef[k] : nullptr;
+    }
+    F.quad[0] = c->vxq;
+    F.quad[1] = c->vyq;
+    F.quad[2] = c->prq;
+    F.q4 = c->uni ? c->vq4 : nullptr;
+    return F;
+}
+
 int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *vx, const double *vy,
                  const double *pr, const double *exx, const double *eyy, const double *exy, const double *sxx,
                  const double *syy, const double *sxy, const double *ga, const double *mu)
@@ -791,8 +853,14 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
         if (!(gx[i] > gx[i - 1])) return fail(c, I2G_EINVAL, "gx must be strictly increasing");
     for (int64_t i = 1; i < ny; i++)
         if (!(gy[i] > gy[i - 1])) return fail(c, I2G_EINVAL, "gy must be strictly increasing");
-    std::vector<double> host((size_t)(line_bytes(nx) + line_bytes(ny)) / sizeof(double), 0.0);
-    uint8_t *hl = reinterpret_cast<uint8_t *>(host.data());
+    // the tables on the host: in the pinned room of a small grid (free between calls,
+    // which end synchronised), else in memory of their own
+    const size_t lbytes = (size_t)(line_bytes(nx) + line_bytes(ny));
+    const double *src[G_N] = {vx, vy, pr, exx, eyy, exy, sxx, syy, sxy, ga, mu};
+    const bool staged = staged_arrays(c, src, G_N);
+    std::vector<double> host(staged ? 0 : lbytes / sizeof(double), 0.0);
+    uint8_t *hl = staged ? c->stage : reinterpret_cast<uint8_t *>(host.data());
+    if (staged) memset(hl, 0, lbytes);
     const bool px = fill_axis(axis_tables(hl, nx), gx, nx), py = fill_axis(axis_tables(hl + line_bytes(nx), ny), gy, ny);
     c->pairs = px && py;
     c->inv_x = (double)(nx - 1) / (gx[nx - 1] - gx[0]);
@@ -816,28 +884,34 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
     c->uwx = uwx;
     c->uwy = uwy;
     c->fz.ready = false;
-    CK(cudaMemcpyAsync(c->lines, hl, (size_t)(line_bytes(nx) + line_bytes(ny)), cudaMemcpyHostToDevice, c->stream));
-    const double *src[G_N] = {vx, vy, pr, exx, eyy, exy, sxx, syy, sxy, ga, mu};
+    const size_t fb = sizeof(double) * (size_t)nn;
+    if (staged) {
+        // one copy: the tables and the fields up to the last one that changes
+        int last = G_N - 1;
+        while (last > 0 && !src[last] && c->gzero[last]) last--;
+        uint8_t *d = nullptr;
+        for (int k = 0; k <= last; k++) {
+            d = c->stage + (reinterpret_cast<uint8_t *>(c->g[k]) - c->lines);
+            if (src[k]) memcpy(d, src[k], fb);
+            else memset(d, 0, fb);
+        }
+        CK(cudaMemcpyAsync(c->lines, c->stage, (size_t)(d - c->stage) + fb, cudaMemcpyHostToDevice, c->stream));
+    } else {
+        CK(cudaMemcpyAsync(c->lines, hl, lbytes, cudaMemcpyHostToDevice, c->stream));
+        for (int k = 0; k < G_N; k++) {
+            if (src[k]) CK(cudaMemcpyAsync(c->g[k], src[k], fb, cudaMemcpyHostToDevice, c->stream));
+            else if (!c->gzero[k]) CK(cudaMemsetAsync(c->g[k], 0, fb, c->stream));
+        }
+    }
     for (int k = 0; k < G_N; k++) {
         c->gpresent[k] = src[k] != nullptr;
-        if (src[k]) CK(cudaMemcpyAsync(c->g[k], src[k], sizeof(double) * nn, cudaMemcpyHostToDevice, c->stream));
-        else CK(cudaMemsetAsync(c->g[k], 0, sizeof(double) * nn, c->stream));
+        c->gzero[k] = src[k] == nullptr;
     }
     if (c->P.precision == I2G_PREC_MIXED) {
-        launch_f64_to_f32(c->stream, nn, c->g[G_VX], c->vxf);
-        launch_f64_to_f32(c->stream, nn, c->g[G_VY], c->vyf);
-        launch_f64_to_f32(c->stream, nn, c->g[G_PR], c->prf);
-        launch_quads(c->stream, c->nx, c->ny, c->vxf, c->vxq);
-        launch_quads(c->stream, c->nx, c->ny, c->vyf, c->vyq);
-        launch_quads(c->stream, c->nx, c->ny, c->prf, c->prq);
         // a uniform grid's quarter-cell forms (indexed in int32 by the kernels)
-        if (c->uni && 8 * (c->nx - 1) * (c->ny - 1) < (int64_t)INT32_MAX) {
-            if (!c->vq4) TRY(dalloc(c, &c->vq4, 8 * (c->nx - 1) * (c->ny - 1)));
-            launch_quarters(c->stream, c->nx, c->ny, c->vxf, c->vyf, c->vq4);
-        }
-        launch_f64_to_f32(c->stream, nn, c->g[G_GA], c->gaf);
-        for (int k = G_EXX; k <= G_SXY; k++)
-            if (c->gpresent[k]) launch_f64_to_f32(c->stream, nn, c->g[k], c->ef[k]);
+        if (c->uni && 8 * (c->nx - 1) * (c->ny - 1) < (int64_t)INT32_MAX && !c->vq4)
+            TRY(dalloc(c, &c->vq4, 8 * (c->nx - 1) * (c->ny - 1)));
+        c->launches += launch_grid_forms(c->stream, grid_forms(c));
         CKL();
     }
     CK(cudaStreamSynchronize(c->stream));
@@ -917,8 +991,18 @@ static int get_nodes_impl(i2g_ctx *c, double *const *f, cudaMemcpyKind kind)
         CK(cudaStreamSynchronize(c->stream));
         return I2G_OK;
     }
+    const size_t fb = sizeof(double) * (size_t)c->nn, pb = sizeof(double) * (size_t)c->pitch;
+    if (kind == cudaMemcpyDeviceToHost && staged_arrays(c, f, N_N)) {
+        // a small grid: every field in one copy, then into the caller's arrays
+        static_assert(N_N <= G_N, "the node fields fit the room of the grid's");
+        CK(cudaMemcpyAsync(c->stage, c->node[0], N_N * pb, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        for (int k = 0; k < N_N; k++)
+            if (f[k]) memcpy(f[k], c->stage + k * pb, fb);
+        return I2G_OK;
+    }
     for (int k = 0; k < N_N; k++)
-        if (f[k]) CK(cudaMemcpyAsync(f[k], c->node[k], sizeof(double) * (size_t)c->nn, kind, c->stream));
+        if (f[k]) CK(cudaMemcpyAsync(f[k], c->node[k], fb, kind, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return I2G_OK;
 }
@@ -2115,13 +2199,10 @@ int i2g_adjoint_forward(i2g_ctx *c, const double *amps, int32_t nsteps, double t
         A.ck_segs = nseg;
     }
     CK(cudaMemcpyAsync(A.amps, amps, sizeof(double) * A.nm, cudaMemcpyHostToDevice, c->stream));
-    c->launches += launch_combine_modes(c->stream, c->nn, A.nm, mode_capacity(A.nm), A.mvx, A.mvy, A.amps, c->g[G_VX], c->g[G_VY],
-                                        c->vxf, c->vyf);
-    if (c->vxf) {
-        c->launches += launch_quads(c->stream, c->nx, c->ny, c->vxf, c->vxq);
-        c->launches += launch_quads(c->stream, c->nx, c->ny, c->vyf, c->vyq);
-        if (c->vq4) c->launches += launch_quarters(c->stream, c->nx, c->ny, c->vxf, c->vyf, c->vq4);
-    }
+    c->launches += launch_combine_modes(c->stream, c->nn, A.nm, mode_capacity(A.nm), A.mvx, A.mvy, A.amps, c->g[G_VX],
+                                        c->g[G_VY]);
+    if (c->vxf) c->launches += launch_grid_forms(c->stream, grid_forms(c));
+    c->gzero[G_VX] = c->gzero[G_VY] = false;
     c->gpresent[G_VX] = c->gpresent[G_VY] = true;
     if (!c->order_sorted) TRY(resort(c));
     const MarkerBuf &b = c->mb[c->cur];

@@ -281,14 +281,22 @@ struct AdjLaunch {
 };
 int launch_adjoint_fp64(const StepLaunch &L, const MoveArgs &A, const AdjLaunch &J);
 int launch_adjoint_mixed(const StepLaunch &L, const MoveArgs &A, const AdjLaunch &J);
-// vx = sum_m a_m mvx[.][m] (ld modes per node; FP64, fixed order), float copies when vxf != NULL
-int launch_quads(cudaStream_t s, int64_t nx, int64_t ny, const float *f, float4 *q);
 // allintert() at every marker (k_interp_tnode, FP64 in both forms): out[id], out2[id]
 int launch_interp_tnode(const StepLaunch &L, const double *tk, const double *tk2, double *out, double *out2);
-// the per-quarter-cell forms of vx and vy (GridView.vq4) of a uniform grid
-int launch_quarters(cudaStream_t s, int64_t nx, int64_t ny, const float *vxf, const float *vyf, float4 *q);
+// the mixed form's copies of the grid (k_grid_forms): FP64 fields in, FP32 copies
+// (NULL: none), stencil coefficients of in[0..2] (vx, vy, pr; NULL: none), and the
+// per-quarter-cell forms of vx and vy (NULL: none)
+constexpr int kGridCopies = 10;
+struct GridForms {
+    int64_t nx, ny;
+    const double *in[kGridCopies];
+    float *out[kGridCopies];
+    float4 *quad[3], *q4;
+};
+int launch_grid_forms(cudaStream_t s, const GridForms &F);
+// vx = sum_m a_m mvx[.][m] (ld modes per node; FP64, fixed order)
 int launch_combine_modes(cudaStream_t s, int64_t nn, int32_t nm, int32_t ld, const double *mvx, const double *mvy,
-                         const double *amps, double *vx, double *vy, float *vxf, float *vyf);
+                         const double *amps, double *vx, double *vy);
 int launch_ckpt(cudaStream_t s, const MarkerView &M, double2 *ck);
 int launch_sum_partials(cudaStream_t s, const double *part, int32_t nblk, int32_t nm, double *out);
 

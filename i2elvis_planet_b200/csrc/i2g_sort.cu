@@ -14,6 +14,8 @@
 //   k_fixup     order each cell's slots by caller index (the canonical order):
 //               perm2[slot] = marker and, when asked, rank[marker] = slot
 //   k_gather    move every marker field into its slot
+#include <algorithm>
+
 #include "i2g_launch.h"
 
 #include <cub/device/device_scan.cuh>
@@ -565,8 +567,7 @@ __global__ void k_t0(GridView G, MarkerView M, const int64_t *__restrict__ slot0
 // ------------------------------------------------------------- adjoint helpers
 __global__ void k_combine_modes(int64_t nn, int32_t nm, int32_t ld, const double *__restrict__ mvx,
                                 const double *__restrict__ mvy, const double *__restrict__ amps,
-                                double *__restrict__ vx, double *__restrict__ vy, float *__restrict__ vxf,
-                                float *__restrict__ vyf)
+                                double *__restrict__ vx, double *__restrict__ vy)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += stride) {
@@ -577,8 +578,6 @@ __global__ void k_combine_modes(int64_t nn, int32_t nm, int32_t ld, const double
         }
         vx[i] = a;
         vy[i] = b;
-        if (vxf) vxf[i] = (float)a;
-        if (vyf) vyf[i] = (float)b;
     }
 }
 
@@ -815,41 +814,38 @@ int launch_t0(cudaStream_t s, const GridView &G, const MarkerView &M, const int6
     return 1;
 }
 
-// bilinear coefficients of every 2x2 stencil at its lower-left node (GridView.vxq)
-__global__ void k_quads(int64_t nx, int64_t ny, const float *__restrict__ f, float4 *__restrict__ q)
-{
-    const int64_t m3 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (m3 >= nx * ny) return;
-    const int64_t m1 = m3 / ny, m2 = m3 - m1 * ny;
-    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (m1 + 1 < nx && m2 + 1 < ny) {
-        const float a = f[m3], b = f[m3 + 1], c = f[m3 + ny], d = f[m3 + ny + 1];
-        r = make_float4(a, c - a, b - a, (a - b) - (c - d));
-    }
-    q[m3] = r;
-}
-
-int launch_quads(cudaStream_t s, int64_t nx, int64_t ny, const float *f, float4 *q)
-{
-    const int64_t nn = nx * ny;
-    if (nn <= 0) return 0;
-    k_quads<<<blocks_for(nn, 256, INT32_MAX), 256, 0, s>>>(nx, ny, f, q);
-    return 1;
-}
-
-// Per quarter cell of a uniform grid (half a cell along each axis: hx = 2 i + qx,
-// hy = 2 j + qy), the bilinear forms of vx and vy in the quarter's coordinates
-// fx, fy in [0, 1]: the stencil the mixed RK4 takes there (vx basic in x and
-// staggered in y, vy staggered in x and basic in y; the staggered stencil is the
+// The mixed form's copies of the grid in one launch: FP32 fields, the bilinear
+// coefficients of every 2x2 stencil of vx, vy and pr at its lower-left node
+// (GridView.vxq), and on a uniform grid (q4) per quarter cell (half a cell along each
+// axis: hx = 2 i + qx, hy = 2 j + qy) the bilinear forms of vx and vy in the quarter's
+// coordinates fx, fy in [0, 1]: the stencil the mixed RK4 takes there (vx basic in x
+// and staggered in y, vy staggered in x and basic in y; the staggered stencil is the
 // lower neighbour in a lower half, clamped to [0, n - 3], markmart.c:1403-1437)
 // with X = ax + fx / 2, Y = ay + fy / 2 substituted into A + B X + C Y + D X Y,
-// in FP64 from the FP32 node values, rounded once.
-__global__ void k_quarters(int64_t nx, int64_t ny, const float *__restrict__ vxf, const float *__restrict__ vyf,
-                           float4 *__restrict__ q)
+// in FP64 from the FP32 node values, rounded once.  A thread per quarter and per node.
+__global__ void __launch_bounds__(256) k_grid_forms(const __grid_constant__ GridForms F)
 {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nx = F.nx, ny = F.ny;
+    if (t < nx * ny) {
+#pragma unroll
+        for (int k = 0; k < kGridCopies; k++)
+            if (F.out[k]) F.out[k][t] = (float)F.in[k][t];
+        const int64_t m1 = t / ny, m2 = t - m1 * ny;
+        const bool whole = m1 + 1 < nx && m2 + 1 < ny;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            if (!F.quad[k]) continue;
+            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (whole) {
+                const double *f = F.in[k] + t;
+                const float a = (float)f[0], b = (float)f[1], c = (float)f[ny], d = (float)f[ny + 1];
+                r = make_float4(a, c - a, b - a, (a - b) - (c - d));
+            }
+            F.quad[k][t] = r;
+        }
+    }
     const int64_t nhy = 2 * (ny - 1), nq = 2 * (nx - 1) * nhy;
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nq) return;
+    if (!F.q4 || t >= nq) return;
     const int64_t hx = t / nhy, hy = t - hx * nhy;
     const int64_t i = hx >> 1, j = hy >> 1;
     const int qx = (int)(hx & 1), qy = (int)(hy & 1);
@@ -859,30 +855,29 @@ __global__ void k_quarters(int64_t nx, int64_t ny, const float *__restrict__ vxf
         if (m > n - 3) m = n - 3;
         return m;
     };
-    auto form = [&](const float *f, int64_t s1, int64_t s2, double ax, double ay) {
-        const int64_t m3 = s1 * ny + s2;
-        const double a = f[m3], b = f[m3 + 1], c = f[m3 + ny], d = f[m3 + ny + 1];
+    auto form = [&](const double *g, int64_t s1, int64_t s2, double ax, double ay) {
+        const double *f = g + s1 * ny + s2;
+        const double a = (float)f[0], b = (float)f[1], c = (float)f[ny], d = (float)f[ny + 1];
         const double B = c - a, C = b - a, D = (a - b) - (c - d);
         return make_float4((float)(a + B * ax + C * ay + D * ax * ay), (float)(0.5 * (B + D * ay)),
                            (float)(0.5 * (C + D * ax)), (float)(0.25 * D));
     };
     const int64_t my = stag(j, qy, ny), mx = stag(i, qx, nx);
-    q[2 * t] = form(vxf, i, my, 0.5 * qx, (double)(j - my) - 0.5 + 0.5 * qy);
-    q[2 * t + 1] = form(vyf, mx, j, (double)(i - mx) - 0.5 + 0.5 * qx, 0.5 * qy);
+    F.q4[2 * t] = form(F.in[0], i, my, 0.5 * qx, (double)(j - my) - 0.5 + 0.5 * qy);
+    F.q4[2 * t + 1] = form(F.in[1], mx, j, (double)(i - mx) - 0.5 + 0.5 * qx, 0.5 * qy);
 }
 
-int launch_quarters(cudaStream_t s, int64_t nx, int64_t ny, const float *vxf, const float *vyf, float4 *q)
+int launch_grid_forms(cudaStream_t s, const GridForms &F)
 {
-    const int64_t nq = 4 * (nx - 1) * (ny - 1);
-    if (nq <= 0) return 0;
-    k_quarters<<<blocks_for(nq, 256, INT32_MAX), 256, 0, s>>>(nx, ny, vxf, vyf, q);
+    const int64_t n = std::max(F.nx * F.ny, F.q4 ? 4 * (F.nx - 1) * (F.ny - 1) : 0);
+    k_grid_forms<<<blocks_for(n, 256, INT32_MAX), 256, 0, s>>>(F);
     return 1;
 }
 
 int launch_combine_modes(cudaStream_t s, int64_t nn, int32_t nm, int32_t ld, const double *mvx, const double *mvy,
-                         const double *amps, double *vx, double *vy, float *vxf, float *vyf)
+                         const double *amps, double *vx, double *vy)
 {
-    k_combine_modes<<<blocks_for(nn, 256, 148 * 16), 256, 0, s>>>(nn, nm, ld, mvx, mvy, amps, vx, vy, vxf, vyf);
+    k_combine_modes<<<blocks_for(nn, 256, 148 * 16), 256, 0, s>>>(nn, nm, ld, mvx, mvy, amps, vx, vy);
     return 1;
 }
 
