@@ -739,7 +739,7 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
         uint8_t *ovf = nullptr;
         const int64_t cb = ((int64_t)fused_counters_bytes() + 255) / 256 * 256;
         A(ovf, (int64_t)fused_ovf_bytes() * (c->cap > 0 ? c->cap : 1));
-        c->fz.zero_bytes = cb + (int64_t)sizeof(int32_t) * c->ncells;
+        c->fz.zero_bytes = (cb + (int64_t)sizeof(int32_t) * c->ncells + 15) / 16 * 16;
         A(c->fz.zero, c->fz.zero_bytes);
         c->fz.ovf = reinterpret_cast<OvfRec *>(ovf);
         c->fz.ctr = reinterpret_cast<FusedCounters *>(c->fz.zero);
@@ -1401,6 +1401,8 @@ int i2g_movemark(i2g_ctx *c, double timestep, double timesum, uint32_t flags)
         F.ovf = c->fz.ovf;
         F.count = c->fz.count;
         F.ctr = c->fz.ctr;
+        F.zero = c->fz.zero;
+        F.zero_bytes = c->fz.zero_bytes;
         F.treset = c->fz.treset;
         F.defer = c->fz.defer;
         F.spilled = c->fz.spilled_dev;
@@ -1410,7 +1412,6 @@ int i2g_movemark(i2g_ctx *c, double timestep, double timesum, uint32_t flags)
         const AvgArgsK V = avg_args(c, timesum, 0);
         {
             PhaseTimer t(c, 0);
-            CK(cudaMemsetAsync(c->fz.zero, 0, (size_t)c->fz.zero_bytes, c->stream));
             c->launches += launch_move_fused(L, A, V, F);
         }
         CKL();

@@ -92,6 +92,18 @@ __device__ __forceinline__ int floor_fm(float u, float &fl)
     return __float_as_int(s) - 0x4B400000;
 }
 __device__ __forceinline__ float flt_of(int d) { return __int_as_float(0x4B400000 + d) - kF32Magic; }  // |d| < 2^22
+// The two ends of a programmatic launch (launch_next): the kernel before lets the next
+// one's CTAs start, the next one waits until every kernel before it is done and its
+// writes are seen.  What those wrote is read by plain loads, or through a pointer from
+// after_wait, which no load can be moved ahead of.
+__device__ __forceinline__ void allow_next() { cudaTriggerProgrammaticLaunchCompletion(); }
+__device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
+template <typename T>
+__device__ __forceinline__ T *after_wait(T *p)
+{
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
 // max and min that pass a NaN on, as "if (e < lo) e = lo" does, in one instruction
 __device__ __forceinline__ float max_nan(float a, float b)
 {
@@ -515,6 +527,8 @@ __global__ void __launch_bounds__(kMoveTile, VISC ? 4 : 4) k_move_fused(const __
     __shared__ uint8_t order[kMoveTile], types[kMoveTile];
     __shared__ int cnt[kMoveTile / 32][4];
     __shared__ uint8_t type[kMoveTypes];
+    allow_next();
+    wait_previous();
     if (VISC && threadIdx.x < kAvgTypes) VT[threadIdx.x] = visc_type(Ty->t, threadIdx.x);
     if (threadIdx.x < kMoveTypes)
         type[threadIdx.x] = (threadIdx.x < kAvgTypes ? F.type[threadIdx.x] : 0) | (Ty->t.markim[threadIdx.x] ? 1 : 0);
@@ -1137,21 +1151,24 @@ __global__ void __launch_bounds__(kCnThreads, 2) k_cellnodes(const __grid_consta
     using C = CellSums<NT>;
     Shape &M = *reinterpret_cast<Shape *>(smraw);
     constexpr int ROWS = Shape::ROWS, CS = (kCnCols + 1) * ROWS;
+    allow_next();
+    wait_previous();
     slot_heat_init(P);  // block_qconst syncs the block
     const QConst Q = block_qconst(P.ctr, P.viscmod);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % S;
     const int cs = (int)(blockIdx.x % P.ntx) * P.ncol, d0 = (int)(blockIdx.x / P.ntx) * (ROWS - 1);
     const int groups = (P.ncol + 1) / kCnCols;
-    const uint4 *recs = reinterpret_cast<const uint4 *>(P.ra);
+    const uint4 *recs = reinterpret_cast<const uint4 *>(after_wait(P.ra));
     double vmin = 0.0, vmax = 0.0;
     int any = 0;
     unsigned owned = 0;
+    const int32_t *count = after_wait(P.count);
     for (int g = 0; g < groups; g++) {
         const int cc = cs - 1 + kCnCols * g + warp;
         const int row = lane / S, cr = d0 - 1 + row;
         const bool valid = cc >= 0 && cc < P.nc1 && cr >= 0 && cr < P.nc2;
         const int64_t cell = (int64_t)cc * P.nc2 + cr;
-        const int32_t n = valid ? __ldg(P.count + cell) : 0;
+        const int32_t n = valid ? count[cell] : 0;
         if (sub == 0 && row >= 1 && !(g == 0 && warp == 0)) owned += (unsigned)n;  // each cell counted by one CTA
         const int32_t nb = min(n, P.cap);
         // the lane's pairs of records: sub, sub + S, ...; every lane runs the warp's
@@ -1267,6 +1284,8 @@ __global__ void __launch_bounds__(256) k_fused_begin(const __grid_constant__ Gri
                                                      const __grid_constant__ FusedMove F, int32_t first,
                                                      unsigned long long *navg)
 {
+    allow_next();
+    wait_previous();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         F.ctr->any = 0;
         F.ctr->kmin = ~0ull;
@@ -1301,6 +1320,16 @@ __global__ void __launch_bounds__(256) k_fused_begin(const __grid_constant__ Gri
     }
 }
 
+// movemark's counters and bucket counts to zero, as a kernel so that the launches of a
+// run of steps overlap at this boundary too (a memset waits for and holds up both sides)
+static __global__ void __launch_bounds__(256) k_fused_zero(uint4 *p, int64_t n)
+{
+    allow_next();
+    wait_previous();
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = make_uint4(0, 0, 0, 0);
+}
+
 // marktmax (markmart.c:354-360) on a fused averaging call
 static __global__ void k_fused_tmax(const __grid_constant__ GridView G, const __grid_constant__ MarkerView M,
                              const __grid_constant__ AvgArgsK V)
@@ -1318,10 +1347,11 @@ static __global__ void k_fused_tmax(const __grid_constant__ GridView G, const __
 }
 
 // the contrast clamp (markmart.c:995-1009) from the call's viscosity range
-static __global__ void __launch_bounds__(256) k_fused_clamp(int64_t nn, const FusedCounters *__restrict__ ctr, double nucontr,
-                                                     double *__restrict__ nu, double *__restrict__ nd,
-                                                     double *__restrict__ stats)
+static __global__ void __launch_bounds__(256) k_fused_clamp(int64_t nn, const FusedCounters *ctr, double nucontr,
+                                                     double *nu, double *nd, double *stats)
 {
+    allow_next();
+    wait_previous();
     double numin = 0.0, numax = 0.0;
     if (ctr->any) {
         numin = okey_inv(ctr->kmin);
@@ -1335,11 +1365,11 @@ static __global__ void __launch_bounds__(256) k_fused_clamp(int64_t nn, const Fu
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t m3 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m3 < nn; m3 += stride) {
         double v = nu[m3], u = v;
+        const double w = nd[m3];
         if (u < numin) u = numin;
         if (u > numax) u = numax;
         if (u != v) nu[m3] = u;
-        v = nd[m3];
-        u = v;
+        v = u = w;
         if (u < numin) u = numin;
         if (u > numax) u = numax;
         if (u != v) nd[m3] = u;

@@ -186,19 +186,21 @@ static void move_fused(const StepLaunch &L, const MoveArgs &A, const FusedMove &
     if (!resident) resident = resident_ctas((const void *)k_move_fused<VISC, UNI>, kMoveTile);
     const int64_t tiles = (L.M.n + kMoveTile - 1) / kMoveTile;
     const unsigned nb = (unsigned)std::min<int64_t>(tiles, resident);
-    k_move_fused<VISC, UNI><<<nb, kMoveTile, 0, L.stream>>>(L.G, L.M, L.types, A, M);
+    launch_next(k_move_fused<VISC, UNI>, nb, kMoveTile, 0, L.stream, L.G, L.M, L.types, A, M);
 }
 
 int launch_move_fused(const StepLaunch &L, const MoveArgs &A, const AvgArgsK &V, const FusedLaunch &F)
 {
-    if (L.M.n <= 0) return 0;
+    const int64_t n16 = F.zero_bytes / 16;
+    launch_next(k_fused_zero, (unsigned)grid_for(n16, 256, 148 * 8), 256, 0, L.stream, (uint4 *)F.zero, n16);
+    if (L.M.n <= 0) return 1;
     const FusedMove M = fused_move_args(L.G, V, F);
     const bool visc = (A.flags & I2G_MOVE_UPDATE_VISC) != 0, uni = L.G.uni != 0;
     if (visc && uni) move_fused<true, true>(L, A, M);
     else if (visc) move_fused<true, false>(L, A, M);
     else if (uni) move_fused<false, true>(L, A, M);
     else move_fused<false, false>(L, A, M);
-    return 1;
+    return 2;
 }
 
 template <int NT, int S>
@@ -210,7 +212,7 @@ static void cellnodes_shape(const StepLaunch &L, CellNodesArgs P, int groups)
     P.ncol = kCnCols * groups - 1;
     P.ntx = (P.nx + P.ncol - 1) / P.ncol;
     const int nty = (P.ny + Shape::ROWS - 2) / (Shape::ROWS - 1);
-    k_cellnodes<NT, S><<<(unsigned)(P.ntx * nty), kCnThreads, sizeof(Shape), L.stream>>>(P);
+    launch_next(k_cellnodes<NT, S>, (unsigned)(P.ntx * nty), kCnThreads, sizeof(Shape), L.stream, P);
 }
 
 // Two lanes to a cell while that leaves a CTA at most to an SM: there a launch lasts
@@ -251,7 +253,8 @@ int launch_avg_fused(const StepLaunch &L, const AvgArgsK &V, const FusedLaunch &
 {
     int nl = 0;
     const int64_t nn = L.G.nx * L.G.ny;
-    k_fused_begin<true><<<148, 256, 0, L.stream>>>(L.G, L.M, L.types, fused_move_args(L.G, V, F), F.first ? 1 : 0, F.navg);
+    launch_next(k_fused_begin<true>, 148, 256, 0, L.stream, L.G, L.M, L.types, fused_move_args(L.G, V, F), F.first ? 1 : 0,
+                F.navg);
     nl++;
     if (F.track_tmax && L.M.tmax && L.M.n > 0) {
         AvgArgsK V2 = V;
@@ -292,7 +295,8 @@ int launch_avg_fused(const StepLaunch &L, const AvgArgsK &V, const FusedLaunch &
     default: nl += cellnodes<4>(L, P); break;
     }
     // a node per thread: every node's two loads in flight at once
-    k_fused_clamp<<<grid_for(nn, 256, kOneEach), 256, 0, L.stream>>>(nn, F.ctr, F.nucontr, O.nu, O.nd, F.stats);
+    launch_next(k_fused_clamp, (unsigned)grid_for(nn, 256, kOneEach), 256, 0, L.stream, nn, F.ctr, F.nucontr, O.nu, O.nd,
+                F.stats);
     return nl + 1;
 }
 
