@@ -1643,10 +1643,9 @@ int i2g_ronurecalc(i2g_ctx *c, double timesum, uint32_t flags)
     StepLaunch L{c->stream, G, M, c->dtypes};
     {
         PhaseTimer t(c, 2);
-        c->launches += launch_t0(c->stream, G, M, c->sb.slot0, A.tmp_ambient, c->T0);
+        c->launches += launch_t0(c->stream, G, M, c->sb.slot0, A.tmp_ambient, c->T0, c->ndeferred, c->navg);
         if (inplace && const_properties_call(c, timesum)) {
             // sb.perm1 is free once the ranking is done: the deferred-marker list
-            CK(cudaMemsetAsync(c->ndeferred, 0, sizeof(int32_t), c->stream));
             V.tab = c->tconst;
             c->launches += mixed ? launch_contrib_const_mixed(L, A, V, c->sb.rank, c->sb.key, c->sb.perm1, c->ndeferred)
                                  : launch_contrib_const_fp64(L, A, V, c->sb.rank, c->sb.key, c->sb.perm1, c->ndeferred);
@@ -1662,7 +1661,6 @@ int i2g_ronurecalc(i2g_ctx *c, double timesum, uint32_t flags)
     if (mag) c->mag.cur = 1 - c->mag.cur;  // the time the call's last assigning marker left
     {
         PhaseTimer t(c, 3);
-        CK(cudaMemsetAsync(c->navg, 0, sizeof(unsigned long long), c->stream));
         c->launches += mixed ? launch_cellsums_mixed(L, V) : launch_cellsums_fp64(L, V);
     }
     CKL();

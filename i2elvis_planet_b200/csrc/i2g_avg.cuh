@@ -299,8 +299,12 @@ __global__ void __launch_bounds__(256, MIXED ? 5 : 3) k_contrib_inplace(const __
 {
     __shared__ uint8_t order[256];
     __shared__ int cnt[8][4];
+    allow_next();
+    wait_previous();
+    rank = after_wait(rank);
+    key = after_wait(key);
     uint4 *P = reinterpret_cast<uint4 *>(payload);
-    const double T0 = *T0p;
+    const double T0 = *after_wait(T0p);
     int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (args.densimod == 2)
         i = (int64_t)blockIdx.x * 256 + class_order(i < A.n ? table_class(A.type[i]) : 0, order, cnt);
@@ -324,6 +328,10 @@ __global__ void __launch_bounds__(256) k_contrib_const(const __grid_constant__ G
     using W = typename AvgCfg<MIXED>::W;
     using PV = PayVec<MIXED, true>;
     __shared__ TypeConst S;
+    allow_next();
+    wait_previous();
+    rank = after_wait(rank);
+    key = after_wait(key);
     const i2g_types &T = Ty->t;
     for (int t = threadIdx.x; t < kAvgTypes; t += blockDim.x) {
         const double ro = T.markro[t];
@@ -417,9 +425,14 @@ __global__ void __launch_bounds__(256, 3) k_contrib_deferred(const __grid_consta
                                                              const int32_t *__restrict__ deferred,
                                                              const int32_t *__restrict__ ndeferred)
 {
+    allow_next();
+    wait_previous();
+    rank = after_wait(rank);
+    key = after_wait(key);
+    deferred = after_wait(deferred);
     uint4 *P = reinterpret_cast<uint4 *>(payload);
-    const double T0 = *T0p;
-    const int64_t m = *ndeferred;
+    const double T0 = *after_wait(T0p);
+    const int64_t m = *after_wait(ndeferred);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < m; q += stride)
         contrib_inplace<MIXED, true>(G, A, rank, key, Ty->t, args, T0, P, deferred[q]);
@@ -433,8 +446,11 @@ __global__ void __launch_bounds__(256, 4) k_contrib(const __grid_constant__ Grid
                                                     const __grid_constant__ AvgArgsK args,
                                                     const double *__restrict__ T0p, void *payload, int64_t *slot0)
 {
+    allow_next();
+    wait_previous();
+    perm = after_wait(perm);
     uint4 *P = reinterpret_cast<uint4 *>(payload);
-    const double T0 = *T0p;
+    const double T0 = *after_wait(T0p);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < A.n; j += stride)
         contrib_marker<MIXED>(G, A, B, perm, Ty->t, args, T0, P, j, slot0);
@@ -614,8 +630,8 @@ __device__ __forceinline__ unsigned cellsums_tile(AvgSmem<MIXED, CONST> &S, cons
         const int64_t cell = c * nc2 + d0 + lane;
         int32_t cb = 0, cn = 0;
         if (lane < NR) {
-            cb = __ldg(cstart + cell);
-            cn = __ldg(cstart + cell + 1) - cb;
+            cb = cstart[cell];
+            cn = cstart[cell + 1] - cb;
         }
         int maxc = cn;
         for (int o = 16; o > 0; o >>= 1) maxc = max(maxc, __shfl_xor_sync(0xffffffffu, maxc, o));
@@ -677,6 +693,11 @@ __global__ void __launch_bounds__(256, 2) k_cellsums(const void *payload, const 
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     AvgSmem<MIXED, CONST> &S = *reinterpret_cast<AvgSmem<MIXED, CONST> *>(smraw);
+    allow_next();
+    wait_previous();
+    payload = after_wait(payload);
+    cstart = after_wait(cstart);
+    tab = after_wait(tab);
     if constexpr (CONST) {
         using W = typename AvgCfg<MIXED>::W;
         for (int t = threadIdx.x; t < kAvgTypes; t += blockDim.x) {

@@ -167,6 +167,19 @@ struct NodeOut {
     double *w1;  // optional: temperature weight sum per node (for the adjoint)
 };
 
+// The two ends of a programmatic launch (launch_next): the kernel before lets the next
+// one's CTAs start, the next one waits until every kernel before it is done and its
+// writes are seen.  What those wrote is read by plain loads, or through a pointer from
+// after_wait, which no load can be moved ahead of.
+__device__ __forceinline__ void allow_next() { cudaTriggerProgrammaticLaunchCompletion(); }
+__device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
+template <typename T>
+__device__ __forceinline__ T *after_wait(T *p)
+{
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
+
 // ------------------------------------------------------------------ search
 // Largest m in [0, n-2] with g[m] <= x (0 when x < g[0]): exactly the result of
 // the reference's bisection for a strictly increasing g (checked at i2g_set_grid).

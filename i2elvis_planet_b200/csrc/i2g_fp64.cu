@@ -40,8 +40,8 @@ int launch_contrib_fp64(const StepLaunch &L, const AvgArgsK &A, const AvgLaunch 
     if (n <= 0) return 0;
     AvgArgsK A2 = A;
     A2.rad2 = radmax_sq_threshold(L.G.xsize);
-    k_contrib<false><<<grid_for(n, 256, kOneEach), 256, 0, L.stream>>>(L.G, L.M, V.dst, V.perm, L.types, A2, V.T0,
-                                                                 V.payload, V.slot0);
+    launch_next(k_contrib<false>, grid_for(n, 256, kOneEach), 256, 0, L.stream, L.G, L.M, V.dst, V.perm, L.types, A2,
+                V.T0, V.payload, V.slot0);
     return 1;
 }
 
@@ -60,8 +60,8 @@ int launch_contrib_inplace_fp64(const StepLaunch &L, const AvgArgsK &A, const Av
     if (n <= 0) return 0;
     AvgArgsK A2 = A;
     A2.rad2 = radmax_sq_threshold(L.G.xsize);
-    k_contrib_inplace<false><<<grid_for(n, 256, kOneEach), 256, 0, L.stream>>>(L.G, L.M, rank, key, L.types, A2, V.T0,
-                                                                         V.payload);
+    launch_next(k_contrib_inplace<false>, grid_for(n, 256, kOneEach), 256, 0, L.stream, L.G, L.M, rank, key, L.types,
+                A2, V.T0, V.payload);
     return 1;
 }
 
@@ -75,10 +75,10 @@ int launch_contrib_const_fp64(const StepLaunch &L, const AvgArgsK &A, const AvgL
     // a block per 256 markers (one wave of resident blocks, as in the mixed form,
     // measured slower here: 1.07 against 0.96 ms at 36M markers)
     const unsigned nb = grid_for(n, 256, kOneEach);
-    k_contrib_const<false><<<nb, 256, 0, L.stream>>>(L.G, L.M, rank, key, L.types, A2, V.payload, deferred, ndeferred,
-                                                   static_cast<TypeConst *>(V.tab));
-    k_contrib_deferred<false><<<148 * 3, 256, 0, L.stream>>>(L.G, L.M, rank, key, L.types, A2, V.T0, V.payload,
-                                                            deferred, ndeferred);
+    launch_next(k_contrib_const<false>, nb, 256, 0, L.stream, L.G, L.M, rank, key, L.types, A2, V.payload, deferred,
+                ndeferred, static_cast<TypeConst *>(V.tab));
+    launch_next(k_contrib_deferred<false>, 148 * 3, 256, 0, L.stream, L.G, L.M, rank, key, L.types, A2, V.T0,
+                V.payload, deferred, ndeferred);
     return 2;
 }
 
@@ -90,8 +90,8 @@ static void cellsums_fp64(const StepLaunch &L, const AvgLaunch &V)
     allow_dynamic_smem((const void *)k_cellsums<false, CONST>, smem, &attr);
     const int64_t nc1 = L.G.nx - 1, nc2 = L.G.ny - 1;
     const int32_t ntx = (int32_t)((nc1 + V.TX - 1) / V.TX), nty = (int32_t)((nc2 + 31) / 32);
-    k_cellsums<false, CONST><<<ntx * nty, 256, smem, L.stream>>>(V.payload, V.cstart, nc1, nc2, V.part, V.TX, ntx, V.navg,
-                                                            static_cast<const TypeConst *>(V.tab));
+    launch_next(k_cellsums<false, CONST>, (unsigned)(ntx * nty), 256, smem, L.stream, V.payload, V.cstart, nc1, nc2,
+                V.part, V.TX, ntx, V.navg, static_cast<const TypeConst *>(V.tab));
 }
 
 int launch_cellsums_fp64(const StepLaunch &L, const AvgLaunch &V)
@@ -113,8 +113,8 @@ int launch_nodes(cudaStream_t s, const GridView &G, const double *part, const Av
 {
     const int64_t nn = G.nx * G.ny;
     const int32_t nb = nodesum_blocks(nn);
-    k_nodesums<<<nb, 256, 0, s>>>(G, part, A, O, mmpart);
-    k_clamp<<<grid_for(nn, 256, 148 * 4), 256, 0, s>>>(nn, mmpart, nb, nucontr, O.nu, O.nd, stats);
+    launch_next(k_nodesums, nb, 256, 0, s, G, part, A, O, mmpart);
+    launch_next(k_clamp, grid_for(nn, 256, 148 * 4), 256, 0, s, nn, mmpart, nb, nucontr, O.nu, O.nd, stats);
     return 2;
 }
 

@@ -92,18 +92,6 @@ __device__ __forceinline__ int floor_fm(float u, float &fl)
     return __float_as_int(s) - 0x4B400000;
 }
 __device__ __forceinline__ float flt_of(int d) { return __int_as_float(0x4B400000 + d) - kF32Magic; }  // |d| < 2^22
-// The two ends of a programmatic launch (launch_next): the kernel before lets the next
-// one's CTAs start, the next one waits until every kernel before it is done and its
-// writes are seen.  What those wrote is read by plain loads, or through a pointer from
-// after_wait, which no load can be moved ahead of.
-__device__ __forceinline__ void allow_next() { cudaTriggerProgrammaticLaunchCompletion(); }
-__device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
-template <typename T>
-__device__ __forceinline__ T *after_wait(T *p)
-{
-    asm volatile("" : "+l"(p) : : "memory");
-    return p;
-}
 // max and min that pass a NaN on, as "if (e < lo) e = lo" does, in one instruction
 __device__ __forceinline__ float max_nan(float a, float b)
 {

@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(256, MIXED || VISC ? 0 : 4) k_move(const __gri
                                               int32_t *__restrict__ key, int32_t *__restrict__ count,
                                               int32_t *__restrict__ sub)
 {
+    allow_next();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += stride) {
         const int32_t k = move_marker<MIXED, VISC>(G, M, Ty->t, A, key, i);

@@ -40,8 +40,8 @@ int launch_contrib_mixed(const StepLaunch &L, const AvgArgsK &A, const AvgLaunch
     if (n <= 0) return 0;
     AvgArgsK A2 = A;
     A2.rad2 = radmax_sq_threshold(L.G.xsize);
-    k_contrib<true><<<grid_for(n, 256, kOneEach), 256, 0, L.stream>>>(L.G, L.M, V.dst, V.perm, L.types, A2, V.T0,
-                                                                 V.payload, V.slot0);
+    launch_next(k_contrib<true>, grid_for(n, 256, kOneEach), 256, 0, L.stream, L.G, L.M, V.dst, V.perm, L.types, A2,
+                V.T0, V.payload, V.slot0);
     return 1;
 }
 
@@ -60,8 +60,8 @@ int launch_contrib_inplace_mixed(const StepLaunch &L, const AvgArgsK &A, const A
     if (n <= 0) return 0;
     AvgArgsK A2 = A;
     A2.rad2 = radmax_sq_threshold(L.G.xsize);
-    k_contrib_inplace<true><<<grid_for(n, 256, kOneEach), 256, 0, L.stream>>>(L.G, L.M, rank, key, L.types, A2, V.T0,
-                                                                         V.payload);
+    launch_next(k_contrib_inplace<true>, grid_for(n, 256, kOneEach), 256, 0, L.stream, L.G, L.M, rank, key, L.types,
+                A2, V.T0, V.payload);
     return 1;
 }
 
@@ -78,10 +78,10 @@ int launch_contrib_const_mixed(const StepLaunch &L, const AvgArgsK &A, const Avg
     static int64_t wave = 0;
     if (!wave) wave = resident_blocks((const void *)k_contrib_const<true>, 256);
     const unsigned nb = grid_for(n, 256, wave);
-    k_contrib_const<true><<<nb, 256, 0, L.stream>>>(L.G, L.M, rank, key, L.types, A2, V.payload, deferred, ndeferred,
-                                                   static_cast<TypeConst *>(V.tab));
-    k_contrib_deferred<true><<<148 * 3, 256, 0, L.stream>>>(L.G, L.M, rank, key, L.types, A2, V.T0, V.payload,
-                                                            deferred, ndeferred);
+    launch_next(k_contrib_const<true>, nb, 256, 0, L.stream, L.G, L.M, rank, key, L.types, A2, V.payload, deferred,
+                ndeferred, static_cast<TypeConst *>(V.tab));
+    launch_next(k_contrib_deferred<true>, 148 * 3, 256, 0, L.stream, L.G, L.M, rank, key, L.types, A2, V.T0,
+                V.payload, deferred, ndeferred);
     return 2;
 }
 
@@ -93,8 +93,8 @@ static void cellsums_mixed(const StepLaunch &L, const AvgLaunch &V)
     allow_dynamic_smem((const void *)k_cellsums<true, CONST>, smem, &attr);
     const int64_t nc1 = L.G.nx - 1, nc2 = L.G.ny - 1;
     const int32_t ntx = (int32_t)((nc1 + V.TX - 1) / V.TX), nty = (int32_t)((nc2 + 31) / 32);
-    k_cellsums<true, CONST><<<ntx * nty, 256, smem, L.stream>>>(V.payload, V.cstart, nc1, nc2, V.part, V.TX, ntx, V.navg,
-                                                            static_cast<const TypeConst *>(V.tab));
+    launch_next(k_cellsums<true, CONST>, (unsigned)(ntx * nty), 256, smem, L.stream, V.payload, V.cstart, nc1, nc2,
+                V.part, V.TX, ntx, V.navg, static_cast<const TypeConst *>(V.tab));
 }
 
 int launch_cellsums_mixed(const StepLaunch &L, const AvgLaunch &V)
@@ -253,7 +253,8 @@ int launch_avg_fused(const StepLaunch &L, const AvgArgsK &V, const FusedLaunch &
 {
     int nl = 0;
     const int64_t nn = L.G.nx * L.G.ny;
-    launch_next(k_fused_begin<true>, 148, 256, 0, L.stream, L.G, L.M, L.types, fused_move_args(L.G, V, F), F.first ? 1 : 0,
+    launch_next(k_fused_begin<true>, 148, 256, 0, L.stream, L.G, L.M, L.types, fused_move_args(L.G, V, F), F.first ? 1
+                : 0,
                 F.navg);
     nl++;
     if (F.track_tmax && L.M.tmax && L.M.n > 0) {
@@ -295,7 +296,8 @@ int launch_avg_fused(const StepLaunch &L, const AvgArgsK &V, const FusedLaunch &
     default: nl += cellnodes<4>(L, P); break;
     }
     // a node per thread: every node's two loads in flight at once
-    launch_next(k_fused_clamp, (unsigned)grid_for(nn, 256, kOneEach), 256, 0, L.stream, nn, F.ctr, F.nucontr, O.nu, O.nd,
+    launch_next(k_fused_clamp, (unsigned)grid_for(nn, 256, kOneEach), 256, 0, L.stream, nn, F.ctr, F.nucontr, O.nu,
+                O.nd,
                 F.stats);
     return nl + 1;
 }

@@ -115,6 +115,9 @@ static __global__ void __launch_bounds__(256) k_nodesums(const __grid_constant__
                                                          const __grid_constant__ AvgArgsK args, NodeOut O,
                                                          double *__restrict__ mmpart)
 {
+    allow_next();
+    wait_previous();
+    part = after_wait(part);
     double vmin = 0, vmax = 0;
     int any = 0;
     const int64_t m3 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -182,6 +185,11 @@ static __global__ void __launch_bounds__(256) k_clamp(int64_t nn, const double *
                                                double nucontr, double *__restrict__ nu, double *__restrict__ nd,
                                                double *__restrict__ stats)
 {
+    allow_next();
+    wait_previous();
+    mmpart = after_wait(mmpart);
+    nu = after_wait(nu);
+    nd = after_wait(nd);
     clamp_nodes(mmpart, nparts, nucontr, nu, nd, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nn,
                 (int64_t)gridDim.x * blockDim.x, blockIdx.x == 0 ? stats : nullptr);
 }

@@ -63,8 +63,13 @@ __global__ void __launch_bounds__(256) k_scatter_sub(const int32_t *__restrict__
                                                      int64_t n, const int32_t *__restrict__ cstart,
                                                      int32_t *__restrict__ slot_of)
 {
+    allow_next();
+    wait_previous();
+    key = after_wait(key);
+    sub = after_wait(sub);
+    cstart = after_wait(cstart);
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) slot_of[__ldg(cstart + __ldg(key + i)) + __ldg(sub + i)] = (int32_t)i;
+    if (i < n) slot_of[cstart[key[i]] + sub[i]] = (int32_t)i;
 }
 
 // One warp per cell: rank the cell's entries by caller index (ids are unique).
@@ -171,6 +176,11 @@ __global__ void __launch_bounds__(256) k_fixup_pairs(const int32_t *__restrict__
                                                      int32_t *__restrict__ dst, int32_t *__restrict__ rank)
 {
     __shared__ int32_t sid[8][kFixSmem];
+    allow_next();
+    wait_previous();
+    cstart = after_wait(cstart);
+    src = after_wait(src);
+    id = after_wait(id);
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, hl = lane & 15;
     const int64_t c0 = 2 * warp;
@@ -178,8 +188,8 @@ __global__ void __launch_bounds__(256) k_fixup_pairs(const int32_t *__restrict__
     const int64_t cell = c0 + (lane >> 4);
     int32_t s = 0, n = 0;
     if (cell < ncells) {
-        s = __ldg(cstart + cell);
-        n = __ldg(cstart + cell + 1) - s;
+        s = cstart[cell];
+        n = cstart[cell + 1] - s;
     }
     const int nmax = max(n, __shfl_xor_sync(0xffffffffu, n, 16));
     if (nmax > 48) {
@@ -272,6 +282,9 @@ __device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t *tota
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int32_t *__restrict__ in, int64_t n,
                                                              int32_t *__restrict__ out, int32_t *__restrict__ tilesum)
 {
+    allow_next();
+    wait_previous();
+    in = after_wait(in);
     const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
     int32_t v[kScanItems], s = 0;
 #pragma unroll
@@ -292,6 +305,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int32_t *__re
 __global__ void __launch_bounds__(kScanThreads) k_scan_top(int32_t *__restrict__ tilesum, int32_t ntiles,
                                                            int32_t *__restrict__ out_total)
 {
+    allow_next();
+    wait_previous();
+    tilesum = after_wait(tilesum);
     const int64_t base = (int64_t)threadIdx.x * kScanItems;
     int32_t v[kScanItems], s = 0;
 #pragma unroll
@@ -312,6 +328,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_top(int32_t *__restrict__
 __global__ void __launch_bounds__(256) k_scan_add(int32_t *__restrict__ out, int64_t n,
                                                   const int32_t *__restrict__ tilesum)
 {
+    allow_next();
+    wait_previous();
+    out = after_wait(out);
+    tilesum = after_wait(tilesum);
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] += tilesum[i / kScanTile];
 }
@@ -552,10 +572,15 @@ __global__ void k_f32_to_f64(int64_t n, const float *__restrict__ in, double *__
 // T of caller marker 0 as the molten-material conductivity reads it (markmart.c:522):
 // marker 0 is processed first by the reference, so after its own sticky-air reset.
 __global__ void k_t0(GridView G, MarkerView M, const int64_t *__restrict__ slot0, double tmp_ambient,
-                     double *__restrict__ T0)
+                     double *__restrict__ T0, int32_t *ndeferred, unsigned long long *navg)
 {
+    allow_next();
+    wait_previous();
     if (threadIdx.x || blockIdx.x) return;
-    const int64_t j = *slot0;
+    // the counters of the passes that follow
+    if (ndeferred) *ndeferred = 0;
+    if (navg) *navg = 0ull;
+    const int64_t j = *after_wait(slot0);
     if (j < 0 || j >= M.n) { *T0 = 0.0; return; }
     const double x = M.x[j], y = M.y[j], t = M.T[j];
     const int mt = M.type[j];
@@ -612,9 +637,9 @@ static inline unsigned blocks_for(int64_t n, int threads, int64_t cap = 1 << 20)
 int scan_exclusive(cudaStream_t s, const int32_t *in, int64_t n, int32_t *out, int32_t *tilesum)
 {
     const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    k_scan_tiles<<<(unsigned)(ntiles > 0 ? ntiles : 1), kScanThreads, 0, s>>>(in, n, out, tilesum);
-    k_scan_top<<<1, kScanThreads, 0, s>>>(tilesum, (int32_t)ntiles, out + n);
-    k_scan_add<<<blocks_for(n, 256, INT32_MAX), 256, 0, s>>>(out, n, tilesum);
+    launch_next(k_scan_tiles, (unsigned)(ntiles > 0 ? ntiles : 1), kScanThreads, 0, s, in, n, out, tilesum);
+    launch_next(k_scan_top, 1, kScanThreads, 0, s, tilesum, (int32_t)ntiles, out + n);
+    launch_next(k_scan_add, blocks_for(n, 256, INT32_MAX), 256, 0, s, out, n, tilesum);
     return 3;
 }
 
@@ -629,8 +654,8 @@ int sort_markers(cudaStream_t s, const SortBufs &B, int64_t n, int64_t ncells, M
     nl += scan_exclusive(s, B.count, ncells, B.cstart, B.tilesum);
     if (n > 0) {
         k_scatter<<<blocks_for(n, 256, INT32_MAX), 256, 0, s>>>(B.key, n, B.cstart, B.cursor, B.perm1);
-        k_fixup_pairs<<<blocks_for((ncells + 1) / 2 * 32, 256, INT32_MAX), 256, 0, s>>>(B.cstart, ncells, B.perm1,
-                                                                                        src.id, B.perm2, nullptr);
+        launch_next(k_fixup_pairs, blocks_for((ncells + 1) / 2 * 32, 256, INT32_MAX), 256, 0, s, B.cstart, ncells,
+                    B.perm1, src.id, B.perm2, (int32_t *)nullptr);
         k_gather<<<blocks_for(n, 256, 148 * 16), 256, 0, s>>>(n, B.perm2, src, dst, B.slot0);
         nl += 3;
     }
@@ -649,8 +674,8 @@ int rank_markers(cudaStream_t s, const SortBufs &B, int64_t n, int64_t ncells, c
     nl += scan_exclusive(s, B.count, ncells, B.cstart, B.tilesum);
     if (n > 0) {
         k_scatter<<<blocks_for(n, 256, INT32_MAX), 256, 0, s>>>(B.key, n, B.cstart, B.cursor, B.perm1);
-        k_fixup_pairs<<<blocks_for((ncells + 1) / 2 * 32, 256, INT32_MAX), 256, 0, s>>>(B.cstart, ncells, B.perm1, id,
-                                                                                        B.perm2, B.rank);
+        launch_next(k_fixup_pairs, blocks_for((ncells + 1) / 2 * 32, 256, INT32_MAX), 256, 0, s, B.cstart, ncells,
+                    B.perm1, id, B.perm2, B.rank);
         nl += 2;
     }
     return nl;
@@ -661,9 +686,9 @@ int rank_moved(cudaStream_t s, const SortBufs &B, int64_t n, int64_t ncells, con
 {
     int nl = scan_exclusive(s, B.count, ncells, B.cstart, B.tilesum);
     if (n > 0) {
-        k_scatter_sub<<<blocks_for(n, 256, INT32_MAX), 256, 0, s>>>(B.key, sub, n, B.cstart, B.perm1);
-        k_fixup_pairs<<<blocks_for((ncells + 1) / 2 * 32, 256, INT32_MAX), 256, 0, s>>>(B.cstart, ncells, B.perm1, id,
-                                                                                        B.perm2, B.rank);
+        launch_next(k_scatter_sub, blocks_for(n, 256, INT32_MAX), 256, 0, s, B.key, sub, n, B.cstart, B.perm1);
+        launch_next(k_fixup_pairs, blocks_for((ncells + 1) / 2 * 32, 256, INT32_MAX), 256, 0, s, B.cstart, ncells,
+                    B.perm1, id, B.perm2, B.rank);
         nl += 2;
     }
     return nl;
@@ -808,9 +833,9 @@ int launch_f32_to_f64(cudaStream_t s, int64_t n, const float *in, double *out)
 }
 
 int launch_t0(cudaStream_t s, const GridView &G, const MarkerView &M, const int64_t *slot0, double tmp_ambient,
-              double *T0)
+              double *T0, int32_t *ndeferred, unsigned long long *navg)
 {
-    k_t0<<<1, 32, 0, s>>>(G, M, slot0, tmp_ambient, T0);
+    launch_next(k_t0, 1, 32, 0, s, G, M, slot0, tmp_ambient, T0, ndeferred, navg);
     return 1;
 }
 
