@@ -2000,9 +2000,17 @@ static int titerate_impl(i2g_ctx *c, const double *tk_new, const double *tk_old,
         c->nsorts++;
     }
     ThermArgs A{f[0], f[1], f[2], f[3], f[4], c->tnodef, c->idx2, c->idy2, heatdif, timestep};
-    if (c->P.precision == I2G_PREC_MIXED)
-        for (int k = 0; k < (sums ? 5 : 2); k++)
-            c->launches += launch_f64_to_f32(c->stream, c->nn, f[k], c->tnodef + k * c->nn);
+    if (c->P.precision == I2G_PREC_MIXED) {
+        // the FP32 copies of the node fields it reads
+        GridForms F{};
+        F.nx = c->nx;
+        F.ny = c->ny;
+        for (int k = 0; k < (sums ? 5 : 2); k++) {
+            F.in[k] = f[k];
+            F.out[k] = c->tnodef + k * c->nn;
+        }
+        c->launches += launch_grid_forms(c->stream, F);
+    }
     AvgLaunch V{};
     V.cstart = c->sb.cstart;
     V.payload = c->payload;

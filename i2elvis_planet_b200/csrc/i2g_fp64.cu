@@ -145,20 +145,23 @@ int launch_titerate_fp64(const StepLaunch &L, const ThermArgs &A, const int32_t 
     const bool sums = A.heatdif != 0;
     k_tmark<false><<<grid_for(n, 256, kOneEach), 256, 0, L.stream>>>(L.G, L.M, rank, A, sums ? V.payload : nullptr);
     if (!sums) return 1;
-    return 1 + launch_cellsums_fp64(L, V) + launch_tnodes(L, V.part, sol1) + launch_tanti_fp64(L, sol1);
+    const int64_t nc = (L.G.nx - 1) * (L.G.ny - 1);
+    launch_next(k_tsums<false>, grid_for(nc, 256, kOneEach), 256, 0, L.stream, static_cast<const uint4 *>(V.payload),
+                V.cstart, nc, V.part);
+    return 2 + launch_tnodes(L, V.part, sol1) + launch_tanti_fp64(L, sol1);
 }
 
 // the node averages of the diffusion changes (both forms)
 int launch_tnodes(const StepLaunch &L, const double *part, double *sol1)
 {
     const int64_t nn = L.G.nx * L.G.ny;
-    k_tnodes<<<grid_for(nn, 256, kOneEach), 256, 0, L.stream>>>(part, L.G.nx, L.G.ny, sol1);
+    launch_next(k_tnodes, grid_for(nn, 256, kOneEach), 256, 0, L.stream, part, L.G.nx, L.G.ny, sol1);
     return 1;
 }
 
 int launch_tanti_fp64(const StepLaunch &L, const double *sol1)
 {
-    k_tanti<false><<<grid_for(L.M.n, 256, kOneEach), 256, 0, L.stream>>>(L.G, L.M, sol1);
+    launch_next(k_tanti<false>, grid_for(L.M.n, 256, kOneEach), 256, 0, L.stream, L.G, L.M, sol1);
     return 1;
 }
 
@@ -176,6 +179,7 @@ void preload_fp64()
     cudaFuncGetAttributes(&a, k_cellsums<false, false>);
     cudaFuncGetAttributes(&a, k_cellsums<false, true>);
     cudaFuncGetAttributes(&a, k_tmark<false>);
+    cudaFuncGetAttributes(&a, k_tsums<false>);
     cudaFuncGetAttributes(&a, k_tanti<false>);
     cudaFuncGetAttributes(&a, k_tnodes);
     cudaFuncGetAttributes(&a, k_nodesums);

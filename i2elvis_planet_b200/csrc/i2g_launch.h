@@ -109,7 +109,6 @@ int launch_gather_in_xy(cudaStream_t s, int64_t n, const int32_t *perm, const vo
                         const MarkerView &dst, int64_t *slot0);
 int launch_gather_in_rest(cudaStream_t s, int64_t n, const int32_t *perm, const void *T, const void *eta,
                           const int8_t *type, bool f32, const MarkerView &dst);
-int launch_f64_to_f32(cudaStream_t s, int64_t n, const double *in, float *out);
 int launch_f32_to_f64(cudaStream_t s, int64_t n, const float *in, double *out);
 int launch_t0(cudaStream_t s, const GridView &G, const MarkerView &M, const int64_t *slot0, double tmp_ambient,
                double *T0,

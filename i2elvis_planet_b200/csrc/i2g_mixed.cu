@@ -129,12 +129,15 @@ int launch_titerate_mixed(const StepLaunch &L, const ThermArgs &A, const int32_t
     const bool sums = A.heatdif != 0;
     k_tmark<true><<<grid_for(n, 256, kOneEach), 256, 0, L.stream>>>(L.G, L.M, rank, A, sums ? V.payload : nullptr);
     if (!sums) return 1;
-    return 1 + launch_cellsums_mixed(L, V) + launch_tnodes(L, V.part, sol1) + launch_tanti_mixed(L, sol1);
+    const int64_t nc = (L.G.nx - 1) * (L.G.ny - 1);
+    launch_next(k_tsums<true>, grid_for(nc, 256, kOneEach), 256, 0, L.stream, static_cast<const uint4 *>(V.payload),
+                V.cstart, nc, V.part);
+    return 2 + launch_tnodes(L, V.part, sol1) + launch_tanti_mixed(L, sol1);
 }
 
 int launch_tanti_mixed(const StepLaunch &L, const double *sol1)
 {
-    k_tanti<true><<<grid_for(L.M.n, 256, kOneEach), 256, 0, L.stream>>>(L.G, L.M, sol1);
+    launch_next(k_tanti<true>, grid_for(L.M.n, 256, kOneEach), 256, 0, L.stream, L.G, L.M, sol1);
     return 1;
 }
 
@@ -331,6 +334,7 @@ void preload_mixed()
     cudaFuncGetAttributes(&a, k_cellsums<true, false>);
     cudaFuncGetAttributes(&a, k_cellsums<true, true>);
     cudaFuncGetAttributes(&a, k_tmark<true>);
+    cudaFuncGetAttributes(&a, k_tsums<true>);
     cudaFuncGetAttributes(&a, k_tanti<true>);
     cudaFuncGetAttributes(&a, k_move_fused<false, true>);
     cudaFuncGetAttributes(&a, k_move_fused<false, false>);

@@ -557,12 +557,6 @@ __global__ void k_unsort_i8(int64_t n, const int32_t *__restrict__ id, const int
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) out[id[j]] = in[j];
 }
 
-__global__ void k_f64_to_f32(int64_t n, const double *__restrict__ in, float *__restrict__ out)
-{
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = (float)in[i];
-}
-
 __global__ void k_f32_to_f64(int64_t n, const float *__restrict__ in, double *__restrict__ out)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -815,13 +809,6 @@ int launch_unsort_i8(cudaStream_t s, int64_t n, const int32_t *id, const int8_t 
 {
     if (n <= 0) return 0;
     k_unsort_i8<<<blocks_for(n, 256, 148 * 16), 256, 0, s>>>(n, id, in, out);
-    return 1;
-}
-
-int launch_f64_to_f32(cudaStream_t s, int64_t n, const double *in, float *out)
-{
-    if (n <= 0) return 0;
-    k_f64_to_f32<<<blocks_for(n, 256, 148 * 16), 256, 0, s>>>(n, in, out);
     return 1;
 }
 

@@ -6,10 +6,9 @@
 //   rock marker (< 50) is reset to the old node temperature if it has none, gets
 //   the subgrid diffusion step toward it when heatdif != 0, then follows the node
 //   change (heatmart.c:538-628).  Its diffusion change and weights go to its slot
-//   of the cell-sorted order as one averaging payload record.
-// k_cellsums (i2g_avg.cuh) sums those records per cell in slot order (weights in
-//   the F_W0 sums, change x weight in F_RO), the same fixed-order segmented
-//   reduction as the averaging.
+//   of the cell-sorted order as one record (TherRec).
+// k_tsums sums those records per cell in slot order: per corner the weights and the
+//   change times the weight, with add_values' products.
 // k_tnodes: per node, the four cells' corner sums in the averaging's fixed order,
 //   then the averaged change sol1 / sol0 (heatmart.c:638-652).
 // k_tanti: per rock marker, the antidiffusion: minus the averaged change of each
@@ -54,22 +53,45 @@ __device__ __forceinline__ void tweights32(const GridView &G, double x, double y
     fdw32(__ldg(G.gy + m20), __ldg(G.iyb + m20), y, wy0, wy1);
 }
 
-// payload: NULL when heatdif == 0 (no sums); rank: NULL when the storage order is
+// What a marker adds to the sums of its cell: its weights (the mixed form's w0 is
+// 1.0f - w1 exactly) and its diffusion change; flag 0: nothing.  With averaging records
+// of 48 and 96 B instead k_tmark took 141 us at 601^2 nodes, mixed; with these 117.
+template <bool MIXED>
+struct TherRec;
+template <>
+struct __align__(16) TherRec<true> {
+    float wx1, wy1, d;
+    uint32_t flag;
+};
+template <>
+struct __align__(16) TherRec<false> {
+    double wx0, wx1, wy0, wy1, d;
+    uint32_t flag, pad;
+};
+template <bool MIXED>
+union TherVec {
+    static constexpr int R4 = sizeof(TherRec<MIXED>) / 16;
+    TherRec<MIXED> r;
+    uint4 v[R4];
+};
+
+// records: NULL when heatdif == 0 (no sums); rank: NULL when the storage order is
 // the sorted order (slot = index).  The FP64 form follows the reference's
 // operations; the mixed form gathers FP32 node copies with FP32 weights and
 // keeps the marker temperature itself in FP64.
 template <bool MIXED>
 __global__ void __launch_bounds__(256) k_tmark(const __grid_constant__ GridView G, const __grid_constant__ MarkerView M,
                                                const int32_t *__restrict__ rank, const __grid_constant__ ThermArgs A,
-                                               void *payload)
+                                               void *records)
 {
+    allow_next();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M.n) return;
     const double x = M.x[i], y = M.y[i];
     const int t = M.type[i];
-    PayVec<MIXED> u;
+    TherVec<MIXED> u;
 #pragma unroll
-    for (int q = 0; q < PayVec<MIXED>::R4; q++) u.v[q] = make_uint4(0u, 0u, 0u, 0u);
+    for (int q = 0; q < TherVec<MIXED>::R4; q++) u.v[q] = make_uint4(0u, 0u, 0u, 0u);
     if (inside_box(G, x, y) && t < 100) {
         const int64_t ny = G.ny;
         int64_t m10, m20;
@@ -97,8 +119,8 @@ __global__ void __launch_bounds__(256) k_tmark(const __grid_constant__ GridView 
                     u.r.wx1 = wx1;
                     u.r.wy0 = wy0;
                     u.r.wy1 = wy1;
-                    u.r.pv[0] = dtk1;
-                    u.r.flag = 3u;  // summed; "immobile": no temperature-weight sums
+                    u.r.d = dtk1;
+                    u.r.flag = 1u;
                 }
                 T += tn - to;
                 M.T[i] = T;
@@ -127,19 +149,72 @@ __global__ void __launch_bounds__(256) k_tmark(const __grid_constant__ GridView 
                     T += (double)d1;
                     u.r.wx1 = wx1;
                     u.r.wy1 = wy1;
-                    u.r.pv[0] = d1;
-                    u.r.flag = 3u;
+                    u.r.d = d1;
+                    u.r.flag = 1u;
                 }
                 T += (double)tn - (double)to;
                 M.T[i] = T;
             }
         }
     }
-    if (payload) {
+    if (records) {
         const int64_t slot = rank ? (int64_t)__ldg(rank + i) : i;
-        uint4 *d = reinterpret_cast<uint4 *>(payload) + slot * PayVec<MIXED>::R4;
+        uint4 *d = reinterpret_cast<uint4 *>(records) + slot * TherVec<MIXED>::R4;
 #pragma unroll
-        for (int q = 0; q < PayVec<MIXED>::R4; q++) d[q] = u.v[q];
+        for (int q = 0; q < TherVec<MIXED>::R4; q++) d[q] = u.v[q];
+    }
+}
+
+// part[2 q + {0, 1}][cell]: the sums of weight and of change times weight at corner q.
+// A thread per cell, its records in slot order, four in flight; neighbouring lanes read
+// neighbouring stretches of the slots, so every line comes once and serves from L1.
+// Bound by the records' read: 601^2 nodes, mixed, 35 us; k_cellsums with its 42 sums, of
+// which 8 were used, 81.
+constexpr int kTherSums = 8;
+template <bool MIXED>
+__global__ void __launch_bounds__(256) k_tsums(const uint4 *__restrict__ records, const int32_t *__restrict__ cstart,
+                                               int64_t ncells, double *__restrict__ part)
+{
+    using TV = TherVec<MIXED>;
+    allow_next();
+    wait_previous();
+    records = after_wait(records);
+    const int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (cell >= ncells) return;
+    const int32_t s = cstart[cell], n = cstart[cell + 1] - s;
+    const uint4 *p = records + (int64_t)s * TV::R4;
+    double s0[4] = {0.0, 0.0, 0.0, 0.0}, s1[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int t = 0; t < n; t += 4) {
+        TV u[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int q = 0; q < TV::R4; q++)
+                u[k].v[q] = t + k < n ? p[(t + k) * TV::R4 + q] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (!(u[k].r.flag & 1u)) continue;
+            double wx0, wy0;
+            if constexpr (MIXED) {
+                wx0 = (double)(1.0f - u[k].r.wx1);
+                wy0 = (double)(1.0f - u[k].r.wy1);
+            } else {
+                wx0 = u[k].r.wx0;
+                wy0 = u[k].r.wy0;
+            }
+            const double wx1 = u[k].r.wx1, wy1 = u[k].r.wy1, d = u[k].r.d;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const double sw = ((q >> 1) ? wx1 : wx0) * ((q & 1) ? wy1 : wy0);
+                s1[q] += d * sw;
+                s0[q] += sw;
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        part[(int64_t)(2 * q) * ncells + cell] = s0[q];
+        part[(int64_t)(2 * q + 1) * ncells + cell] = s1[q];
     }
 }
 
@@ -172,6 +247,9 @@ static __global__ void __launch_bounds__(256) k_interp_tnode(const __grid_consta
 static __global__ void __launch_bounds__(256) k_tnodes(const double *__restrict__ part, int64_t nx, int64_t ny,
                                                        double *__restrict__ sol1)
 {
+    allow_next();
+    wait_previous();
+    part = after_wait(part);
     const int64_t m3 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (m3 >= nx * ny) return;
     const int64_t m1 = m3 / ny, m2 = m3 - m1 * ny, nc = (nx - 1) * (ny - 1);
@@ -182,8 +260,8 @@ static __global__ void __launch_bounds__(256) k_tnodes(const double *__restrict_
         if (c1 < 0 || c2 < 0 || c1 > nx - 2 || c2 > ny - 2) continue;
         const int64_t cell = c1 * (ny - 1) + c2;
         const int q = 3 - qd;
-        s0 += __ldg(part + (int64_t)(q * 10 + F_W0) * nc + cell);
-        s1 += __ldg(part + (int64_t)(q * 10 + F_RO) * nc + cell);
+        s0 += part[(int64_t)(2 * q) * nc + cell];
+        s1 += part[(int64_t)(2 * q + 1) * nc + cell];
     }
     sol1[m3] = s0 != 0.0 ? s1 / s0 : s1;
 }
@@ -194,6 +272,9 @@ template <bool MIXED>
 __global__ void __launch_bounds__(256) k_tanti(const __grid_constant__ GridView G, const __grid_constant__ MarkerView M,
                                                const double *__restrict__ sol1)
 {
+    allow_next();
+    wait_previous();
+    sol1 = after_wait(sol1);
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M.n) return;
     const double x = M.x[i], y = M.y[i];
@@ -208,7 +289,7 @@ __global__ void __launch_bounds__(256) k_tanti(const __grid_constant__ GridView 
     for (int a = 0; a < 2; a++)
 #pragma unroll
         for (int b = 0; b < 2; b++) {
-            const double s = __ldg(sol1 + (m10 + a) * G.ny + m20 + b);
+            const double s = sol1[(m10 + a) * G.ny + m20 + b];
             if (s != 0.0) T -= s * (double)((a ? wx1 : wx0) * (b ? wy1 : wy0));
         }
     M.T[i] = T;
