@@ -529,6 +529,7 @@ int resort(i2g_ctx *c)
     c->cur = 1 - c->cur;
     c->nsorts++;
     c->keys_dirty = false;
+    c->keys_stale = true;  // sb.key is in the order the records had
     c->order_sorted = true;
     c->ranks_valid = false;
     c->since_reorder = 0;
@@ -1570,7 +1571,9 @@ int i2g_ronurecalc(i2g_ctx *c, double timesum, uint32_t flags)
     if (c->P.densimod == 2 && !c->td.set) return fail(c, I2G_ESTATE, "densimod 2 needs the table (i2g_set_td_table)");
     if (c->fz.ready && timesum == c->fz.timesum && fused_call(c, timesum)) return fused_ronurecalc(c, timesum, flags);
     c->fz.ready = false;
-    TRY(refresh_keys(c));
+    // the cells are read by the ranking, the contributions in place and the table
+    // path's melt pass: sorted markers without a table need none
+    if (!c->order_sorted || c->P.densimod == 2) TRY(refresh_keys(c));
     // Markers sorted already: the contributions pass copies them through.  Else,
     // after ranking them by (cell, caller index), every reorder_every-th call moves
     // the records into that order; the calls between leave them in place and only
@@ -1688,6 +1691,7 @@ int i2g_ronurecalc(i2g_ctx *c, double timesum, uint32_t flags)
         c->since_reorder++;
     } else {
         c->cur = 1 - c->cur;
+        c->keys_stale = true;  // sb.key is in the order the records had
         c->order_sorted = true;
         c->ranks_valid = false;
         c->since_reorder = 0;
