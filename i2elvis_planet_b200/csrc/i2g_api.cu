@@ -88,6 +88,7 @@ struct i2g_ctx {
     int64_t stage_bytes = 0;
     int *typecheck_host = nullptr;
     bool gzero[G_N] = {};  // the field is zero on the device
+    std::vector<double> hgx, hgy;  // the lines of the last i2g_set_grid
     int32_t TX = 16;  // averaging tile: cell columns (x 32 cell rows), cellsum_cols()
     unsigned long long *navg = nullptr;
     DevTypes *dtypes = nullptr;
@@ -854,6 +855,15 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
         if (!(gx[i] > gx[i - 1])) return fail(c, I2G_EINVAL, "gx must be strictly increasing");
     for (int64_t i = 1; i < ny; i++)
         if (!(gy[i] > gy[i - 1])) return fail(c, I2G_EINVAL, "gy must be strictly increasing");
+    // other lines: the markers' cells, and so their order by cell, are no longer known
+    if (c->hgx.size() != (size_t)nx || c->hgy.size() != (size_t)ny || memcmp(c->hgx.data(), gx, sizeof(double) * nx) ||
+        memcmp(c->hgy.data(), gy, sizeof(double) * ny)) {
+        c->hgx.clear();  // set again once they are on the device
+        c->keys_stale = true;
+        c->keys_dirty = false;
+        c->order_sorted = false;
+        c->ranks_valid = false;
+    }
     // the tables on the host: in the pinned room of a small grid (free between calls,
     // which end synchronised), else in memory of their own
     const size_t lbytes = (size_t)(line_bytes(nx) + line_bytes(ny));
@@ -916,6 +926,8 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
         CKL();
     }
     CK(cudaStreamSynchronize(c->stream));
+    c->hgx.assign(gx, gx + nx);
+    c->hgy.assign(gy, gy + ny);
     c->grid_set = true;
     return I2G_OK;
 }
