@@ -2491,6 +2491,12 @@ int batch_run_streams_graph(i2g_batch *b, const double *timestep, double *timesu
                             float *ms)
 {
     const int n = (int)b->ctx.size();
+    // the replays run on the batch stream: after what the contexts' streams still hold
+    // (the record moves of the call before, a caller's own steps)
+    for (auto *c : b->ctx) {
+        BCK(cudaEventRecord(b->ev, c->stream));
+        BCK(cudaStreamWaitEvent(b->stream, b->ev, 0));
+    }
     for (auto *c : b->ctx) {
         if (fused_check_overflow(c, b->sexec ? kReplaySpill : 0) != I2G_OK) return bfail(b, I2G_ENOMEM, c->err);
     }
