@@ -89,6 +89,9 @@ struct i2g_ctx {
     int *typecheck_host = nullptr;
     bool gzero[G_N] = {};  // the field is zero on the device
     std::vector<double> hgx, hgy;  // the lines of the last i2g_set_grid
+    // counts the changes of what a captured step holds by value: the lines and what is
+    // derived from them, which fields are present, the rock types
+    uint64_t generation = 0;
     int32_t TX = 16;  // averaging tile: cell columns (x 32 cell rows), cellsum_cols()
     unsigned long long *navg = nullptr;
     DevTypes *dtypes = nullptr;
@@ -791,6 +794,7 @@ int i2g_set_types(i2g_ctx *c, const i2g_types *T)
 {
     if (!c || !T) return I2G_EINVAL;
     CK(cudaSetDevice(c->dev));
+    if (memcmp(&c->Th, T, sizeof *T) != 0) c->generation++;
     c->Th = *T;
     CK(cudaMemcpyAsync(&c->dtypes->t, &c->Th, sizeof(i2g_types), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -859,6 +863,7 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
     if (c->hgx.size() != (size_t)nx || c->hgy.size() != (size_t)ny || memcmp(c->hgx.data(), gx, sizeof(double) * nx) ||
         memcmp(c->hgy.data(), gy, sizeof(double) * ny)) {
         c->hgx.clear();  // set again once they are on the device
+        c->generation++;
         c->keys_stale = true;
         c->keys_dirty = false;
         c->order_sorted = false;
@@ -915,6 +920,7 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
         }
     }
     for (int k = 0; k < G_N; k++) {
+        if (c->gpresent[k] != (src[k] != nullptr)) c->generation++;
         c->gpresent[k] = src[k] != nullptr;
         c->gzero[k] = src[k] == nullptr;
     }
@@ -2227,6 +2233,7 @@ int i2g_adjoint_forward(i2g_ctx *c, const double *amps, int32_t nsteps, double t
                                         c->g[G_VY]);
     if (c->vxf) c->launches += launch_grid_forms(c->stream, grid_forms(c));
     c->gzero[G_VX] = c->gzero[G_VY] = false;
+    if (!c->gpresent[G_VX] || !c->gpresent[G_VY]) c->generation++;
     c->gpresent[G_VX] = c->gpresent[G_VY] = true;
     if (!c->order_sorted) TRY(resort(c));
     const MarkerBuf &b = c->mb[c->cur];
@@ -2319,6 +2326,7 @@ struct i2g_batch {
     cudaGraphExec_t sexec = nullptr;
     cudaGraph_t sgraph = nullptr;
     std::vector<double> skey;
+    std::vector<double> lkey;  // the instances' captured_state at batch_layout
     bool graphs = true;  // i2g_batch_set_graphs
     BatchRun R{};
     std::string err;
@@ -2339,10 +2347,22 @@ int bfail(i2g_batch *b, int code, const std::string &m)
         if (e_ != cudaSuccess) return bfail(b, I2G_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// What captured launches and the descriptor table hold of an instance by value, or
+// choose by, besides its timestep and buffers: a change of any makes them stale.
+void captured_state(const i2g_ctx *c, std::vector<double> &key)
+{
+    const int has = (c->has_tmax ? 1 : 0) | (c->has_hi ? 2 : 0) | (c->has_por ? 4 : 0) | (c->has_mag ? 8 : 0) |
+                    (c->f32_storage ? 16 : 0);
+    key.insert(key.end(), {(double)c->generation, (double)c->n, (double)has, (double)c->fz.nt});
+    for (int k = 0; k < c->fz.nt; k++) key.push_back((double)c->fz.slot_type[k]);
+}
+
 // (re)build the descriptor table and work offsets for the current tile width
 int batch_layout(i2g_batch *b)
 {
     const int n = (int)b->ctx.size();
+    b->lkey.clear();
+    for (auto *c : b->ctx) captured_state(c, b->lkey);
     b->hD.assign(n, InstDesc{});
     b->hoff.assign(4 * (n + 1), 0);
     int64_t *om = b->hoff.data(), *oc = om + (n + 1), *ot = oc + (n + 1), *ob = ot + (n + 1);
@@ -2485,8 +2505,8 @@ constexpr int32_t kReplaySpill = 256;
 // with the per-step constants read from the batch's device table, then
 // replayed once per step.  The host work the replays cannot repeat happens
 // between calls: the bucket-overflow check before, the record moves (every
-// reorder_every steps) after; a change of buffers, bucket sizes, timesteps or
-// flags captures the step again.
+// reorder_every steps) after; a change of buffers, bucket sizes, timesteps, flags or
+// an instance's captured_state captures the step again.
 int batch_run_streams_graph(i2g_batch *b, const double *timestep, double *timesum, int32_t nsteps, uint32_t flags,
                             float *ms)
 {
@@ -2504,8 +2524,8 @@ int batch_run_streams_graph(i2g_batch *b, const double *timestep, double *timesu
     for (int k = 0; k < n; k++) {
         i2g_ctx *c = b->ctx[k];
         const uint32_t fk = ((flags & I2G_AVG_TRACK_TMAX) && c->has_tmax) ? I2G_AVG_TRACK_TMAX : 0u;
-        key.insert(key.end(), {(double)c->cur, (double)(uintptr_t)c->fz.ra, (double)c->fz.cap, timestep[k],
-                               (double)fk, (double)c->fz.nt, (double)c->n});
+        key.insert(key.end(), {(double)c->cur, (double)(uintptr_t)c->fz.ra, (double)c->fz.cap, timestep[k], (double)fk});
+        captured_state(c, key);
     }
     if (!b->sexec || key != b->skey) {
         streams_graph_drop(b);
@@ -2650,6 +2670,24 @@ int batch_run(i2g_batch *b, const double *timestep, double *timesum, int32_t nst
         return batch_run_streams(b, timestep, timesum, nsteps, flags, ms);
     }
     const int n = (int)b->ctx.size();
+    // porosity or magnetisation set since the batch was made: its kernels have neither;
+    // the contexts' own general steps give what they would
+    if (std::any_of(b->ctx.begin(), b->ctx.end(), [](const i2g_ctx *c) { return c->has_por || c->has_mag; })) {
+        std::vector<bool> fused;
+        for (auto *c : b->ctx) {
+            fused.push_back(c->fz.enabled);
+            c->fz.enabled = false;
+        }
+        const int r = batch_run_streams(b, timestep, timesum, nsteps, flags, ms);
+        for (int k = 0; k < n; k++) b->ctx[k]->fz.enabled = fused[k];
+        return r;
+    }
+    std::vector<double> key;
+    for (auto *c : b->ctx) captured_state(c, key);
+    if (key != b->lkey) {
+        TRY(batch_layout(b));
+        if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
+    }
     bool changed = false;
     for (int k = 0; k < n; k++) {
         i2g_ctx *c = b->ctx[k];
