@@ -1474,13 +1474,18 @@ static bool const_properties_call(const i2g_ctx *c, double timesum)
     return true;
 }
 
+// The sticky-air reset temperature, mtk = markk[] = (float)(tmp_ambient)
+// (markmart.c:301): in single-precision storage the FP32 value
+static double ambient(const i2g_ctx *c)
+{
+    return c->f32_storage ? (double)(float)c->P.tmp_ambient : c->P.tmp_ambient;
+}
+
 static AvgArgsK avg_args(const i2g_ctx *c, double timesum, uint32_t flags)
 {
     AvgArgsK A{};
     A.timesum = timesum;
-    // mtk = markk[] = (float)(tmp_ambient) (markmart.c:301): in single-precision
-    // storage the reset temperature is the FP32 value
-    A.tmp_ambient = c->f32_storage ? (double)(float)c->P.tmp_ambient : c->P.tmp_ambient;
+    A.tmp_ambient = ambient(c);
     A.core_form_time = c->P.core_form_time;
     A.k_cutoff = c->P.k_cutoff;
     A.relax_time = c->P.relax_time;
@@ -2384,9 +2389,10 @@ int batch_layout(i2g_batch *b)
         d.O = NodeOut{c->node[N_RO], c->node[N_NU], c->node[N_ND], c->node[N_ET], c->node[N_CP],
                       c->node[N_KT], c->node[N_HT], c->node[N_TK], c->node[N_PO]};
         d.payload = c->payload;
-        d.move = MoveArgs{0.0, 0.0, c->P.relax_time, c->P.nubeg, c->P.nuend, c->P.markmod, c->P.outgrid, 0u};
+        d.move = MoveArgs{0.0, 0.0, c->P.relax_time, c->P.nubeg, c->P.nuend, c->P.markmod, c->P.outgrid, 0u,
+                          c->f32_storage ? 1 : 0};
         AvgArgsK A{};
-        A.tmp_ambient = c->P.tmp_ambient;
+        A.tmp_ambient = ambient(c);
         A.core_form_time = c->P.core_form_time;
         A.k_cutoff = c->P.k_cutoff;
         A.relax_time = c->P.relax_time;

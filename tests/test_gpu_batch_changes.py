@@ -85,3 +85,37 @@ def test_member_changes_between_steps(kind, strategy, precision):
         for f in want:
             np.testing.assert_array_equal(got[f], want[f], err_msg=f)
     b.close()
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED], ids=["fp64", "mixed"])
+def test_single_precision_markers(precision):
+    """The fused strategy keeps the positions of markers set in the reference's
+    single-precision storage in that storage, as a context stepped alone does."""
+    insts = members()
+    fp = C.POINTER(C.c_float)
+
+    def make(inst):
+        ms = lib.MarkerStep.from_instance(inst, precision=precision, upload=False)
+        ms.set_fused(False)
+        ms.set_grid(inst.gx, inst.gy, **inst.grid)
+        ms.set_nodes(**inst.nodes)
+        f = [np.ascontiguousarray(a, dtype=np.float32) for a in (inst.x, inst.y, inst.T, inst.eta)]
+        t = np.ascontiguousarray(inst.mtype, dtype=np.int8)
+        assert ms.lib.i2g_set_markers_f32(ms.h, inst.marknum, *[a.ctypes.data_as(fp) for a in f],
+                                          t.ctypes.data_as(C.c_char_p)) == 0
+        ms.n = inst.marknum
+        return ms
+    for i in insts:
+        i.scal["tmp_ambient"] = 150.1  # no single-precision number
+    batched, alone = [make(i) for i in insts], [make(i) for i in insts]
+    b = lib.Batch(batched)
+    dt = np.array([i.timestep for i in insts])
+    ts = np.array([i.timesum for i in insts])
+    b.step(dt, ts, 3)
+    b.sync()
+    for ms, i in zip(alone, insts):
+        ms.step(i.timestep, i.timesum, 3)
+    for got, want in zip(outputs(batched), outputs(alone)):
+        for f in want:
+            np.testing.assert_array_equal(got[f], want[f], err_msg=f)
+    b.close()
