@@ -350,7 +350,7 @@ bool fill_axis(const AxisTables &t, const double *g, int64_t n)
     bool ok = true;
     auto pair = [&](double x0, double x1) {
         const double h = x1 - x0;
-        ok = ok && h > 0x1p-400 && h < 0x1p400;
+        ok = ok && h > 0x1p-100 && h < 0x1p100;
         return LinePair{x0, x1, h, 1.0 / h};
     };
     for (int64_t i = 0; i < n; i++) t.g[i] = g[i];

@@ -265,8 +265,9 @@ __device__ __forceinline__ void fdw64(double x0, double x1, double xi, double &w
 // (P. Markstein, Computation of elementary functions on the IBM RISC System/6000,
 // 1990: with r correctly rounded and q within one unit of a / h, the remainder
 // a - q h is exact and q + remainder x r rounds to the quotient; a first correction
-// of a r makes q that close).  For h and r in the normal range and a not below
-// 2^-900 in magnitude, where no product underflows.
+// of a r makes q that close).  For h and r within 2^-100 .. 2^100 and a not below
+// 2^-900 in magnitude, where neither the quotient (at least 2^-1000) nor a product
+// or remainder is subnormal.
 __device__ __forceinline__ double div_by(double a, double h, double r)
 {
     double q = a * r;

@@ -8,6 +8,8 @@ correctly rounded, so for a small fraction of doubles the two differ by one unit
 in the last place; never by more, and never in the special values."""
 import ctypes as C
 import ctypes.util
+import os
+import re
 
 import numpy as np
 
@@ -64,6 +66,33 @@ def test_div_by_is_the_division():
     a = a * np.where(rng.random(h.size) < 0.5, 1.0, -1.0)
     a = a[np.abs(a) >= 2.0 ** -900][: h.size]
     h = h[: a.size]
+    bad = 0
+    for x, w in zip(a.tolist(), h.tolist()):
+        r = 1.0 / w
+        v = x * r
+        v = libm.fma(libm.fma(-v, w, x), r, v)
+        v = libm.fma(libm.fma(-v, w, x), r, v)
+        bad += v != x / w
+    assert bad == 0
+
+
+def test_div_by_at_the_ends_of_its_range():
+    """div_by where the device code still uses it: numerators down to kDivTiny
+    (i2g_dev.cuh) against the narrowest and widest cells that fill_axis (i2g_api.cu)
+    takes into its tables; no product underflows there."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "i2elvis_planet_b200", "csrc")
+    tiny = int(re.search(r"kDivTiny = \(1023u - (\d+)u\)", open(os.path.join(csrc, "i2g_dev.cuh")).read()).group(1))
+    low, high = map(int, re.search(r"h > 0x1p-(\d+) && h < 0x1p(\d+)", open(os.path.join(csrc, "i2g_api.cu")).read()).groups())
+    libm.fma.restype = C.c_double
+    libm.fma.argtypes = [C.c_double] * 3
+    rng = np.random.default_rng(8)
+    n = 20000
+    h = np.ldexp(1 + rng.random(n), rng.integers(-low, high, n))
+    a = np.ldexp(1 + rng.random(n), rng.integers(-tiny, 60 - tiny, n)) * np.where(rng.random(n) < 0.5, 1.0, -1.0)
+    # and, where widths reach that far, quotients halfway between two subnormals
+    h[::2] = np.ldexp(1 + rng.integers(0, 2 ** 20, h[::2].size) / 2.0 ** 20, rng.integers(-low, high, h[::2].size))
+    half = np.ldexp(h * (2 * rng.integers(1, 2 ** 30, n) + 1), -1075)
+    a[::2] = np.where((half >= 2.0 ** -tiny)[::2], half[::2], a[::2])
     bad = 0
     for x, w in zip(a.tolist(), h.tolist()):
         r = 1.0 / w
