@@ -567,11 +567,14 @@ __global__ void __launch_bounds__(kMoveTile, VISC ? 4 : 4) k_move_fused(const __
 //           magnitude any node's sum can reach (4 x the largest cell count x the
 //           largest |term|): every partial sum is an integer multiple of q below
 //           2^52 q, an exact FP64 number.  Opposite terms stay opposite.
-//   floors  the sum starts at c / 2 and takes each term as fma(a, b, sum) rounded
-//           down: it stays in its binade (a cell's sum is at most a quarter of a
-//           node's), so every term adds its floor to a multiple of q / 2, whatever
-//           came before it (to the nearest, ties would depend on that).  One FP64
-//           operation per term.
+//   binade  the sum starts at c / 2 and takes each term as fma(a, b, sum): it stays in
+//           its binade (a cell's sum is at most a quarter of a node's), where doubles
+//           are q / 2 apart, so every term adds its nearest multiple of q / 2, whatever
+//           came before it.  Only a tie would depend on that, and there is none: the
+//           last fraction bit of one factor is set (odd), so a term is an odd multiple
+//           of 2^-52 of that factor's leading bit times the other's last bit; were that
+//           2^(e - 54), half the spacing, the term would be 2^(e - 2) or more, where it
+//           is below 2^(e - 4).  One FP64 operation per term, half of quant's error.
 struct QConst {
     double cw, ctk, cnu;  // weights, temperature x weight, log-viscosity x weight
     // a node goes to node_guard where a weight sum is below thr_w (thr_nuw for
@@ -592,7 +595,7 @@ __device__ __forceinline__ QConst qconst_of(uint32_t cmax, uint32_t tkb, uint32_
     Q.cw = ldexp(1.5, ew);
     Q.ctk = ldexp(1.5, etk);
     Q.cnu = ldexp(1.5, enu);
-    // A node sum of up to Nn terms moves by at most Nn q / 2.  A weighted mean
+    // A node sum of up to Nn terms moves by at most Nn q / 2 (in its binade half of that).  A weighted mean
     // S / W then moves by at most (Nn q_S / 2) / |S| + (Nn q_w / 2) / W of
     // itself; keep each part below 1e-9.  For log-viscosity (viscmod 1) the mean
     // is an exponent: its absolute error, (Nn q_S / 2 + |mean| Nn q_w / 2) / W,
@@ -658,7 +661,7 @@ struct CellAcc {
     double x[B + 1], y[B + 1], p[B + 1];   // x, y, x y (quantized): plain, s1, s2, s1 s2
     double w, wx, wy;                      // |x y| plain, sx, sy (sx sy: p[0])
     double n[4];                           // log-viscosity x |x y| (quantized): plain, sx, sy, sx sy
-    double t0, tx, ty, txy, nd, wnd;       // sums of floors
+    double t0, tx, ty, txy, nd, wnd;       // sums in their binade
 };
 
 template <int NT>
@@ -683,7 +686,15 @@ __device__ __forceinline__ double unit_of(uint32_t b)
     return __hiloint2double((int)((b & 0x80000000u) | 0x3FF00000u), 0);
 }
 
-// One record into its cell's sums (markmart.c:859-913): 33 FP64 operations with three
+// v with its last fraction bit set, one unit more for the terms below (their last bits
+// are zero: 24-bit numbers and products of two); 0 becomes the smallest subnormal, which
+// adds nothing to a sum
+__device__ __forceinline__ double odd(double v)
+{
+    return __hiloint2double(__double2hiint(v), __double2loint(v) | 1);
+}
+
+// One record into its cell's sums (markmart.c:859-913): 32 FP64 operations with three
 // slots.
 template <int NT>
 __device__ __forceinline__ void acc_rec(CellAcc<NT> &a, uint4 u, const QConst &Q)
@@ -707,11 +718,11 @@ __device__ __forceinline__ void acc_rec(CellAcc<NT> &a, uint4 u, const QConst &Q
         a.p[k] = fma(s, p, a.p[k]);
     }
     // the temperature of mobile types
-    const double tk = (double)__uint_as_float(u.y & kRecImmobile ? 0u : u.z), tkx = tk * x;  // 24 x 24 bits: exact
-    a.t0 = __dadd_rd(a.t0, tk);
-    a.tx = __dadd_rd(a.tx, tkx);
-    a.ty = __fma_rd(tk, y, a.ty);
-    a.txy = __fma_rd(tkx, y, a.txy);
+    const double tk = odd((double)__uint_as_float(u.y & kRecImmobile ? 0u : u.z));
+    a.t0 += tk;
+    a.tx = fma(tk, x, a.tx);
+    a.ty = fma(tk, y, a.ty);
+    a.txy = fma(tk, xy, a.txy);
     // the nearest node takes the viscosity with the quadrant weight
     // 4 (wa - 1/2)(wb - 1/2), wa = max(X0, X1) = (1 + |x|) / 2 (zero on a midline)
     const double lnu = rec_lnu(u.x, u.y, u.w);
@@ -727,12 +738,13 @@ __device__ __forceinline__ void acc_rec(CellAcc<NT> &a, uint4 u, const QConst &Q
     a.n[3] = fma(t, unit_of(bx ^ by), a.n[3]);
     // the cell centre takes it with the tent weight 4 (dx - 1/2)(dy - 1/2),
     // dx = 1 - |X0 - 1/2| = 1 - |x| / 2
-    const double c = (1.0 - fabs(x)) * (1.0 - fabs(y));
-    a.nd = __fma_rd(lnu, c, a.nd);
-    a.wnd = __dadd_rd(a.wnd, c);
+    const double c = odd((1.0 - fabs(x)) * (1.0 - fabs(y)));
+    a.nd = fma(lnu, c, a.nd);
+    a.wnd += c;
 }
 
-// a record whose terms are zero in every sum but wnd (there 1): x = y = T = 0, lnu = 0
+// a record whose terms are zero in every sum but wnd (there 1, 2^-52 being less than
+// half of any q / 2): x = y = T = 0, lnu = 0
 __device__ __forceinline__ uint4 rec_none() { return make_uint4(1u << 23, 1u << 23, 0u, 0u); }
 
 struct RecPair {
