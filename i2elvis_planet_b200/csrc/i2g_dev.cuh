@@ -293,12 +293,13 @@ __device__ __forceinline__ void fdw_pair(const LinePair *__restrict__ P, int i, 
     }
 }
 
-// v / 6.0 (tiny, infinite and NaN v take the division itself: the correction of an
-// infinite quotient is a NaN)
-__device__ __forceinline__ double sixth_of(double v)
+// a / h for any a: tiny, infinite and NaN ones take the division itself (the correction
+// of an infinite quotient is a NaN)
+__device__ __forceinline__ double div_any(double a, double h, double r)
 {
-    return abs_hi(v) - kDivTiny >= 0x7ff00000u - kDivTiny ? v / 6.0 : div_by(v, 6.0, 1.0 / 6.0);
+    return abs_hi(a) - kDivTiny >= 0x7ff00000u - kDivTiny ? a / h : div_by(a, h, r);
 }
+__device__ __forceinline__ double sixth_of(double v) { return div_any(v, 6.0, 1.0 / 6.0); }
 
 // FP32 weights from an FP64 offset and a precomputed FP32 reciprocal spacing.
 __device__ __forceinline__ void fdw32(double x0, float inv_h, double xi, float &w0, float &w1)

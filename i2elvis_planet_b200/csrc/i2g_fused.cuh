@@ -863,6 +863,7 @@ struct CellNodesArgs {
     const OvfRec *ovf;
     FusedCounters *ctr;
     double sv[4][4];  // per type slot: ro, cp, kt, ht
+    int32_t plain;    // none of them is above 2^500 or no number (div_by's means)
     // a step replayed from a CUDA graph: the slots' radiogenic heat from the
     // step's row of a device table (stepc[4 * *stepi + group] x density, group
     // 1..3 = silicate, iron, chondrite, 0 = none) instead of sv[.][3]; NULL otherwise
@@ -960,12 +961,15 @@ __device__ __forceinline__ void node_write(const CellNodesArgs &P, int64_t m3, c
             k += P.sv[s][2] * S[s];
             h += slot_heat()[s] * S[s];
         }
+        // the quotients over one reciprocal (a weight sum is at least one quantum: within
+        // div_by's range)
         const double iw = 1.0 / W0;
-        P.O.ro[m3] = r * iw;
+        auto mean = [&](double v) { return P.plain ? div_by(v, W0, iw) : v / W0; };
+        P.O.ro[m3] = mean(r);
         P.O.et[m3] = 0.0;  // beta is zero on constant-property calls
-        P.O.cp[m3] = c * iw;
-        P.O.kt[m3] = k * iw;
-        P.O.ht[m3] = h * iw;
+        P.O.cp[m3] = mean(c);
+        P.O.kt[m3] = mean(k);
+        P.O.ht[m3] = mean(h);
         if (W1 != 0.0) P.O.tk[m3] = TK / W1;
     }
 }

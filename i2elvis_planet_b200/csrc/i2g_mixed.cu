@@ -289,6 +289,10 @@ int launch_avg_fused(const StepLaunch &L, const AvgArgsK &V, const FusedLaunch &
     P.viscmod = V.viscmod;
     P.nubeg = V.nubeg;
     P.nuend = V.nuend;
+    P.plain = 1;
+    for (int k = 0; k < F.nt; k++)
+        for (double v : F.sv[k])
+            if (!(fabs(v) < 0x1p500)) P.plain = 0;
     P.mu = L.G.mu;
     P.O = O;
     P.navg = F.navg;

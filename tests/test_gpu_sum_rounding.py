@@ -1,5 +1,5 @@
-"""Rounding of the fused averaging's cell sums, on records whose exact sums are known:
-n equal markers in one cell of a grid that does not move.
+"""Rounding of the fused averaging's cell sums and means, on records whose exact sums
+are known: n equal markers in one cell of a grid that does not move.
 
 Every term of a sum is rounded to a multiple of u, half the spacing of doubles at the
 sum's start (2^(e-53), 2^e the power of two above 4 max(n, 4) (1 + 2^-20) times the
@@ -79,3 +79,17 @@ def test_cell_centre_viscosity_rounds_to_nearest(lines, n):
     bound = 0.5 * un / (eta * w) + 2 * UNIT
     got = nodes["nd"][c + 1, c + 1]
     assert abs(got / eta - 1) <= bound, (got / eta - 1) / bound
+
+
+@pytest.mark.parametrize("lines", [33, 193], ids=["two-lanes", "one-lane"])
+def test_means_are_quotients(lines):
+    """49 markers in the middle of a cell: every weight sum is 49/4, and a product with
+    it divides back to the value (times its reciprocal it does not)."""
+    for cp, kt in ((1000.0, 3.0), (800.0, 40.0)):
+        inst, nodes, c = crowd(49, lines, 0, 0, 512.0, 1e19)
+        t = inst.types
+        assert (t["markcp"][5] * 12.25) * (1 / 12.25) != t["markcp"][5]
+        at = np.s_[c:c + 2, c:c + 2]
+        np.testing.assert_array_equal(nodes["ro"][at], t["markro"][5])
+        np.testing.assert_array_equal(nodes["cp"][at], t["markcp"][5])
+        np.testing.assert_array_equal(nodes["kt"][at], t["markkt"][5])
