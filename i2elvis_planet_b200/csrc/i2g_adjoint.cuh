@@ -289,11 +289,12 @@ __device__ __forceinline__ void rk4_reverse(const GridView &G, const AdjView &Md
     // v0 = (v1 + 2 v2 + 2 v3 + v4) / 6; a stage point's own dependence on the stage
     // before it enters that stage's factor
     double px = 0.0, py = 0.0;
+    const double ax = nst == 1 ? g0x : sixth_of(g0x), ay = nst == 1 ? g0y : sixth_of(g0y);
 #pragma unroll 1
     for (int st = nst - 1; st >= 0; st--) {
-        const double c = nst == 1 ? 1.0 : (st == 0 || st == 3 ? 1.0 / 6.0 : 1.0 / 3.0);
+        const double c = st == 0 || st == 3 ? 1.0 : 2.0;
         const double h = st == 2 ? dt : 0.5 * dt;  // (the last stage: px = py = 0)
-        const double kx = g0x * c + h * px, ky = g0y * c + h * py;
+        const double kx = ax * c + h * px, ky = ay * c + h * py;
         const VStencil<MIXED> S = Q.get(st);
         double wx[2], wy[2];
         a_weights<MIXED>(S, wx, wy);
