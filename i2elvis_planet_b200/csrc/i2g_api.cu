@@ -81,11 +81,14 @@ struct i2g_ctx {
     int *typecheck = nullptr;       // device: {bad-type bits, first bad marker}
     int32_t *ndeferred = nullptr;   // device: markers deferred to the general property model
     uint8_t *tconst = nullptr;      // device: per-type table of a constant-property averaging call
-    // pinned host memory, one block: the set call's mirror of typecheck, the fused
-    // step's overflow flag, and room for small grids' tables and fields (kStageBytes)
+    // pinned host memory, one block: the set call's mirror of typecheck and the fused
+    // step's overflow flag
     uint8_t *pinned = nullptr;
+    // room in pinned memory for a small grid's tables and fields (kStageBytes), from the
+    // second i2g_set_grid on: a run that sets its grid once needs none
     uint8_t *stage = nullptr;
-    int64_t stage_bytes = 0;
+    int64_t stage_bytes = 0;  // 0: the grid is not small, or no such memory was to be had
+    bool grid_sent = false;   // an i2g_set_grid that could have used it is behind
     int *typecheck_host = nullptr;
     bool gzero[G_N] = {};  // the field is zero on the device
     std::vector<double> hgx, hgy;  // the lines of the last i2g_set_grid
@@ -645,6 +648,7 @@ int i2g_destroy(i2g_ctx *c)
     for (void *p : c->allocs) cudaFree(p);
     if (c->fz.ra) cudaFree(c->fz.ra);
     if (c->pinned) cudaFreeHost(c->pinned);
+    if (c->stage) cudaFreeHost(c->stage);
     for (auto &p : c->pending) {
         cudaEventDestroy(p.a);
         cudaEventDestroy(p.b);
@@ -761,14 +765,13 @@ int i2g_create(i2g_ctx **out, const i2g_params *P, const i2g_types *T)
 #undef A
     c->stage_bytes = lb + (int64_t)sizeof(double) * G_N * c->pitch;
     if (c->stage_bytes > kStageBytes) c->stage_bytes = 0;
-    if (cudaHostAlloc((void **)&c->pinned, 256 + (size_t)c->stage_bytes, cudaHostAllocMapped) != cudaSuccess) {
+    if (cudaHostAlloc((void **)&c->pinned, 256, cudaHostAllocMapped) != cudaSuccess) {
         cudaGetLastError();
         c->pinned = nullptr;
         return bail(I2G_ENOMEM);
     }
     c->typecheck_host = reinterpret_cast<int *>(c->pinned);
     c->fz.spilled = reinterpret_cast<int32_t *>(c->pinned + 128);
-    c->stage = c->stage_bytes ? c->pinned + 256 : nullptr;
     *c->fz.spilled = 0;
     uint8_t *pinned_dev = nullptr;
     if (cudaHostGetDevicePointer((void **)&pinned_dev, c->pinned, 0) != cudaSuccess) return bail(I2G_ECUDA);
@@ -805,12 +808,12 @@ int i2g_set_types(i2g_ctx *c, const i2g_types *T)
     return I2G_OK;
 }
 
-// Whether the caller's arrays go through the context's pinned memory: a small grid, every
-// non-NULL p[k] host memory (device memory is left to cudaMemcpy, which refuses it as
-// it always did), pinned only while small
+// Whether the caller's arrays may go through the context's pinned memory: a small grid,
+// every non-NULL p[k] host memory (device memory is left to cudaMemcpy, which takes it
+// as it always did), pinned only while small
 static bool staged_arrays(const i2g_ctx *c, const double *const *p, int k)
 {
-    if (!c->stage) return false;
+    if (!c->stage_bytes) return false;
     const bool small = (int64_t)sizeof(double) * c->nn <= kStagePinned;
     for (int a = 0; a < k; a++) {
         if (!p[a]) continue;
@@ -822,6 +825,22 @@ static bool staged_arrays(const i2g_ctx *c, const double *const *p, int k)
         if (at.type != cudaMemoryTypeUnregistered && !(at.type == cudaMemoryTypeHost && small)) return false;
     }
     return true;
+}
+
+// The context's pinned room, allocated by the second call that asks for it
+static bool stage_room(i2g_ctx *c)
+{
+    if (c->stage) return true;
+    if (!c->grid_sent) {
+        c->grid_sent = true;
+        return false;
+    }
+    if (cudaHostAlloc((void **)&c->stage, (size_t)c->stage_bytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        c->stage = nullptr;
+        c->stage_bytes = 0;
+    }
+    return c->stage != nullptr;
 }
 
 // the mixed form's copies of the context's grid fields
@@ -873,7 +892,7 @@ int i2g_set_grid(i2g_ctx *c, const double *gx, const double *gy, const double *v
     // which end synchronised), else in memory of their own
     const size_t lbytes = (size_t)(line_bytes(nx) + line_bytes(ny));
     const double *src[G_N] = {vx, vy, pr, exx, eyy, exy, sxx, syy, sxy, ga, mu};
-    const bool staged = staged_arrays(c, src, G_N);
+    const bool staged = staged_arrays(c, src, G_N) && stage_room(c);
     std::vector<double> host(staged ? 0 : lbytes / sizeof(double), 0.0);
     uint8_t *hl = staged ? c->stage : reinterpret_cast<uint8_t *>(host.data());
     if (staged) memset(hl, 0, lbytes);
@@ -1011,7 +1030,7 @@ static int get_nodes_impl(i2g_ctx *c, double *const *f, cudaMemcpyKind kind)
         return I2G_OK;
     }
     const size_t fb = sizeof(double) * (size_t)c->nn, pb = sizeof(double) * (size_t)c->pitch;
-    if (kind == cudaMemcpyDeviceToHost && staged_arrays(c, f, N_N)) {
+    if (kind == cudaMemcpyDeviceToHost && c->stage && staged_arrays(c, f, N_N)) {
         // a small grid: every field in one copy, then into the caller's arrays
         static_assert(N_N <= G_N, "the node fields fit the room of the grid's");
         CK(cudaMemcpyAsync(c->stage, c->node[0], N_N * pb, cudaMemcpyDeviceToHost, c->stream));
