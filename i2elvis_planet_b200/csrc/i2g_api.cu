@@ -1419,10 +1419,10 @@ static bool fused_call(const i2g_ctx *c, double timesum)
 static int fused_check_overflow(i2g_ctx *c, int32_t tolerate = 0)
 {
     if (c->in_graph || !*(volatile int32_t *)c->fz.spilled) return I2G_OK;
-    CK(cudaStreamSynchronize(c->stream));
-    *(volatile int32_t *)c->fz.spilled = 0;
     std::vector<uint8_t> ctr(fused_counters_bytes());
-    CK(cudaMemcpy(ctr.data(), c->fz.ctr, ctr.size(), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(ctr.data(), c->fz.ctr, ctr.size(), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    *(volatile int32_t *)c->fz.spilled = 0;  // (no movemark is in flight)
     int32_t cmax = 0, novf = 0;
     fused_host_stats(ctr.data(), &cmax, &novf);
     if (novf > tolerate && cmax > c->fz.cap) {
