@@ -115,7 +115,7 @@ __device__ __forceinline__ void contrib_marker(const GridView &G, const MarkerVi
 {
     using W = typename AvgCfg<MIXED>::W;
     const bool has_tmax = A.tmax != nullptr, has_por = A.por != nullptr, has_hi = A.hi != nullptr;
-    const int64_t i = perm ? (int64_t)__ldg(perm + j) : j;
+    const int64_t i = perm ? (int64_t)perm[j] : j;
     MarkerRec r;
     r.x = A.x[i];
     r.y = A.y[i];
@@ -202,7 +202,7 @@ __device__ __forceinline__ void contrib_inplace(const GridView &G, const MarkerV
     r.mgt = A.mgo ? A.mgt[i] : -1.0;
     const double T_in = r.T, tmax_in = r.tmax, por_in = r.por;
     const int type_in = r.type;
-    const int32_t k = __ldg(key + i);
+    const int32_t k = key[i];
     const int32_t nc2 = (int32_t)(G.ny - 1);
     const int32_t m10 = k / nc2, m20 = k - m10 * nc2;
     MarkerContrib mc;
@@ -243,7 +243,7 @@ __device__ __forceinline__ void contrib_inplace(const GridView &G, const MarkerV
             u.r.flag = fl;
         }
     }
-    uint4 *d = P + (int64_t)__ldg(rank + i) * PayVec<MIXED, CONST>::R4;
+    uint4 *d = P + (int64_t)rank[i] * PayVec<MIXED, CONST>::R4;
 #pragma unroll
     for (int q = 0; q < PayVec<MIXED, CONST>::R4; q++) d[q] = u.v[q];
 }
@@ -409,8 +409,8 @@ __global__ void __launch_bounds__(256) k_contrib_const(const __grid_constant__ G
         for (int q = 0; q < PV::R4; q++) d[q] = u.v[q];
     };
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += (int64_t)gridDim.x * blockDim.x)
-        one(i, A.x[i], A.y[i], A.T[i], A.eta[i], A.type[i], args.gridmod > 1 ? A.id[i] : 0, __ldg(key + i),
-            __ldg(rank + i));
+        one(i, A.x[i], A.y[i], A.T[i], A.eta[i], A.type[i], args.gridmod > 1 ? A.id[i] : 0, key[i],
+            rank[i]);
 }
 
 // the markers k_contrib_const deferred, through the general property model

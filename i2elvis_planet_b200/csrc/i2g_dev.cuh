@@ -169,8 +169,10 @@ struct NodeOut {
 
 // The two ends of a programmatic launch (launch_next): the kernel before lets the next
 // one's CTAs start, the next one waits until every kernel before it is done and its
-// writes are seen.  What those wrote is read by plain loads, or through a pointer from
-// after_wait, which no load can be moved ahead of.
+// writes are seen.  What those wrote is read by plain loads, and through a pointer from
+// after_wait where the compiler takes the pointer's memory for constant (const and
+// __restrict__ parameters), so that no load moves ahead of the wait; the read-only path
+// (__ldg) is for what no kernel of the step writes.
 __device__ __forceinline__ void allow_next() { cudaTriggerProgrammaticLaunchCompletion(); }
 __device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
 template <typename T>

@@ -305,7 +305,7 @@ static __device__ __forceinline__ int td_branch(const i2g_types &T, const AvgArg
 {
     const int nt = MIXED ? td_props_mixed(A.td, T, A.nubeg, A.nuend, mtk, mpb, mm2, mro, mcp, mbb, mkt, mnu)
                          : td_props(A.td, T, A.nubeg, A.nuend, mtk, mpb, mm2, mro, mcp, mbb, mkt, mnu);
-    if (id == __ldg(A.td.last)) td_write_state(A.td, mtk, mpb, mm2);
+    if (id == *A.td.last) td_write_state(A.td, mtk, mpb, mm2);
     return nt;
 }
 

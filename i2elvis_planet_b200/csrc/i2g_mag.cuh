@@ -65,11 +65,11 @@ __device__ __forceinline__ int mag_state(int dynamo, int mm2, double mtk, int ol
 __device__ __forceinline__ double mag_time_of(const AvgArgsK &A, int32_t id, bool assigns, double val)
 {
     if (assigns) {
-        if (id == __ldg(A.mag_last)) *A.mag_out = val;
+        if (id == *A.mag_last) *A.mag_out = val;
         return val;
     }
-    const int32_t p = id > 0 ? __ldg(A.mag_prev + id - 1) : -1;
-    return p >= 0 ? __ldg(A.mag_val + p) : __ldg(A.mag_in);
+    const int32_t p = id > 0 ? A.mag_prev[id - 1] : -1;
+    return p >= 0 ? A.mag_val[p] : *A.mag_in;
 }
 
 }  // namespace i2g

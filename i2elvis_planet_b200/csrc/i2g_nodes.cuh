@@ -23,22 +23,27 @@ __device__ __forceinline__ void node_finalize(const GridView &G, const double *_
 {
     const int64_t nx = G.nx, ny = G.ny, nc2 = ny - 1, ncells = (nx - 1) * nc2;
     const int64_t m1 = m3 / ny, m2 = m3 - m1 * ny;
-    double s[10];
-#pragma unroll
-    for (int f = 0; f < 10; f++) s[f] = 0.0;
+    // the four cells' sums, all of them in flight at once, then added in their order
+    double v[4][10], s[10];
 #pragma unroll
     for (int qq = 0; qq < 4; qq++) {
         const int64_t c1 = m1 - 1 + (qq >> 1), c2 = m2 - 1 + (qq & 1);
-        if (c1 < 0 || c2 < 0 || c1 > nx - 2 || c2 > ny - 2) continue;
+        const bool on = c1 >= 0 && c2 >= 0 && c1 <= nx - 2 && c2 <= ny - 2;
         const double *src = part + (int64_t)((3 - qq) * 10) * ncells + c1 * nc2 + c2;
 #pragma unroll
-        for (int f = 0; f < 10; f++) s[f] += __ldg(src + (int64_t)f * ncells);
+        for (int f = 0; f < 10; f++) v[qq][f] = on ? src[(int64_t)f * ncells] : 0.0;
+    }
+#pragma unroll
+    for (int f = 0; f < 10; f++) {
+        s[f] = 0.0;
+#pragma unroll
+        for (int qq = 0; qq < 4; qq++) s[f] += v[qq][f];
     }
     double snd = 0.0, swnd = 0.0;
     if (m1 >= 1 && m2 >= 1) {
         const int64_t cc = (m1 - 1) * nc2 + (m2 - 1);
-        snd += __ldg(part + 40 * ncells + cc);
-        swnd += __ldg(part + 41 * ncells + cc);
+        snd += part[40 * ncells + cc];
+        swnd += part[41 * ncells + cc];
     }
     const double mu = G.mu ? __ldg(G.mu + m3) : 0.0;
     if (s[F_WNU]) {

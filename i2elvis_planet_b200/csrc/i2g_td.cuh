@@ -436,13 +436,13 @@ static __device__ __noinline__ double td_last_melt(const TdArgs &D, double mtk, 
 // table marker before it in the caller's order, else the state the call began with
 __device__ __forceinline__ void td_prev_melt(const TdArgs &D, int32_t id, double &xsi, double &xfe)
 {
-    const int32_t p = id > 0 ? __ldg(D.prev + id - 1) : -1;
+    const int32_t p = id > 0 ? D.prev[id - 1] : -1;
     if (p >= 0) {
-        xsi = __ldg(D.si + p);
+        xsi = D.si[p];
         xfe = 0.0;
     } else {
-        xsi = __ldg(D.melt_in + 0);
-        xfe = __ldg(D.melt_in + 2);
+        xsi = D.melt_in[0];
+        xfe = D.melt_in[2];
     }
 }
 

@@ -179,6 +179,7 @@ __global__ void __launch_bounds__(256) k_tsums(const uint4 *__restrict__ records
     allow_next();
     wait_previous();
     records = after_wait(records);
+    cstart = after_wait(cstart);
     const int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (cell >= ncells) return;
     const int32_t s = cstart[cell], n = cstart[cell + 1] - s;
