@@ -52,9 +52,8 @@ struct FusedCounters {
 };
 
 struct OvfRec {
-    float4 a;      // the record (rec_pack)
-    double lnu;    // its log-viscosity, unrounded (not read by the sums)
-    int32_t cell, pad;
+    float4 a;  // the record (rec_pack)
+    int32_t cell, pad[3];
 };
 
 struct FusedMove {
@@ -428,12 +427,8 @@ __device__ __forceinline__ void move_record(const GridView &G, const MarkerView 
         } else {
             const int32_t o = atomicAdd(&F.ctr->novf, 1);
             if (o == 0) *(volatile int32_t *)F.spilled = 1;
-            OvfRec r;
-            r.a = rec;
-            r.lnu = lnu;
-            r.cell = key;
-            r.pad = 0;
-            F.ovf[o] = r;
+            F.ovf[o].a = rec;
+            F.ovf[o].cell = key;
             place = -(o + 1);
         }
         if (defer) F.defer[atomicAdd(&F.ctr->ndefer, 1)] = make_int2((int32_t)i, place);
@@ -503,7 +498,7 @@ __device__ __forceinline__ void move_stage_issue(const MarkerView &M, MoveStage 
 // 642k markers: 69.0 -> 67.0 us and 624 -> 604 instructions per warp and tile with the
 // types' flags in shared memory, the box tests shared, and clamps of one instruction.
 template <bool VISC, bool UNI>
-__global__ void __launch_bounds__(kMoveTile, VISC ? 4 : 4) k_move_fused(const __grid_constant__ GridView G,
+__global__ void __launch_bounds__(kMoveTile, 4) k_move_fused(const __grid_constant__ GridView G,
                                                     const __grid_constant__ MarkerView M,
                                                     const DevTypes *__restrict__ Ty, const __grid_constant__ MoveArgs A,
                                                     const __grid_constant__ FusedMove F)
@@ -1318,7 +1313,6 @@ __global__ void __launch_bounds__(256) k_fused_begin(const __grid_constant__ Gri
         } else {
             OvfRec &r = F.ovf[-d.y - 1];
             r.a = rec_with_lnu(r.a, lnu);
-            r.lnu = lnu;
         }
         atomicMax(&F.ctr->part[q % kFusedParts][2], __float_as_uint(__double2float_ru(fabs(lnu))));
     }
