@@ -78,12 +78,13 @@ def peaks():
     return FALLBACK_HBM_GBS, "fallback"
 
 
-def profile_traffic(kernel: str):
-    """DRAM bytes per marker of `kernel` from a committed ncu summary (profiles/)."""
+def profile_traffic(kernel: str, precision: str = "mixed"):
+    """DRAM bytes per marker of `kernel` from a committed ncu summary (profiles/), of
+    this precision's form where there is one."""
     d = os.path.join(ROOT, "profiles")
     if not os.path.isdir(d):
         return None
-    for fn in sorted(os.listdir(d)):
+    for fn in sorted(os.listdir(d), key=lambda f: (not f.endswith(f"_{precision}.txt"), f)):
         # <kernel>_<workload>_<precision>.txt
         if not fn.endswith(".txt") or fn.rsplit("_", 2)[0] != kernel:
             continue
@@ -518,7 +519,7 @@ def run_ours(args) -> None:
     per_launch_ms = prof["ms"][dom] / calls
     alg = bm * nm + bn * nn
     achieved = alg / (per_launch_ms / 1e3) / 1e9 if alg else 0.0
-    tr = profile_traffic(kname)
+    tr = profile_traffic(kname, args.precision)
     step_bytes = B_MARKER * nm + B_NODE * nn
     step_gbs = step_bytes / (ms_total / args.steps / 1e3) / 1e9
 

@@ -317,8 +317,8 @@ struct AxisTables {
 
 // Grids whose tables and fields take this much or less cross through pinned memory of
 // the context in one copy each way: a coupled step (grid up, move, average, nodes back)
-// of 21^2 nodes 235 -> 104 us, 101^2 340 -> 167, 201^2 (4.1 MB) 540 -> 424.  At 301^2
-// (9.2 MB) the host's copies cost what the calls save: 821 -> 808, not worth the memory.
+// of 21^2 nodes 235 -> 104 us, 101^2 340 -> 167, 201^2 (3.6 MB) 540 -> 424.  At 301^2
+// (8.0 MB) the host's copies cost what the calls save: 821 -> 808, not worth the memory.
 constexpr int64_t kStageBytes = 5 << 20;
 // Fields in the caller's own pinned memory cross at full rate by themselves; theirs
 // are staged only while a field is this small, where the call costs more than its bytes

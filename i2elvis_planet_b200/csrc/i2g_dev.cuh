@@ -589,8 +589,8 @@ __device__ __forceinline__ ViscType visc_type(const i2g_types &T, int m)
 // 128-bit arithmetic is viscalc's (300 to 1800 K, strain rates of 1e-17 to 1e-13, mean and
 // largest: power law 2.7e-15 and 1.4e-14 in both, brittle 1.0e-16 and 5.5e-16, Peierls
 // creep 1.0e-15 and 1.6e-12); with the powers as exp and log of what they multiply it was
-// 9% larger for the power law and three times for the brittle strength, for 6% of the
-// rheology workload's time.
+// 9% larger for the power law and three times for the brittle strength, for 3 to 6% less
+// of the rheology workload's time.
 __device__ __forceinline__ double viscalc_mixed(const i2g_types &T, const ViscType &V, double mtk, double mpb, double hi,
                                                 double epsin, double sigin, double et, double timesum,
                                                 double relax_time, double nubeg, double nuend, int mm2)

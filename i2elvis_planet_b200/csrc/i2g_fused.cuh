@@ -493,10 +493,11 @@ __device__ __forceinline__ void move_stage_issue(const MarkerView &M, MoveStage 
 // viscosity update a thread reads the marker its class order gives it, behind the
 // order's barriers.  Viscosity update, nonuniform grid, 4M markers: 564 us with
 // viscalc's own expressions and searches and walks by the whole axis, 348 with
-// viscalc_mixed and the class order, 284 with the axis bins and branch-free stage steps;
-// two or three CTAs per SM 401, five 350.  Uniform grid without the update, 401^2 nodes,
-// 642k markers: 69.0 -> 67.0 us and 624 -> 604 instructions per warp and tile with the
-// types' flags in shared memory, the box tests shared, and clamps of one instruction.
+// viscalc_mixed and the class order (two or three CTAs per SM 401, five 350), 284 with
+// the axis bins and branch-free stage steps; viscalc_mixed's powers as pow, for its
+// precision, have added 11 since.  Uniform grid without the update, 401^2 nodes, 2.56M
+// markers: 69.0 -> 67.0 us and 624 -> 604 instructions per warp and tile with the types'
+// flags in shared memory, the box tests shared, and clamps of one instruction.
 template <bool VISC, bool UNI>
 __global__ void __launch_bounds__(kMoveTile, 4) k_move_fused(const __grid_constant__ GridView G,
                                                     const __grid_constant__ MarkerView M,
@@ -1127,13 +1128,18 @@ static __device__ __noinline__ void node_guard(const CellNodesArgs &P, int m1, i
 // (column w + 1; column 0 holds the last one of the group before); then a thread
 // finishes a node from its four cells.
 //
-// Bound by issue and the FP64 pipe: per record and lane 33 FP64 operations and
-// about 75 instructions in all, no branch; a cell and its node add about 500 once.
-// A lane to a cell reads whole kilobytes (rec_place) and needs no staging; S = 2
+// Per record and lane 32 FP64 operations and about 75 instructions in all, no branch; a
+// cell and its node add about 500 once.  No one resource bounds it: at 13M records and
+// 601^2 nodes 53% of the issue slots, 42% of the FP64 pipe and 30% of the DRAM rate
+// (18.4 B a record) are in use, with 260 CTAs for 296 places and 16 warps on a full SM;
+// a warp runs as long as its fullest cell in whole batches (14% more than the mean after
+// five steps at 36 a cell), and waits for its records' loads and its sums' dependent
+// steps with few others to fill in.  A lane to a cell reads whole kilobytes (rec_place) and needs no staging; S = 2
 // halves the serial chain where a grid leaves the device idle.  Per launch, with the
 // kernel that staged the records and picked slots and quadrants by one-hot factors
 // (226 instructions per record) before: 36M records, 1001^2 nodes 314 -> 207 us (DRAM
 // alone: 120); 2.56M, 401^2 41 -> 30; 160k, 101^2 24.5 -> 8.3; 6400, 21^2 21.7 -> 8.0.
+// The means as quotients have added 1 to 2% since.
 constexpr int kCnCols = 8, kCnThreads = 32 * kCnCols;
 constexpr int kCnBatch = 2;  // pairs of records per batch
 template <int NT, int S>
