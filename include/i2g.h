@@ -372,8 +372,9 @@ int i2g_adjoint_backward(i2g_ctx *ctx, const double *dL_dtk, double *dL_dT0, dou
  * averaging run as persistent grids), the eleven launches of a step are captured
  * once into a CUDA graph and replayed per step.  Results are identical, bit for
  * bit, to stepping each context alone; the batch borrows the contexts' device
- * state and leaves it current on return.  No counterpart in the reference,
- * which runs one planetesimal per process. */
+ * state and leaves it current on return.  Between two calls a member's types, grid,
+ * markers and extras may be set and the member stepped alone.  No counterpart in
+ * the reference, which runs one planetesimal per process. */
 typedef struct i2g_batch i2g_batch;
 
 /* launch shape of a batch: averaging tile width in cell columns (8|16|32) and

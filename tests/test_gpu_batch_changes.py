@@ -45,6 +45,9 @@ def change(kind, ms, inst):
         t = inst.mtype.copy()
         t[inst.mtype == 5], t[inst.mtype == 7] = 7, 6
         ms.set_markers(inst.x, inst.y, inst.T + 3.0, inst.eta, t)
+    elif kind == "fewer":
+        half = slice(0, inst.marknum // 2)
+        ms.set_markers(inst.x[half], inst.y[half], inst.T[half], inst.eta[half], inst.mtype[half])
     elif kind == "extras":
         ms.set_marker_extras(tmax=inst.tmax, hi=np.full(inst.marknum, 0.5))
     elif kind == "porosity":
@@ -55,7 +58,7 @@ def outputs(steps):
     return [dict(ms.get_markers(), **{"node_" + k: v for k, v in ms.get_nodes().items()}) for ms in steps]
 
 
-@pytest.mark.parametrize("kind", ["types", "lines", "field", "markers", "extras", "porosity"])
+@pytest.mark.parametrize("kind", ["types", "lines", "field", "markers", "fewer", "extras", "porosity"])
 @pytest.mark.parametrize("strategy,precision", [(abi.BATCH_STREAMS, abi.PREC_MIXED), (abi.BATCH_FUSED, abi.PREC_MIXED),
                                                 (abi.BATCH_FUSED, abi.PREC_FP64)], ids=["graph", "fused-mixed", "fused-fp64"])
 def test_member_changes_between_steps(kind, strategy, precision):
