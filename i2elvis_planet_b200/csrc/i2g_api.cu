@@ -1432,6 +1432,19 @@ static int fused_check_overflow(i2g_ctx *c, int32_t tolerate = 0)
     return I2G_OK;
 }
 
+// What a fused movemark at timesum leaves: records in the buckets, and markers whose
+// cells and order nobody has worked out
+static void fused_moved(i2g_ctx *c, double timesum)
+{
+    c->fz.ready = true;
+    c->fz.resets_done = false;
+    c->fz.timesum = timesum;
+    c->keys_stale = true;
+    c->keys_dirty = false;
+    c->order_sorted = false;
+    c->ranks_valid = false;
+}
+
 int i2g_movemark(i2g_ctx *c, double timestep, double timesum, uint32_t flags)
 {
     int r = check_ctx(c, true);
@@ -1473,14 +1486,8 @@ int i2g_movemark(i2g_ctx *c, double timestep, double timesum, uint32_t flags)
             c->launches += launch_move_fused(L, A, V, F);
         }
         CKL();
-        c->fz.ready = true;
-        c->fz.resets_done = false;
-        c->fz.timesum = timesum;
+        fused_moved(c, timesum);
         c->fz.calls++;
-        c->keys_stale = true;
-        c->keys_dirty = false;
-        c->order_sorted = false;
-        c->ranks_valid = false;
         return I2G_OK;
     }
     {
@@ -2630,6 +2637,7 @@ int batch_run_streams_graph(i2g_batch *b, const double *timestep, double *timesu
         BCK(cudaEventCreate(&e1));
     }
     bool first = true;
+    std::vector<double> last(timesum, timesum + n);  // the last step's timesum
     for (int32_t done = 0; done < nsteps;) {
         const int ns = std::min<int32_t>(nsteps - done, i2g_batch::kMaxSteps);
         std::vector<double> tnext;
@@ -2637,7 +2645,11 @@ int batch_run_streams_graph(i2g_batch *b, const double *timestep, double *timesu
         if (ms && first) BCK(cudaEventRecord(e0, b->stream));
         first = false;
         for (int s = 0; s < ns; s++) BCK(cudaGraphLaunch(b->sexec, b->stream));
-        for (int k = 0; k < n; k++) timesum[k] = tnext[k];
+        for (int k = 0; k < n; k++) {
+            last[k] = timesum[k];
+            for (int s = 1; s < ns; s++) last[k] += timestep[k];  // as the steps add it up
+            timesum[k] = tnext[k];
+        }
         done += ns;
     }
     if (ms) {
@@ -2647,11 +2659,16 @@ int batch_run_streams_graph(i2g_batch *b, const double *timestep, double *timesu
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
     }
-    // the contexts' streams order after the replays; record moves of the
-    // instances that are due, copied back into the buffer the graph reads
+    // the contexts' streams order after the replays, whose last movemark and averaging
+    // the contexts take note of; record moves of the instances that are due, copied
+    // back into the buffer the graph reads
     BCK(cudaEventRecord(b->ev, b->stream));
-    for (auto *c : b->ctx) {
+    for (int k = 0; k < n; k++) {
+        i2g_ctx *c = b->ctx[k];
         BCK(cudaStreamWaitEvent(c->stream, b->ev, 0));
+        fused_moved(c, last[k]);
+        c->fz.resets_done = true;
+        c->timestep = timestep[k];
         c->fz.calls += nsteps;
         c->since_reorder += nsteps;
         if (c->since_reorder >= fused_reorder_every(c)) {

@@ -40,3 +40,42 @@ def test_replays_wait_for_the_contexts_streams():
             for f in c:
                 np.testing.assert_array_equal(a[f], c[f], err_msg=f)
     b.close()
+
+
+@pytest.mark.parametrize("every", [1, 8], ids=["sorted-between", "ranked-between"])
+def test_members_know_that_replays_moved_them(every):
+    """Temperature updates and averaging of the general path between replayed steps:
+    the members' ranks and order are of the positions the replays left."""
+    insts = [synth.make_instance(f"m{i}", n=n, k=3, nsteps=1, seed=700 + i, r_disk=150e3, vmax=10.0 ** (-9.0 + i), extra_modes=2)
+             for i, n in enumerate((61, 41))]
+    batched, alone = ([lib.MarkerStep.from_instance(i, precision=abi.PREC_MIXED) for i in insts] for _ in range(2))
+    for ms in batched:
+        ms.set_reorder_interval(every)
+    b = lib.Batch(batched)
+    b.set_tune(strategy=abi.BATCH_STREAMS)
+    dt = np.array([i.timestep for i in insts])
+    ts = np.array([i.timesum for i in insts])
+
+    def between(ms, k, call):
+        tk = insts[k].nodes["tk"] + 500.0 + 20.0 * np.sin(np.arange(insts[k].nodenum) + call)
+        ones = np.ones(tk.size)
+        ms.titerate_markers(tk + 3.0, tk, 1.0, dt[k], kt=3.0 * ones, cp=1000.0 * ones, ro=3300.0 * ones)
+    for call in range(5):
+        t = ts.copy()
+        b.step(dt, ts, 2)
+        for k, ms in enumerate(alone):
+            for _ in range(2):
+                ms.movemark(dt[k], t[k])
+                ms.ronurecalc(t[k])
+                t[k] += dt[k]
+        for ms in (*batched, *alone):
+            k = (batched.index(ms) if ms in batched else alone.index(ms))
+            between(ms, k, call)
+        if call == 4:  # the general path's averaging of the markers as they are
+            for ms, k in zip((*batched, *alone), (0, 1, 0, 1)):
+                ms.ronurecalc(t[k] + dt[k])
+    for got, want in zip(batched, alone):
+        for a, c in ((got.get_markers(), want.get_markers()), (got.get_nodes(), want.get_nodes())):
+            for f in c:
+                np.testing.assert_array_equal(a[f], c[f], err_msg=f)
+    b.close()
